@@ -346,17 +346,91 @@ __device__ __forceinline__ StepCoefs<T> make_coefs(double tau, double dt, double
     return c;
 }
 
-// Radius-1 stencil sum, fixed association order shared by every kernel:
-// ((x- + x+) + (y- + y+)) + (z- + z+), then centre * (-2 d) fused.
+// Sums of the neighbours of a site, shared by every kernel. Float: the fixed
+// association order ((x- + x+) + (y- + y+)) + (z- + z+).
+//
+// Double: GB300's FP64 pipe takes one warp instruction per 16 cycles and SM, so
+// an FP64 addition costs as much as 32 integer instructions there, and the FP64 kernels
+// are bound by their count of FP64 operations. The neighbour sums are
+// therefore formed on the integer pipe (sum_fixed): the terms' 53-bit
+// significands are aligned to the largest exponent E with 7 bits below its
+// last place, added as 64-bit integers and rounded once to double. A term
+// loses less than 2^-59 of 2^E, so six terms lose less than 0.05 units in the last
+// place of the largest one before the one rounding (to nearest, ties away from
+// zero), where the chain of five FP64 additions rounds five times: against the
+// exact sum its largest error over random, smooth and wide-range terms is
+// about half the chain's. The result does not depend on the order of the
+// terms. Terms all tiny (E < 64: zeros, subnormals), huge or not finite take
+// the FP64 additions, out of line: inline, the compiler predicates them, and a
+// predicated-off FP64 instruction still takes its slot of the pipe. One 3D
+// site's kick and drift (two sums of six, nine other FP64 operations): 343
+// cycles per warp and SM with FP64 sums, 161 with these, the integer work under the
+// nine operations.
+__device__ __noinline__ static double sum4_fp64(double a, double b, double c, double d) { return (a + b) + (c + d); }
+__device__ __noinline__ static double sum6_fp64(double a, double b, double c, double d, double e, double f) {
+    return ((a + b) + (c + d)) + (e + f);
+}
+template <int K>
+__device__ __forceinline__ double sum_fixed(const double (&v)[K]) {
+    static_assert(K == 4 || K == 6, "four or six neighbours: the sum stays below 2^63");
+    unsigned m[K], top = 0;
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+        m[i] = (unsigned)__double2hiint(v[i]) & 0x7fffffffu;
+        top = max(top, m[i]);
+    }
+    const unsigned E = top >> 20;
+    if (E - 64u >= 0x7f0u - 64u) {
+        if constexpr (K == 4) return sum4_fp64(v[0], v[1], v[2], v[3]);
+        else return sum6_fp64(v[0], v[1], v[2], v[3], v[4], v[5]);
+    }
+    top |= 0xfffffu;   // (top - m) >> 20 is then the difference of the exponents
+    uint64_t s = 0;
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+        const unsigned lo = (unsigned)__double2loint(v[i]);
+        const unsigned hi = (m[i] & 0xfffffu) | 0x100000u;   // a subnormal's implicit bit is shifted out
+        uint64_t x = ((uint64_t)__funnelshift_l(lo, hi, 7) << 32) | (lo << 7);   // below 2^60
+        asm("shr.u64 %0, %0, %1;" : "+l"(x) : "r"((top - m[i]) >> 20));      // 0 past 63
+        if (__double2hiint(v[i]) < 0) s -= x;
+        else s += x;
+    }
+    // s 2^(E - 1023 - 59): magnitude, leading bit to bit 63, 53 bits kept, the next one rounds
+    const int sg = (int)(s >> 32) >> 31;
+    const uint64_t a = (s ^ (uint64_t)(int64_t)sg) - (uint64_t)(int64_t)sg;
+    if (a == 0) return 0.0;
+    const int lz = __clzll((long long)a);
+    const uint64_t t = a << lz;
+    const uint64_t b = ((uint64_t)(unsigned)((int)E + 3 - lz) << 52) + (t >> 11) + ((t >> 10) & 1);
+    return __longlong_as_double((long long)(b | ((uint64_t)(unsigned)sg << 63)));
+}
+template <typename T>
+__device__ __forceinline__ T nsum7(T xm, T xp, T ym, T yp, T zm, T zp) {
+    if constexpr (sizeof(T) == 8) {
+        const double v[6] = {xm, xp, ym, yp, zm, zp};
+        return sum_fixed<6>(v);
+    } else {
+        return ((xm + xp) + (ym + yp)) + (zm + zp);
+    }
+}
+template <typename T>
+__device__ __forceinline__ T nsum5(T xm, T xp, T ym, T yp) {
+    if constexpr (sizeof(T) == 8) {
+        const double v[4] = {xm, xp, ym, yp};
+        return sum_fixed<4>(v);
+    } else {
+        return (xm + xp) + (ym + yp);
+    }
+}
+
+// Radius-1 stencil sums: the neighbours, then centre * (-2 d) fused.
 template <typename T>
 __device__ __forceinline__ T lap7(T c, T xm, T xp, T ym, T yp, T zm, T zp) {
-    T s = ((xm + xp) + (ym + yp)) + (zm + zp);
-    return fma((T)-6, c, s);
+    return fma((T)-6, c, nsum7<T>(xm, xp, ym, yp, zm, zp));
 }
 template <typename T>
 __device__ __forceinline__ T lap5(T c, T xm, T xp, T ym, T yp) {
-    T s = (xm + xp) + (ym + yp);
-    return fma((T)-4, c, s);
+    return fma((T)-4, c, nsum5<T>(xm, xp, ym, yp));
 }
 
 // The fused kick + drift of one site. (a, b) = psi, L = stencil sums (not
@@ -387,10 +461,6 @@ __device__ __forceinline__ void site_update_fold(T a, T b, T S1, T S2, T &p1, T 
     an = fma(c.dt, p1, a);
     bn = fma(c.dt, p2, b);
 }
-template <typename T>
-__device__ __forceinline__ T nsum7(T xm, T xp, T ym, T yp, T zm, T zp) { return ((xm + xp) + (ym + yp)) + (zm + zp); }
-template <typename T>
-__device__ __forceinline__ T nsum5(T xm, T xp, T ym, T yp) { return (xm + xp) + (ym + yp); }
 
 // Synchronised momentum of one site: pi_n = pih_{n-1} + dt/2 K(psi_n) with
 // c = make_coefs(tau_n, dt, dt/2, ...); (L1, L2) the stencil sums.

@@ -83,12 +83,15 @@ __device__ __forceinline__ void stencil_at(const typename Cplx<T>::type *__restr
     for (int l = 1; l <= R; ++l) {
         C xm = psi[rowbase + wrapi(x - l, N)], xp = psi[rowbase + wrapi(x + l, N)];
         C ym = psi[planebase + wrapi(y - l, N) * N + x], yp = psi[planebase + wrapi(y + l, N) * N + x];
-        T s1 = (xm.x + xp.x) + (ym.x + yp.x), s2 = (xm.y + xp.y) + (ym.y + yp.y);
-        if (ND == 3) {
+        T s1, s2;
+        if constexpr (ND == 3) {
             int64_t yx = y * N + x;
             C zm = psi[wrapi(z - l, N) * NN + yx], zp = psi[wrapi(z + l, N) * NN + yx];
-            s1 = s1 + (zm.x + zp.x);
-            s2 = s2 + (zm.y + zp.y);
+            s1 = nsum7<T>(xm.x, xp.x, ym.x, yp.x, zm.x, zp.x);
+            s2 = nsum7<T>(xm.y, xp.y, ym.y, yp.y, zm.y, zp.y);
+        } else {
+            s1 = nsum5<T>(xm.x, xp.x, ym.x, yp.x);
+            s2 = nsum5<T>(xm.y, xp.y, ym.y, yp.y);
         }
         T cl = (T)stencil_coef(setting, ND, l);
         a1 = fma(cl, s1, a1);

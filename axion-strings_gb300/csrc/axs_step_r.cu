@@ -320,10 +320,8 @@ __device__ __forceinline__ void zmarch2r_body(const ZLat *__restrict__ lats, int
 #pragma unroll
                         for (int j = 0; j < K::VS; ++j) {
                             const C xm = win[K::RP + j - l], xp = win[K::RP + j + l];
-                            T s1 = (xm.x + xp.x) + (ym[j].x + yp[j].x);
-                            T s2 = (xm.y + xp.y) + (ym[j].y + yp[j].y);
-                            s1 = s1 + (zm[j].x + zp[j].x);
-                            s2 = s2 + (zm[j].y + zp[j].y);
+                            const T s1 = nsum7<T>(xm.x, xp.x, ym[j].x, yp[j].x, zm[j].x, zp[j].x);
+                            const T s2 = nsum7<T>(xm.y, xp.y, ym[j].y, yp[j].y, zm[j].y, zp[j].y);
                             a1[j] = fma(coef[l], s1, a1[j]);
                             a2[j] = fma(coef[l], s2, a2[j]);
                         }
