@@ -116,6 +116,10 @@ static void lattice_init(Lattice *L, const axs_params &p, cudaStream_t shared) {
     L->scratch = dalloc(cbytes);
     L->dclock = (double *)dalloc(2 * sizeof(double));
     L->derr = (int *)dalloc(sizeof(int));
+    if (p.NDIMS == 2) {
+        L->dstep2d = dalloc(2 * kStep2dSlot);
+        AXS_CUDA(cudaMemsetAsync(L->dstep2d, 0xff, 2 * kStep2dSlot, L->stream));   // NaN tags: no table yet
+    }
     AXS_CUDA(cudaMemsetAsync(L->psi[0], 0, cbytes, L->stream));
     AXS_CUDA(cudaMemsetAsync(L->psi[1], 0, cbytes, L->stream));
     AXS_CUDA(cudaMemsetAsync(L->pih, 0, cbytes, L->stream));
@@ -141,6 +145,7 @@ static void lattice_free(Lattice *L) {
     dfree(L->pih);
     dfree(L->scratch);
     dfree(L->dclock);
+    dfree(L->dstep2d);
     dfree(L->derr);
     dfree(L->dstage);
     if (L->own_stream && L->stream) cudaStreamDestroy(L->stream);

@@ -116,6 +116,13 @@ struct GraphEntry {
     std::vector<uint8_t> swapped;     // per member: pih and scratch exchanged an odd number of times
 };
 
+// Shape of a multi-step 2D launch (axs_step_2d.cu): sites per lane, rows per
+// warp, warps, steps, tiles across and in all, and its estimated time.
+struct Plan2d {
+    int xs = 0, v = 0, nw = 0, k = 1, ntx = 0, ntiles = 0;
+    double us = 1e30;
+};
+
 struct Lattice {
     axs_params p{};
     int64_t length = 0;   // N^NDIMS
@@ -127,6 +134,8 @@ struct Lattice {
     // exchanged after every launch; the contents of scratch never outlive a call)
     void *scratch = nullptr;
     double *dclock = nullptr; // [2]
+    void *dstep2d = nullptr;  // 2D: [2] coefficient tables of the multi-step launches, one per clock slot
+    std::map<int, Plan2d> plans2d;   // 2D: the plan for at most so many steps
     int *derr = nullptr;      // device error flags
     int *dcounter = nullptr;  // [2] work counters of the persistent step kernel
     int cur = 0;              // psi[cur] holds the current field; dclock[cur] its tau
@@ -219,6 +228,12 @@ void lattice_autotune(Lattice *L);
 void ensemble_setup(Ensemble *E);
 void ensemble_evolve(Ensemble *E, int nsteps);
 void ensemble_autotune(Ensemble *E);
+// 2D steps, several per launch (axs_step_2d.cu): from psi[cur], pih and the
+// clock into psi[cur ^ 1], scratch and the other clock; returns the steps taken
+// (step2d_steps's answer for the same arguments, at most max_steps)
+constexpr int kStep2dSlot = 1024;   // bytes of one coefficient table
+int step2d_launch(Lattice *L, int max_steps);
+int step2d_steps(Lattice *L, int max_steps);
 // radius-R z-march kernels (axs_step_r.cu), by tile shape; zr = 1 keeps the
 // z-neighbours in registers with a ring of 2R + 2 or more slots
 void launch_zmarch_r(int esz, int ty, int txmax, int slots, int r, int zr, const ZLat *d, int nlat, int64_t items,

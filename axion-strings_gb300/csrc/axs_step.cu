@@ -101,9 +101,9 @@ __device__ __forceinline__ void stencil_at(const typename Cplx<T>::type *__restr
     L2 = a2;
 }
 
-// One step, one thread per site (grid-stride). Used for 2D, stencil radii
-// 2..4 and lattice shapes the z-march kernel does not tile.
-template <typename T, int ND, int R>
+// One 3D step, one thread per site (grid-stride). Used for lattice shapes the
+// z-march kernels do not tile, and where it is the fastest candidate.
+template <typename T, int R>
 __global__ void __launch_bounds__(256) k_step_generic(const typename Cplx<T>::type *__restrict__ psi,
                                                       typename Cplx<T>::type *__restrict__ out,
                                                       typename Cplx<T>::type *__restrict__ pih,
@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(256) k_step_generic(const typename Cplx<T>::ty
     double tau = *clock_in;
     StepCoefs<T> c = make_coefs<T>(tau, dt, dt, inv_dx2, lambda, T0sq3, prs, form);
     constexpr bool FOLD = sizeof(T) == 8 && R == 1;
+    constexpr int ND = 3;
     const T kctr = c.kdt_idx2 * (T)(-2 * ND);
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; m < len; m += stride) {
@@ -1958,7 +1959,7 @@ static int radius(const ZVariant &v) { return v.r > 0 ? v.r : 1; }
 
 std::string StepConfig::describe() const {
     char b[200];
-    if (kind == 0) snprintf(b, sizeof b, "generic per-site kernel");
+    if (kind == 0) snprintf(b, sizeof b, "generic per-site kernel");   // 2D: axs_step_2d.cu
     else if (two_step(variant))
         snprintf(b, sizeof b, "TMA z-march variant %d (two steps per pass, halo depth 2%s; odd step on variant %d), tx=%d, zchunk=%d",
                  variant, kZVariants[variant].lean ? ", lean" : "", kZVariants[variant].partner, tx, zchunk);
@@ -2485,13 +2486,13 @@ void step_release(Lattice *L) {
     L->dcounter = nullptr;
 }
 
-template <typename T, int ND, int R>
+template <typename T, int R>
 static void launch_generic_t(Lattice *L, const double *cin, double *cout) {
     typedef typename Cplx<T>::type C;
     const axs_params &p = L->p;
     double dx = p.space_step;
     double T0 = p.T_initial;
-    k_step_generic<T, ND, R><<<grid_for(L->length), 256, 0, L->stream>>>(
+    k_step_generic<T, R><<<grid_for(L->length), 256, 0, L->stream>>>(
         (const C *)L->psi[L->cur], (C *)L->psi[L->cur ^ 1], (C *)L->pih, cin, cout, p.N, L->length,
         (double)p.time_step, 1.0 / (dx * dx), (double)p.lambda, (T0 * T0) / 3.0, p.prs, p.stencil_setting, p.form);
     AXS_CUDA(cudaGetLastError());
@@ -2500,21 +2501,11 @@ static void launch_generic_t(Lattice *L, const double *cin, double *cout) {
 
 template <typename T>
 static void launch_generic_dispatch(Lattice *L, const double *cin, double *cout) {
-    int R = L->p.stencil_setting + 1;
-    if (L->p.NDIMS == 2) {
-        switch (R) {
-        case 1: launch_generic_t<T, 2, 1>(L, cin, cout); break;
-        case 2: launch_generic_t<T, 2, 2>(L, cin, cout); break;
-        case 3: launch_generic_t<T, 2, 3>(L, cin, cout); break;
-        default: launch_generic_t<T, 2, 4>(L, cin, cout); break;
-        }
-    } else {
-        switch (R) {
-        case 1: launch_generic_t<T, 3, 1>(L, cin, cout); break;
-        case 2: launch_generic_t<T, 3, 2>(L, cin, cout); break;
-        case 3: launch_generic_t<T, 3, 3>(L, cin, cout); break;
-        default: launch_generic_t<T, 3, 4>(L, cin, cout); break;
-        }
+    switch (L->p.stencil_setting + 1) {
+    case 1: launch_generic_t<T, 1>(L, cin, cout); break;
+    case 2: launch_generic_t<T, 2>(L, cin, cout); break;
+    case 3: launch_generic_t<T, 3>(L, cin, cout); break;
+    default: launch_generic_t<T, 4>(L, cin, cout); break;
     }
 }
 
@@ -2630,6 +2621,9 @@ int lattice_advance(Lattice *L, int max_steps) {
             L->debug_tx_excess = 0;
             L->zlat_variant = -1;
         }
+    } else if (L->p.NDIMS == 2) {
+        k = step2d_launch(L, max_steps);
+        swap = true;
     } else {
         if (L->esz == 4) launch_generic_dispatch<float>(L, cin, cout);
         else launch_generic_dispatch<double>(L, cin, cout);
@@ -2710,7 +2704,9 @@ void lattice_evolve(Lattice *L, int nsteps) {
         if (--nsteps == 0) return;
     }
     prepare_tables(L);
-    if (nsteps < 2 || !env_flag("AXS_GRAPHS", true) || L->p.laplacian == 1) {   // spectral: transforms run eagerly
+    // a graph only where it saves launches: not for one or two
+    const bool few = nsteps < 2 || (L->p.NDIMS == 2 && L->p.laplacian == 0 && nsteps <= 2 * step2d_steps(L, nsteps));
+    if (few || !env_flag("AXS_GRAPHS", true) || L->p.laplacian == 1) {   // spectral: transforms run eagerly
         while (nsteps > 0) nsteps -= lattice_advance(L, nsteps);
         return;
     }
@@ -2978,8 +2974,19 @@ static bool ensemble_table_valid(Ensemble *E) {
 // One launch over every member; returns the steps taken (see lattice_advance).
 static int ensemble_advance(Ensemble *E, int max_steps) {
     if (E->cfg.kind != 1) {
-        for (Lattice *m : E->members) lattice_advance(m, 1);
-        return 1;
+        // member by member; 2D members take several steps per launch, as many
+        // as the member with the fewest takes at once
+        int k = 1;
+        if (E->members[0]->p.NDIMS == 2 && E->members[0]->p.laplacian == 0) {
+            k = max_steps;
+            for (int k0 = 0; k0 != k;) {
+                k0 = k;
+                for (Lattice *m : E->members) k = std::min(k, step2d_steps(m, k));
+            }
+        }
+        for (Lattice *m : E->members)
+            if (lattice_advance(m, k) != k) fail(AXS_ERR_STATE, "internal: ensemble members advanced by different steps");
+        return k;
     }
     if (!ensemble_table_valid(E)) {
         if (t_capturing) fail(AXS_ERR_STATE, "internal: ensemble table rebuilt inside a graph capture");

@@ -1,0 +1,465 @@
+// 2D leapfrog steps, several per launch (temporal blocking): the 2D form of
+// vvsl_field_rescaled (src/standard/s_integrate.cpp:305-348).
+//
+// A 2D lattice is small: 512^2 fits L2, and one step per launch was bound by
+// the launch, the FP64 time coefficients that every thread formed and two
+// passes over the state, not by arithmetic. Here a block takes a tile through
+// k steps in registers:
+//  * it loads psi and pih over the tile plus a k R halo (periodic) once; lane i
+//    of a warp holds XS neighbouring sites of V rows, the warps lie above one
+//    another, and psi and pih stay in those registers for all k steps;
+//  * per step the x neighbours come by shuffles, the y neighbours from the
+//    thread's own rows, and only the first and last R rows of each warp go
+//    through shared memory (double-buffered: one barrier per step). With psi in
+//    a shared tile and every neighbour read from it a step of a row took twice
+//    as long (shared-memory wavefronts);
+//  * the region that is still right shrinks by R on each side per step (rows
+//    past it are skipped, columns past it carry values that nobody reads);
+//    after k steps the tile itself is written, psi and pih out of place (other
+//    tiles still read the old ones in their halos).
+// Each site goes through site_update / site_update_fold with one step's
+// coefficients, so k steps in one launch and k launches of one step give the
+// same bits.
+//
+// Measured (GB300, graph of launches, us per step): FP32 radius 1 at 128^2 /
+// 512^2 / 1500^2 / 4096^2: 0.58 / 1.03 / 4.9 / 34 with 10 / 6 / 6 / 6 steps
+// per launch, against 5 / 11 / 26 / 99 with one thread per site and one step per
+// launch; FP64 (bound by its FP64 pipe, 9 operations per site and step)
+// 1.8 / 7.2 / 49 / 340 against 6 / 17 / 70 / 520. A launch costs about 3 us
+// before its first step; it was 0.6 us more when every block formed the time
+// coefficients (FP64 divisions, one dependent chain): an extra block now forms
+// those of the next launch while the others step. Programmatic dependent
+// launch gained nothing (the next launch's blocks take slots from this one's).
+#include <algorithm>
+#include <cmath>
+
+#include "axs_internal.h"
+
+namespace axs {
+
+// Two floats in one 64-bit register pair: sm_100's packed FP32 operations
+// round each half as the scalar ones do.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 r;
+    asm("{.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 z, x, y;\n\t"
+        "mov.b64 {%0, %1}, z;}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 r;
+    asm("{.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+        "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
+
+struct Step2dArgs {
+    const void *psi;
+    void *psi_out;
+    const void *pih;
+    void *pih_out;
+    const double *clock_in;
+    double *clock_out;
+    const void *tab_in;  // Step2dTable<T>: the coefficients from the clock this launch starts at, if its tag says so
+    void *tab_out;       // those from the clock it ends at
+    int N, k;            // k steps in this launch
+    int ntx, ntiles;     // tiles across, tiles in all
+    double dt, inv_dx2, lambda, T0sq3;
+    int prs, form;
+};
+constexpr int kStep2dMaxK = 16;
+// The coefficients of the next steps, formed by an extra block of the launch
+// before. A table serves a launch only when its tag is the clock and the step
+// that launch reads (lambda, T0 and the rest are fixed for a lattice);
+// otherwise (a state just set, a resumed run) the launch's blocks form them.
+template <typename T>
+struct Step2dTable {
+    double tau, dt;
+    StepCoefs<T> c[kStep2dMaxK];
+    T kctr[kStep2dMaxK];
+};
+
+// One site's update from its neighbours (x pair and y pair at distances 1..R).
+template <typename T, int R>
+struct Site2d {
+    typedef typename Cplx<T>::type C;
+    StepCoefs<T> c;
+    T kctr;
+    __device__ __forceinline__ void update(C &a, C &p, const C (&xm)[R], const C (&xp)[R], const C (&ym)[R],
+                                           const C (&yp)[R]) const {
+        if constexpr (sizeof(T) == 4 && R == 1) {
+            const float2 s = add2(add2(xm[0], xp[0]), add2(ym[0], yp[0]));
+            const float2 L = fma2(make_float2(-4.f, -4.f), a, s);
+            const float r = fmaf(a.x, a.x, fmaf(a.y, a.y, c.c0)), g = c.kdt_coef * r;
+            p = fma2(make_float2(c.kdt_idx2, c.kdt_idx2), L, fma2(make_float2(g, g), a, p));
+            a = fma2(make_float2(c.dt, c.dt), p, a);
+        } else if constexpr (R == 1) {
+            const T S1 = nsum5<T>(xm[0].x, xp[0].x, ym[0].x, yp[0].x), S2 = nsum5<T>(xm[0].y, xp[0].y, ym[0].y, yp[0].y);
+            T an, bn;
+            site_update_fold<T>(a.x, a.y, S1, S2, p.x, p.y, an, bn, c, kctr);
+            a.x = an;
+            a.y = bn;
+        } else {
+            T a1 = (T)stencil_coef(R - 1, 2, 0) * a.x, a2 = (T)stencil_coef(R - 1, 2, 0) * a.y;
+#pragma unroll
+            for (int l = 0; l < R; ++l) {
+                const T w = (T)stencil_coef(R - 1, 2, l + 1);
+                a1 = fma(w, nsum5<T>(xm[l].x, xp[l].x, ym[l].x, yp[l].x), a1);
+                a2 = fma(w, nsum5<T>(xm[l].y, xp[l].y, ym[l].y, yp[l].y), a2);
+            }
+            T an, bn;
+            site_update<T>(a.x, a.y, a1, a2, p.x, p.y, an, bn, c);
+            a.x = an;
+            a.y = bn;
+        }
+    }
+};
+
+__device__ __forceinline__ float2 shfl_c(float2 v, int lane) {
+    return make_float2(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
+}
+__device__ __forceinline__ double2 shfl_c(double2 v, int lane) {
+    return make_double2(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
+}
+
+template <typename T, int XS>
+__device__ __forceinline__ void load_sites(const typename Cplx<T>::type *p, typename Cplx<T>::type (&v)[XS]) {
+    if constexpr (sizeof(T) == 4 && XS == 2) {
+        const float4 q = *reinterpret_cast<const float4 *>(p);
+        v[0] = make_float2(q.x, q.y);
+        v[1] = make_float2(q.z, q.w);
+    } else {
+#pragma unroll
+        for (int j = 0; j < XS; ++j) v[j] = p[j];
+    }
+}
+template <typename T, int XS>
+__device__ __forceinline__ void store_sites(typename Cplx<T>::type *p, const typename Cplx<T>::type (&v)[XS]) {
+    if constexpr (sizeof(T) == 4 && XS == 2) {
+        *reinterpret_cast<float4 *>(p) = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+    } else {
+#pragma unroll
+        for (int j = 0; j < XS; ++j) p[j] = v[j];
+    }
+}
+
+// XS sites per lane, V rows per warp; the block's warps (1 .. 16, at run time)
+// lie above one another. R <= V.
+template <typename T, int R, int XS, int V>
+__global__ void __launch_bounds__(V <= 2 ? 512 : 256) k_step2d(const Step2dArgs A) {
+    typedef typename Cplx<T>::type C;
+    static_assert(R <= V, "the halo rows come from the next warps");
+    constexpr int RX = 32 * XS;
+    constexpr int LN = (R + XS - 1) / XS;   // lanes to either side that hold x neighbours
+    extern __shared__ __align__(16) unsigned char smem[];
+    // the first and last R rows of each warp, two buffers: [2][warps][2R][RX]
+    C *edge = reinterpret_cast<C *>(smem);
+    __shared__ StepCoefs<T> coefs[kStep2dMaxK];
+    __shared__ T kctrs[kStep2dMaxK];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
+    const int x = XS * lane, y0 = w * V, RY = V * nw;
+    const int N = A.N, k = A.k, H = k * R, HX = (H + XS - 1) / XS * XS;
+    const int TX = RX - 2 * HX, TY = RY - 2 * H;
+    const C *psi = reinterpret_cast<const C *>(A.psi), *pih = reinterpret_cast<const C *>(A.pih);
+    C *po = reinterpret_cast<C *>(A.psi_out), *qo = reinterpret_cast<C *>(A.pih_out);
+    auto make = [&](double tau, int n, StepCoefs<T> &c, T &kc) {   // step n from tau, advanced as single steps advance it
+        for (int s = 0; s < n; ++s) tau = tau + A.dt;
+        c = make_coefs<T>(tau, A.dt, A.dt, A.inv_dx2, A.lambda, A.T0sq3, A.prs, A.form);
+        kc = sizeof(T) == 8 ? c.kdt_idx2 * (T)-4 : (T)0;
+    };
+    if (blockIdx.x == gridDim.x - 1) {   // the last block: the next clock and its table
+        if (tid < kStep2dMaxK) {
+            double tau = *A.clock_in;
+            for (int s = 0; s < k; ++s) tau = tau + A.dt;
+            Step2dTable<T> *t = reinterpret_cast<Step2dTable<T> *>(A.tab_out);
+            StepCoefs<T> c;
+            T kc;
+            make(tau, tid, c, kc);
+            t->c[tid] = c;
+            t->kctr[tid] = kc;
+            if (tid == 0) {
+                t->tau = tau;
+                t->dt = A.dt;
+                *A.clock_out = tau;
+            }
+        }
+        return;
+    }
+    if (tid < k) {
+        const Step2dTable<T> *t = reinterpret_cast<const Step2dTable<T> *>(A.tab_in);
+        const double tau = *A.clock_in;
+        const bool made = t->tau == tau && t->dt == A.dt;
+        StepCoefs<T> c = t->c[tid];
+        T kc = t->kctr[tid];
+        if (!made) make(tau, tid, c, kc);
+        coefs[tid] = c;
+        if (sizeof(T) == 8) kctrs[tid] = kc;
+    }
+    for (int tile = blockIdx.x; tile < A.ntiles; tile += gridDim.x - 1) {
+        const int ty = tile / A.ntx, gx0 = (tile - ty * A.ntx) * TX, gy0 = ty * TY;
+        int gx = (gx0 - HX + x) % N, gy = (gy0 - H + y0) % N;
+        if (gx < 0) gx += N;
+        if (gy < 0) gy += N;
+        C a[V][XS], p[V][XS];
+        {
+            int yy = gy;
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                const int o = yy * N + gx;
+                load_sites<T, XS>(psi + o, a[v]);
+                load_sites<T, XS>(pih + o, p[v]);
+                yy = yy + 1 == N ? 0 : yy + 1;
+            }
+        }
+        for (int s = 0; s < k; ++s) {
+            C *eb = edge + (s & 1) * nw * 2 * R * RX;
+#pragma unroll
+            for (int l = 0; l < R; ++l) {
+                store_sites<T, XS>(eb + (w * 2 * R + l) * RX + x, a[l]);
+                store_sites<T, XS>(eb + (w * 2 * R + R + l) * RX + x, a[V - R + l]);
+            }
+            __syncthreads();
+            Site2d<T, R> st;
+            st.c = coefs[s];
+            st.kctr = sizeof(T) == 8 ? kctrs[s] : (T)0;
+            const int lo = R * (s + 1), hi = RY - lo;   // rows with all their neighbours
+            C up[R][XS], dn[R][XS];   // rows y - 1 .. y - R before this step; rows past the warp's last
+            const int wu = max(w - 1, 0), wd = min(w + 1, nw - 1);
+#pragma unroll
+            for (int l = 0; l < R; ++l) {
+                load_sites<T, XS>(eb + (wu * 2 * R + 2 * R - 1 - l) * RX + x, up[l]);
+                load_sites<T, XS>(eb + (wd * 2 * R + l) * RX + x, dn[l]);
+            }
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                C old[XS];
+#pragma unroll
+                for (int j = 0; j < XS; ++j) old[j] = a[v][j];
+                const int y = y0 + v;
+                if (y >= lo && y < hi) {   // the same in the whole warp
+                    C win[XS + 2 * LN * XS];   // sites x - LN XS .. x + XS + LN XS - 1 of the row
+#pragma unroll
+                    for (int j = 0; j < XS; ++j) win[LN * XS + j] = old[j];
+#pragma unroll
+                    for (int n = 1; n <= LN; ++n)
+#pragma unroll
+                        for (int j = 0; j < XS; ++j) {
+                            if ((n - 1) * XS + XS - j <= R) win[(LN - n) * XS + j] = shfl_c(old[j], lane - n);
+                            if ((n - 1) * XS + j + 1 <= R) win[(LN + n) * XS + j] = shfl_c(old[j], lane + n);
+                        }
+#pragma unroll
+                    for (int j = 0; j < XS; ++j) {
+                        C xm[R], xp[R], ym[R], yp[R];
+#pragma unroll
+                        for (int l = 0; l < R; ++l) {
+                            xm[l] = win[LN * XS + j - 1 - l];
+                            xp[l] = win[LN * XS + j + 1 + l];
+                            ym[l] = up[l][j];
+                            yp[l] = v + 1 + l < V ? a[v + 1 + l < V ? v + 1 + l : 0][j] : dn[v + 1 + l < V ? 0 : v + 1 + l - V][j];
+                        }
+                        st.update(a[v][j], p[v][j], xm, xp, ym, yp);
+                    }
+                }
+#pragma unroll
+                for (int l = R - 1; l >= 0; --l)
+#pragma unroll
+                    for (int j = 0; j < XS; ++j) up[l][j] = l > 0 ? up[l > 0 ? l - 1 : 0][j] : old[j];
+            }
+        }
+        // the tile's sites inside the lattice
+        const int ox = gx0 + x - HX;
+        if (x >= HX && x < RX - HX && ox < N) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                const int y = y0 + v, oy = gy0 + y - H;
+                if (y >= H && y < RY - H && oy < N) {
+                    store_sites<T, XS>(po + oy * N + ox, a[v]);
+                    store_sites<T, XS>(qo + oy * N + ox, p[v]);
+                }
+            }
+        }
+        __syncthreads();   // the edge buffers are free for the next tile
+    }
+}
+
+// ---------------------------------------------------------------- dispatch
+//
+// The shape of a launch (sites per lane, rows per warp, warps, steps) follows
+// from a cost estimate over the shapes below, in SM cycles fitted to
+// measurements: a launch costs t0 plus a barrier's latency per step; an SM takes
+// ceil(tiles / SMs) tiles, each as many 32-site rows as its shrinking region
+// has over the steps, at the cost of a row (FP32 9 cycles at radius 1, FP64
+// 18.5 per FP64 operation); and the tiles' loads and stores go at L2's rate while
+// the state fits it, else HBM's. More steps per launch amortise t0 and the
+// memory traffic, and cost halo: at 128^2 ten to twelve steps per launch win
+// in FP32, at 1500^2 four to six, in FP64 one to four.
+struct Shape2d {
+    int xs, v, nwmin, nwmax, nwstep;
+};
+
+template <typename T, int R>
+static int shapes2d(const Shape2d *&s) {
+    static constexpr Shape2d f1[] = {{2, 2, 4, 8, 4}, {2, 4, 4, 8, 4}, {2, 8, 4, 8, 4}};
+    static constexpr Shape2d f2[] = {{2, 4, 4, 8, 4}, {2, 8, 4, 8, 4}};
+    static constexpr Shape2d f4[] = {{2, 4, 4, 8, 4}};
+    static constexpr Shape2d d1[] = {{1, 1, 4, 16, 1}, {1, 2, 3, 12, 1}, {1, 4, 4, 8, 1}};
+    static constexpr Shape2d d2[] = {{1, 2, 4, 12, 1}, {1, 4, 4, 8, 1}};
+    static constexpr Shape2d d4[] = {{1, 4, 4, 8, 1}};
+    if constexpr (sizeof(T) == 4) {
+        if constexpr (R == 1) { s = f1; return 3; }
+        else if constexpr (R == 2) { s = f2; return 2; }
+        else { s = f4; return 1; }
+    } else {
+        if constexpr (R == 1) { s = d1; return 3; }
+        else if constexpr (R == 2) { s = d2; return 2; }
+        else { s = d4; return 1; }
+    }
+}
+
+template <typename T, int R>
+static Plan2d plan2d_k(int N, int k, int sms) {
+    const Shape2d *sh = nullptr;
+    const int n = shapes2d<T, R>(sh);
+    const bool f32 = sizeof(T) == 4;
+    const double row = f32 ? 9.0 * (0.4 + 0.6 * R) : 18.5 * (R == 1 ? 9 : 11 + 2 * R);
+    const double ghz = 1.92, t0 = 3.0, step = f32 ? 0.12 : 0.5;
+    const double csz = 2.0 * sizeof(T);
+    const double bw = 4.0 * N * N * csz < 100e6 ? 10e6 : 6.5e6;   // bytes per us
+    Plan2d best;
+    for (int i = 0; i < n; ++i)
+        for (int nw = sh[i].nwmin; nw <= sh[i].nwmax; nw += sh[i].nwstep) {
+            const int rx = 32 * sh[i].xs, ry = sh[i].v * nw, h = k * R, hx = (h + sh[i].xs - 1) / sh[i].xs * sh[i].xs;
+            const int tx = rx - 2 * hx, ty = ry - 2 * h;
+            if (tx < 8 || ty < 2) continue;
+            const int ntx = (N + tx - 1) / tx;
+            const double tiles = (double)ntx * ((N + ty - 1) / ty);
+            const double rows = (double)k * ry - R * (double)k * (k + 1);   // sum of ry - 2 R s
+            const double per_sm = tiles / sms <= 8.0 ? std::ceil(tiles / sms) : tiles / sms;
+            const double us = t0 + step * k + per_sm * rows * sh[i].xs * row / (ghz * 1e3) +
+                              tiles * ((double)rx * ry + (double)tx * ty) * 2.0 * csz / bw;
+            if (us < best.us) {
+                best.xs = sh[i].xs;
+                best.v = sh[i].v;
+                best.nw = nw;
+                best.k = k;
+                best.ntx = ntx;
+                best.ntiles = (int)tiles;
+                best.us = us;
+            }
+        }
+    return best;
+}
+
+// The plan for at most max_steps steps of a lattice: the steps per launch with
+// the least estimated time per step, the launches of an interval evened out.
+template <typename T, int R>
+static Plan2d plan2d(int N, int max_steps) {
+    const int sms = num_sms();
+    Plan2d best;
+    for (int k = 1; k <= std::min(12, max_steps); ++k) {
+        const Plan2d p = plan2d_k<T, R>(N, k, sms);
+        if (p.nw && p.us / k < best.us / best.k) best = p;
+    }
+    const int launches = (max_steps + best.k - 1) / best.k, k = (max_steps + launches - 1) / launches;
+    return k == best.k ? best : plan2d_k<T, R>(N, k, sms);
+}
+
+template <typename T, int R, int XS, int V>
+static void launch2d_t(const Step2dArgs &a, int nw, cudaStream_t st) {
+    typedef typename Cplx<T>::type C;
+    const int smem = 2 * nw * 2 * R * 32 * XS * (int)sizeof(C);
+    constexpr int smax = 2 * (V <= 2 ? 16 : 8) * 2 * R * 32 * XS * (int)sizeof(C);
+    static PerDevice ready;   // the kernel's shared-memory attribute belongs to the device
+    ready.get([] {
+        AXS_CUDA(cudaFuncSetAttribute(k_step2d<T, R, XS, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
+        return 1;
+    });
+    static PerDevice occ[17];
+    const int per = occ[nw].get([nw, smem] {
+        int o = 0;
+        AXS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_step2d<T, R, XS, V>, 32 * nw, smem));
+        return std::max(1, o);
+    });
+    const int grid = (int)std::min<int64_t>(a.ntiles, (int64_t)per * num_sms()) + 1;   // and the next launch's coefficients
+    k_step2d<T, R, XS, V><<<grid, 32 * nw, smem, st>>>(a);
+    AXS_CUDA(cudaGetLastError());
+    count_launches(1);
+}
+
+template <typename T, int R>
+static void launch2d(const Step2dArgs &a, const Plan2d &p, cudaStream_t st) {
+    if constexpr (sizeof(T) == 4) {
+        if constexpr (R == 1)
+            if (p.v == 2) return launch2d_t<T, R, 2, 2>(a, p.nw, st);
+        if constexpr (R <= 2)
+            if (p.v == 8) return launch2d_t<T, R, 2, 8>(a, p.nw, st);
+        launch2d_t<T, R, 2, 4>(a, p.nw, st);
+    } else {
+        if constexpr (R == 1)
+            if (p.v == 1) return launch2d_t<T, R, 1, 1>(a, p.nw, st);
+        if constexpr (R <= 2)
+            if (p.v == 2) return launch2d_t<T, R, 1, 2>(a, p.nw, st);
+        launch2d_t<T, R, 1, 4>(a, p.nw, st);
+    }
+}
+
+template <typename T, int R>
+static int step2d_t(Lattice *L, int max_steps, bool launch) {
+    const axs_params &p = L->p;
+    auto it = L->plans2d.find(max_steps);
+    if (it == L->plans2d.end()) {
+        if (L->plans2d.size() >= 64) L->plans2d.clear();
+        it = L->plans2d.emplace(max_steps, plan2d<T, R>(p.N, max_steps)).first;
+    }
+    const Plan2d pl = it->second;
+    if (!launch) return pl.k;
+    const double dx = p.space_step, T0 = p.T_initial;
+    Step2dArgs a;
+    a.psi = L->psi[L->cur];
+    a.psi_out = L->psi[L->cur ^ 1];
+    a.pih = L->pih;
+    a.pih_out = L->scratch;
+    a.clock_in = L->dclock + L->cur;
+    a.clock_out = L->dclock + (L->cur ^ 1);
+    a.tab_in = (const char *)L->dstep2d + L->cur * kStep2dSlot;
+    a.tab_out = (char *)L->dstep2d + (L->cur ^ 1) * kStep2dSlot;
+    a.N = p.N;
+    a.k = pl.k;
+    a.ntx = pl.ntx;
+    a.ntiles = pl.ntiles;
+    a.dt = (double)p.time_step;
+    a.inv_dx2 = 1.0 / (dx * dx);
+    a.lambda = (double)p.lambda;
+    a.T0sq3 = (T0 * T0) / 3.0;
+    a.prs = p.prs;
+    a.form = p.form;
+    launch2d<T, R>(a, pl, L->stream);
+    return pl.k;
+}
+
+static int step2d(Lattice *L, int max_steps, bool launch) {
+    static_assert(sizeof(Step2dTable<double>) <= kStep2dSlot, "a slot holds a table");
+    const int R = L->p.stencil_setting + 1;
+    if (L->esz == 4) {
+        switch (R) {
+        case 1: return step2d_t<float, 1>(L, max_steps, launch);
+        case 2: return step2d_t<float, 2>(L, max_steps, launch);
+        case 3: return step2d_t<float, 3>(L, max_steps, launch);
+        default: return step2d_t<float, 4>(L, max_steps, launch);
+        }
+    }
+    switch (R) {
+    case 1: return step2d_t<double, 1>(L, max_steps, launch);
+    case 2: return step2d_t<double, 2>(L, max_steps, launch);
+    case 3: return step2d_t<double, 3>(L, max_steps, launch);
+    default: return step2d_t<double, 4>(L, max_steps, launch);
+    }
+}
+
+int step2d_launch(Lattice *L, int max_steps) { return step2d(L, max_steps, true); }
+int step2d_steps(Lattice *L, int max_steps) { return step2d(L, max_steps, false); }
+
+}  // namespace axs
