@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(256) k_zmarch(const ZLat *__restrict__ lats, i
         const int64_t local = item - Lt.item_base;
         const int ncols = ntx * nty;
         const int zq = (int)(local / ncols), col = (int)(local % ncols);
-        const int x0 = (col % ntx) * tx, y0 = (col / ntx) * TY;
+        const int x0 = min((col % ntx) * tx, N - tx), y0 = min((col / ntx) * TY, N - TY);
         const int za = (int)((int64_t)zq * N / nzc), zb = (int)((int64_t)(zq + 1) * N / nzc);
         const int T_steps = zb - za;
         const int nload = T_steps + 2;
@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(Z2Cfg<T, TY, TXMAX, S>::NT)
                 const int64_t local = item - Lt.item_base;
                 const int ncols = ntx * nty;
                 const int zq = (int)(local / ncols), col = (int)(local % ncols);
-                const int x0 = (col % ntx) * tx, y0 = (col / ntx) * TY;
+                const int x0 = min((col % ntx) * tx, N - tx), y0 = min((col / ntx) * TY, N - TY);
                 const int za = (int)((int64_t)zq * N / nzc), zb = (int)((int64_t)(zq + 1) * N / nzc);
                 const int nload = zb - za + 2;
                 const int bin = Lt.a_index ^ parity;
@@ -740,7 +740,7 @@ __global__ void __launch_bounds__(Z2Cfg<T, TY, TXMAX, S>::NT)
             const int64_t local = item - Lt.item_base;
             const int ncols = ntx * nty;
             const int zq = (int)(local / ncols), col = (int)(local % ncols);
-            const int x0 = (col % ntx) * tx, y0 = (col / ntx) * TY;
+            const int x0 = min((col % ntx) * tx, N - tx), y0 = min((col / ntx) * TY, N - TY);
             const int za = (int)((int64_t)zq * N / nzc), zb = (int)((int64_t)(zq + 1) * N / nzc);
             const int T_steps = zb - za;
             const int bin = Lt.a_index ^ parity;
@@ -990,7 +990,7 @@ __device__ __forceinline__ void zmarch_2step_body(const ZLat *__restrict__ lats,
                 const int64_t local = item - Lt.item_base;
                 const int ncols = ntx * nty;
                 const int zq = (int)(local / ncols), col = (int)(local % ncols);
-                const int x0 = (col % ntx) * tx, y0 = (col / ntx) * TY;
+                const int x0 = min((col % ntx) * tx, N - tx), y0 = min((col / ntx) * TY, N - TY);
                 const int za = (int)((int64_t)zq * N / nzc), zb = (int)((int64_t)(zq + 1) * N / nzc);
                 const int nload = zb - za + 4;
                 const int bin = Lt.a_index ^ parity;
@@ -1071,7 +1071,7 @@ __device__ __forceinline__ void zmarch_2step_body(const ZLat *__restrict__ lats,
             const int64_t local = item - Lt.item_base;
             const int ncols = ntx * nty;
             const int zq = (int)(local / ncols), col = (int)(local % ncols);
-            const int x0 = (col % ntx) * tx, y0 = (col / ntx) * TY;
+            const int x0 = min((col % ntx) * tx, N - tx), y0 = min((col / ntx) * TY, N - TY);
             const int za = (int)((int64_t)zq * N / nzc), zb = (int)((int64_t)(zq + 1) * N / nzc);
             const int T_steps = zb - za;
             const int bin = Lt.a_index ^ parity;
@@ -1469,7 +1469,7 @@ __device__ __forceinline__ void zmarch_3step_body(const ZLat *__restrict__ lats,
                 const int64_t local = item - Lt.item_base;
                 const int ncols = ntx * nty;
                 const int zq = (int)(local / ncols), col = (int)(local % ncols);
-                const int x0 = (col % ntx) * tx, y0 = (col / ntx) * TY;
+                const int x0 = min((col % ntx) * tx, N - tx), y0 = min((col / ntx) * TY, N - TY);
                 const int za = (int)((int64_t)zq * N / nzc), zb = (int)((int64_t)(zq + 1) * N / nzc);
                 const int nload = zb - za + 6;   // psi_n planes za-3 .. zb+2
                 const int bin = Lt.a_index ^ parity;
@@ -1551,7 +1551,7 @@ __device__ __forceinline__ void zmarch_3step_body(const ZLat *__restrict__ lats,
             const int64_t local = item - Lt.item_base;
             const int ncols = ntx * nty;
             const int zq = (int)(local / ncols), col = (int)(local % ncols);
-            const int x0 = (col % ntx) * tx, y0 = (col / ntx) * TY;
+            const int x0 = min((col % ntx) * tx, N - tx), y0 = min((col / ntx) * TY, N - TY);
             const int za = (int)((int64_t)zq * N / nzc), zb = (int)((int64_t)(zq + 1) * N / nzc);
             const int T_steps = zb - za;
             const int bin = Lt.a_index ^ parity;
@@ -1952,8 +1952,17 @@ static const int kNumZVariants = sizeof(kZVariants) / sizeof(kZVariants[0]);
 
 static bool two_step(int variant) { return variant >= 0 && variant < kNumZVariants && kZVariants[variant].gen == 3; }
 static bool three_step(int variant) { return variant >= 0 && variant < kNumZVariants && kZVariants[variant].gen == 5; }
+static int variant_tx(const ZVariant &v, int N, int esz);
+// the variant's tiles do not divide N: the last ones overlap their neighbours (variant_tx)
+static bool overlapped(const ZVariant &v, int N, int esz) {
+    const int tx = variant_tx(v, N, esz);
+    return tx > 0 && (N % tx != 0 || N % v.ty != 0);
+}
 // the momentum is written out of place (pih and scratch exchange after every launch)
-static bool out_of_place(int variant) { return two_step(variant) || three_step(variant); }
+static bool out_of_place(int variant, const Lattice *L) {
+    return two_step(variant) || three_step(variant) ||
+           (variant >= 0 && variant < kNumZVariants && overlapped(kZVariants[variant], L->p.N, L->esz));
+}
 static int steps_per_pass(int variant) { return three_step(variant) ? 3 : (two_step(variant) ? 2 : 1); }
 static int radius(const ZVariant &v) { return v.r > 0 ? v.r : 1; }
 
@@ -2294,39 +2303,60 @@ static int max_smem_optin() {
     });
 }
 
-// The tx a variant would use for an N (largest admissible divisor), or 0.
-static int variant_tx(const ZVariant &v, int N, int esz) {
-    if (v.gen == 5) {
-        // complex float, x-tiled (the kernel takes its x halo from strips), and
-        // the two-step partner tiles N the same way
-        if (esz != 4 || variant_smem(v, esz) > max_smem_optin() || v.ty < 3) return 0;
-        const ZVariant &pv = kZVariants[v.partner];
-        int tx = variant_tx(pv, N, esz);
-        if (!tx || pv.ty != v.ty || tx > v.txmax || tx >= N || tx < 4) return 0;
-        return tx;
-    }
+static int variant_txmax(const ZVariant &v, int esz) {
+    return esz == 8 ? std::min(v.txmax, 128) : v.txmax;   // box inner dim: 2*tx doubles <= 256
+}
+// The largest admissible tx that divides an N whose rows ty divides, or 0.
+static int exact_tx(const ZVariant &v, int N, int esz) {
+    const int unit = 128 / (2 * esz);   // shared-memory destinations stay 128-byte aligned
     if (v.gen == 3) {
-        // complex float only; the partner must tile N the same way
-        if (esz != 4 || variant_smem(v, esz) > max_smem_optin()) return 0;
         const ZVariant &pv = kZVariants[v.partner];
-        int tx = variant_tx(pv, N, esz);
-        if (!tx || pv.ty != v.ty || tx > v.txmax || N < 4) return 0;
-        return tx;
+        const int tx = exact_tx(pv, N, esz);
+        return esz == 4 && pv.ty == v.ty && tx <= v.txmax && variant_smem(v, esz) <= max_smem_optin() ? tx : 0;
     }
-    int cs = 2 * esz;
-    int vs = 16 / cs;
-    int txmax = v.txmax;
-    if (esz == 8) txmax = std::min(txmax, 128);   // box inner dim: 2*tx doubles <= 256
     if (variant_smem(v, esz) > max_smem_optin()) return 0;
     if (N % v.ty != 0 || N < 4 || v.ty < radius(v)) return 0;
     if (v.gen == 4 && (v.lean || v.slots < 2 * v.r + 2) && esz != 4) return 0;   // register z-ring: float fields only
-    for (int tx = std::min(txmax, N); tx >= vs; --tx) {
-        if (N % tx) continue;
-        if (tx % vs) continue;
-        if ((tx * cs) % 128) continue;   // shared-memory destinations stay 128-byte aligned
-        return tx;
-    }
+    for (int tx = std::min(variant_txmax(v, esz), N) / unit * unit; tx >= unit; tx -= unit)
+        if (N % tx == 0) return tx;
     return 0;
+}
+
+// The tx a variant uses for an N, or 0 when it does not serve it.
+//
+// A CTA's time per tile is that of its widest tile whatever tx is, so tx is
+// chosen for the fewest tiles across: a divisor of N where one gives that
+// number, else the smallest admissible width that does, and the last tile of a
+// row (and of a column, where ty does not divide N) starts at N - tx (N - ty)
+// and overlaps the one before: both compute the shared sites from the same
+// inputs and store the same bits. The momentum then goes out of place, so that
+// neither tile reads what the other has stored. (At 250^3 FP32 the two-step
+// kernel on overlapping tiles takes 50 us per step, one thread per site
+// took 135.) Every halo box must still lie wholly on one side of the
+// periodic edge: boxes are R rows or R sites (rounded up to 16 bytes) wide
+// and start at multiples of 2, so any N serves R <= 2, multiples of 4 the rest.
+static int variant_tx(const ZVariant &v, int N, int esz) {
+    if (v.gen == 5) {
+        // complex float, x-tiled (the kernel takes its x halo from strips),
+        // without overlap (its halo boxes are three rows high)
+        if (esz != 4 || variant_smem(v, esz) > max_smem_optin() || v.ty < 3) return 0;
+        const int tx = exact_tx(kZVariants[v.partner], N, esz);
+        return tx >= 4 && tx <= v.txmax && tx < N ? tx : 0;
+    }
+    if (v.gen == 3) {   // complex float only; the partner tiles N the same way (same widths, same rows)
+        if (esz != 4 || variant_smem(v, esz) > max_smem_optin()) return 0;
+        const ZVariant &pv = kZVariants[v.partner];
+        const int tx = variant_tx(pv, N, esz);
+        return tx && pv.ty == v.ty && tx <= v.txmax ? tx : 0;
+    }
+    const int exact = exact_tx(v, N, esz), unit = 128 / (2 * esz), txmax = variant_txmax(v, esz);
+    if (variant_smem(v, esz) > max_smem_optin() || N < std::max(unit, v.ty) || v.ty < radius(v)) return exact;
+    if (v.gen == 4 && (v.lean || v.slots < 2 * v.r + 2) && esz != 4) return 0;   // register z-ring: float fields only
+    const int fewest = (N + txmax - 1) / txmax;
+    if ((exact && N / exact == fewest) || (radius(v) > 2 && N % 4 != 0)) return exact;
+    const int tx = ((N + fewest - 1) / fewest + unit - 1) / unit * unit;
+    if (tx <= N) return tx;
+    return exact ? exact : N / unit * unit;   // N just above a multiple of the unit
 }
 
 // A variant serves a lattice when its stencil radius is the lattice's and it tiles N.
@@ -2373,17 +2403,17 @@ static void encode_map(CUtensorMap *m, void *base, int N, int esz, int box_x_sit
 // Fill the z-march table entry of lattice L for a variant; returns items.
 // a_index: the psi buffer that launch parity 0 treats as current. The entry's
 // pih[b] is the momentum buffer that goes with psi[b]: L->pih for the current
-// psi, and for a two-step variant L->scratch for the other one (the momentum
-// is then written out of place and the host exchanges pih and scratch after
-// every launch); one-step variants update the momentum in place.
+// psi, and for a two-step variant or overlapping tiles L->scratch for the other
+// one (the momentum is then written out of place and the host exchanges pih and
+// scratch after every launch); other one-step variants update it in place.
 static int64_t fill_zlat(ZLat &z, Lattice *L, int variant, int zchunk, int64_t item_base, int a_index) {
     const ZVariant &v = kZVariants[variant];
     int N = L->p.N;
     int tx = variant_tx(v, N, L->esz);
     if (!tx) fail(AXS_ERR_ARG, "z-march variant %d cannot tile N=%d", variant, N);
     prepare_zmarch(L->esz, variant);
-    const bool oop = v.gen == 3 || v.gen == 5;
-    if (oop && (!L->scratch || L->scratch == L->pih)) fail(AXS_ERR_STATE, "multi-step variant without a second momentum buffer");
+    const bool oop = out_of_place(variant, L), multi = v.gen == 3 || v.gen == 5;
+    if (oop && (!L->scratch || L->scratch == L->pih)) fail(AXS_ERR_STATE, "out-of-place variant without a second momentum buffer");
     memset(&z, 0, sizeof z);
     int vs = 16 / (2 * L->esz);
     const int R = radius(v);
@@ -2396,7 +2426,7 @@ static int64_t fill_zlat(ZLat &z, Lattice *L, int variant, int zchunk, int64_t i
         encode_map(&z.tm_main[b], L->psi[b], N, L->esz, tx, v.ty);
         encode_map(&z.tm_xh[b], L->psi[b], N, L->esz, rp, v.ty);   // x-halo strip
         encode_map(&z.tm_pih[b], pb[b], N, L->esz, tx, v.ty);
-        if (oop) {   // the two-step kernel's maps (a three-step variant's partner)
+        if (multi) {   // the two-step kernel's maps (a three-step variant's partner)
             encode_map(&z.t2_row2[b], L->psi[b], N, L->esz, tx, 2);
             encode_map(&z.t2_str2[b], L->psi[b], N, L->esz, vs, 2);
             encode_map(&z.t2_prow[b], pb[b], N, L->esz, tx, 1);
@@ -2415,8 +2445,8 @@ static int64_t fill_zlat(ZLat &z, Lattice *L, int variant, int zchunk, int64_t i
     z.clock = L->dclock;
     z.N = N;
     z.tx = tx;
-    z.ntx = N / tx;
-    z.nty = N / v.ty;
+    z.ntx = (N + tx - 1) / tx;
+    z.nty = (N + v.ty - 1) / v.ty;
     z.nzc = std::max(1, N / std::max(1, zchunk));
     z.a_index = a_index;
     z.item_base = item_base;
@@ -2454,7 +2484,7 @@ static void ensure_single_table(Lattice *L) {
 static bool single_table_valid(const Lattice *L) {
     if (!L->dzlat || L->zlat_variant != L->cfg.variant || L->zlat_zchunk != L->cfg.zchunk) return false;
     if (L->zlat_pih[L->cur] != L->pih) return false;
-    return out_of_place(L->cfg.variant) ? L->zlat_pih[L->cur ^ 1] == L->scratch : L->zlat_pih[L->cur ^ 1] == L->pih;
+    return out_of_place(L->cfg.variant, L) ? L->zlat_pih[L->cur ^ 1] == L->scratch : L->zlat_pih[L->cur ^ 1] == L->pih;
 }
 
 void step_setup(Lattice *L) {
@@ -2606,13 +2636,12 @@ int lattice_advance(Lattice *L, int max_steps) {
     } else if (L->cfg.kind == 1) {
         if (!single_table_valid(L)) ensure_single_table(L);
         int kv = L->cfg.variant;
+        swap = out_of_place(kv, L);
         if (three_step(kv)) {   // an interval's last one or two steps run on the partners
-            swap = true;
             if (max_steps >= 3) k = 3;
             else kv = kZVariants[kv].partner;
         }
         if (two_step(kv)) {
-            swap = true;
             if (max_steps >= 2) k = 2;
             else kv = kZVariants[kv].partner;
         }
@@ -2849,7 +2878,7 @@ void lattice_autotune(Lattice *L) {
     }
     const int zchunks[] = {32, 64, 128, 256};
     auto trial = [&](int v, int zc, int nrep, int nwarm) {
-        const bool two = out_of_place(v);
+        const bool oop = out_of_place(v, L);
         StepConfig c;
         c.kind = 1;
         c.variant = v;
@@ -2859,7 +2888,7 @@ void lattice_autotune(Lattice *L) {
         double ms = time_launches(L->stream, nrep, [&] {
             launch_zmarch(L->esz, v, L->dzlat, 1, L->zitems, L->dcounter, L->cur, L->derr, L->stream, 0);
             L->cur ^= 1;
-            if (two) std::swap(L->pih, L->scratch);
+            if (oop) std::swap(L->pih, L->scratch);
         }, nwarm);
         ms /= steps_per_pass(v);   // per step
         c.tx = L->cfg.tx;
@@ -2961,12 +2990,12 @@ static bool ensemble_table_valid(Ensemble *E) {
     // every member must sit at the same parity relative to its entry, with the
     // momentum buffer the entry expects
     const int d = ensemble_parity(E);
-    const bool two = two_step(E->cfg.variant);
     for (size_t i = 0; i < E->members.size(); ++i) {
         const Lattice *m = E->members[i];
+        const bool oop = out_of_place(E->cfg.variant, m);
         if ((m->cur ^ E->tab_cur[i]) != d) return false;
         if (E->tab_pih[2 * i + m->cur] != m->pih) return false;
-        if (E->tab_pih[2 * i + (m->cur ^ 1)] != (two ? m->scratch : m->pih)) return false;
+        if (E->tab_pih[2 * i + (m->cur ^ 1)] != (oop ? m->scratch : m->pih)) return false;
     }
     return true;
 }
@@ -2993,8 +3022,7 @@ static int ensemble_advance(Ensemble *E, int max_steps) {
         ensemble_table(E, 0.f, false);
     }
     int kv = E->cfg.variant, k = 1;
-    const bool two = two_step(kv);
-    if (two) {
+    if (two_step(kv)) {
         if (max_steps >= 2) k = 2;
         else kv = kZVariants[kv].partner;
     }
@@ -3002,7 +3030,7 @@ static int ensemble_advance(Ensemble *E, int max_steps) {
                   E->derr, E->stream, E->cfg.ctas_per_sm);
     for (Lattice *m : E->members) {
         m->cur ^= 1;
-        if (two) std::swap(m->pih, m->scratch);
+        if (out_of_place(E->cfg.variant, m)) std::swap(m->pih, m->scratch);
         for (int s = 0; s < k; ++s) m->tau = m->tau + (double)m->p.time_step;
         m->steps += k;
     }
@@ -3055,7 +3083,7 @@ void ensemble_autotune(Ensemble *E) {
                               ensemble_parity(E), E->derr, E->stream, 0);
                 for (Lattice *m : E->members) {
                     m->cur ^= 1;
-                    if (two) std::swap(m->pih, m->scratch);
+                    if (out_of_place(v, m)) std::swap(m->pih, m->scratch);
                 }
             });
             if (two) ms *= 0.5;   // per step

@@ -99,7 +99,7 @@ __device__ __forceinline__ void zmarch2r_body(const ZLat *__restrict__ lats, int
                 const int64_t local = item - Lt.item_base;
                 const int ncols = ntx * nty;
                 const int zq = (int)(local / ncols), col = (int)(local % ncols);
-                const int x0 = (col % ntx) * tx, y0 = (col / ntx) * TY;
+                const int x0 = min((col % ntx) * tx, N - tx), y0 = min((col / ntx) * TY, N - TY);
                 const int za = (int)((int64_t)zq * N / nzc), zb = (int)((int64_t)(zq + 1) * N / nzc);
                 const int nload = zb - za + 2 * R;
                 const int bin = Lt.a_index ^ parity;
@@ -166,7 +166,7 @@ __device__ __forceinline__ void zmarch2r_body(const ZLat *__restrict__ lats, int
             const int64_t local = item - Lt.item_base;
             const int ncols = ntx * nty;
             const int zq = (int)(local / ncols), col = (int)(local % ncols);
-            const int x0 = (col % ntx) * tx, y0 = (col / ntx) * TY;
+            const int x0 = min((col % ntx) * tx, N - tx), y0 = min((col / ntx) * TY, N - TY);
             const int za = (int)((int64_t)zq * N / nzc), zb = (int)((int64_t)(zq + 1) * N / nzc);
             const int T_steps = zb - za;
             const int bin = Lt.a_index ^ parity;
