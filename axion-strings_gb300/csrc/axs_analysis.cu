@@ -1293,8 +1293,8 @@ __global__ void k_gather_axion(const typename Cplx<T>::type *__restrict__ psi, c
 // the energies for radius 2..4)
 //
 // f = |phi| dtheta/dtau = (psi2 pi1 - psi1 pi2) / (tau |psi|) and the energies
-// need pi_n = pih + dt/2 K(psi), formed per site with k_sync_pi's arithmetic
-// (stencil_at's order) and never stored. A block marches 32 x 8 columns
+// need pi_n = pih + dt/2 K(psi), formed per site by sync_pi_site
+// (stencil_at's order). A block marches 32 x 8 columns
 // through z with every load from DRAM staged by cp.async into shared memory,
 // so the loads in flight hold no registers:
 // per plane, the block's psi tile with an R-wide periodic halo (the in-plane
@@ -1365,7 +1365,7 @@ struct ZStage {
 
 // The radius-R stencil sums of a column's site in plane z, in stencil_at's
 // order (coefficient 0 times the centre; per distance l the x pair plus the y
-// pair, plus the z pair, added with one fma), so pi_n keeps k_sync_pi's bits.
+// pair, plus the z pair, added with one fma), so every kernel forms the same pi_n.
 // t points at the site in its plane tile (row length TW); the column's plane
 // z + d is zr[(g + d) % W].
 template <typename T, int R, int W, int TW>
@@ -1393,15 +1393,16 @@ __device__ __forceinline__ void tile_stencil(const typename Cplx<T>::type *t, co
     L2 = a2;
 }
 
-// The march itself, shared by the radius-R axion field and energies: for
-// each site of the thread's column (threads past the lattice's edge take part
-// in the staging and barriers only) it forms pi_n with k_sync_pi's
-// arithmetic and calls site(h, z, zc, zp, p, t): the site's psi, psi of plane
-// z + 1, pi_n and its place in the staged tile. The register ring holds
-// planes z-R-1 .. z+R at site z; plane z+R+1 replaces plane z-R-1 from the
-// staged tile, so the ring has period W and the march runs W sites per trip
-// (no register moves). N > 2R and A <= 2R + 2 <= N, so a plane index past
-// the end wraps with one subtraction.
+// The march itself, shared by the radius-R axion field, energies and
+// synchronised momentum: for
+// each site of the thread's column in the block's z-chunk (threads past the
+// lattice's edge take part in the staging and barriers only) it forms pi_n with
+// sync_pi_site and calls site(h, z, zc, zp, p, t): the site's psi,
+// psi of plane z + 1, pi_n and its place in the staged tile. The register ring
+// holds planes z-R-1 .. z+R at site z; plane z+R+1 replaces plane z-R-1 from
+// the staged tile, so the ring has period W and the march runs W sites per trip
+// (no register moves). Block (c, q) takes columns c and z-chunk q of gridDim.y;
+// chunks are whole z-pairs (N is even), so sites pair up within a chunk.
 template <typename T, int R, class Site>
 __device__ __forceinline__ void zcol_march(const typename Cplx<T>::type *__restrict__ psi,
                                            const typename Cplx<T>::type *__restrict__ pih, int N, int fresh,
@@ -1413,32 +1414,37 @@ __device__ __forceinline__ void zcol_march(const typename Cplx<T>::type *__restr
     C *tiles = reinterpret_cast<C *>(zsm), *pown = tiles + S * M::E;
     const int nbx = (N + 31) / 32, bx0 = (int)(blockIdx.x % nbx) * 32, by0 = (int)(blockIdx.x / nbx) * 8;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, x = bx0 + tx, y = by0 + ty;
+    const int za = 2 * (int)((int64_t)blockIdx.y * (N / 2) / gridDim.y);
+    const int zb = 2 * (int)((int64_t)(blockIdx.y + 1) * (N / 2) / gridDim.y);
     const bool active = x < N && y < N;
     const int col = active ? y * N + x : 0;
     const ZStage<T, R> st(bx0, by0, N);
-    const int64_t NN = (int64_t)N * N, len = NN * N;
+    const int64_t NN = (int64_t)N * N;
 #pragma unroll
     for (int a = 0; a < A; ++a) {
-        st.issue(psi, pih, a * NN, a, tiles, pown, active, col);
+        st.issue(psi, pih, (int64_t)((za + a) % N) * NN, a, tiles, pown, active, col);
         cp_async_commit();
     }
     C zr[W];   // at a trip's start z0: zr[j] = plane z0 - R - 1 + j
 #pragma unroll
-    for (int j = 1; j < W; ++j) zr[j] = psi[(int64_t)(j <= R ? j - R - 1 + N : j - R - 1) * NN + col];
-    zr[0] = zr[1];   // plane -R-1 is never read
+    for (int j = 1; j < W; ++j) zr[j] = psi[(int64_t)((za + N + j - R - 1) % N) * NN + col];
+    zr[0] = zr[1];   // plane za-R-1 is never read
     const int cidx = (ty + R) * M::TW + tx + M::RX;
     int slot = 0, rslot = R + 1;   // ring slots of planes z and z + R + 1
-    int64_t pa = A * NN;
-    for (int z0 = 0; z0 < N; z0 += W) {
+    int pl = (za + A) % N;         // the plane to stage next, and its offset
+    int64_t po = pl * NN;
+    for (int z0 = za; z0 < zb; z0 += W) {
 #pragma unroll
         for (int h = 0; h < W; ++h) {
             const int z = z0 + h;
-            if (z < N) {   // uniform over the block
+            if (z < zb) {   // uniform over the block
                 cp_async_wait<A - R - 2>();   // this thread's copies of planes <= z + R + 1 are in
                 __syncthreads();              // everyone's are; slot (z - 1) is no longer read
-                st.issue(psi, pih, z + A < N ? pa : pa - len, slot == 0 ? A : slot - 1, tiles, pown, active, col);
+                st.issue(psi, pih, po, slot == 0 ? A : slot - 1, tiles, pown, active, col);
                 cp_async_commit();
-                pa += NN;
+                ++pl;
+                po += NN;
+                if (pl == N) pl = 0, po = 0;
                 if (active) {
                     const C *ts = tiles + slot * M::E + cidx;
                     zr[h] = tiles[rslot * M::E + cidx];   // plane z + R + 1 over plane z - R - 1
@@ -1459,9 +1465,149 @@ __device__ __forceinline__ void zcol_march(const typename Cplx<T>::type *__restr
     cp_async_wait<0>();
 }
 
+// The grid of the staged marches: blocks of 32 x 8 columns, and as many
+// z-chunks as fill the resident blocks once, none shorter than 8 planes (a
+// chunk stages A planes more than it has; lattices small enough to be cut that
+// far lie in L2). At 128^3 whole columns are 64 blocks for 152 SMs.
+template <typename T, int R>
+static dim3 zcol_grid(int N) {
+    const int cols = ((N + 31) / 32) * ((N + 7) / 8), slots = num_sms() * ZMarch<T, R>::MINB;
+    return dim3(cols, std::max(1, std::min((slots + cols / 2) / cols, N / 8)));
+}
+
+// One thread's coefficients for the block: GB300's FP64 pipe makes them cost
+// hundreds of cycles per warp.
+template <typename T>
+__device__ __forceinline__ StepCoefs<T> block_coefs(const double *clock, double dt, double kick, double inv_dx2,
+                                                    double lambda, double T0sq3, int prs, int form) {
+    __shared__ StepCoefs<T> sc;
+    if (threadIdx.x == 0) sc = make_coefs<T>(*clock, dt, kick, inv_dx2, lambda, T0sq3, prs, form);
+    __syncthreads();
+    return sc;
+}
+
+// pi_n by the staged march: SOA, all four fields (psi and pi_n) into the
+// caller's separate arrays, 16 B read and 16 B written per FP32 site; otherwise
+// pi_n alone as complex values into out[0]. One thread per site (64-bit index
+// divisions, neighbours from L1/L2) into scratch and two unpacking passes took
+// 56 B per site; 20 steps and a snapshot at 1024^3 FP32 went from 69.6 to
+// 62.4 ms, 10 steps of radius 2 at 384^3 from 4.13 to 3.18 ms.
+template <typename T>
+struct SnapOut {
+    T *f[4];
+};
+template <typename T, int R, bool SOA>
+__global__ void __launch_bounds__(256, (ZMarch<T, R>::MINB))
+    k_sync_zcol(const typename Cplx<T>::type *__restrict__ psi, const typename Cplx<T>::type *__restrict__ pih,
+                SnapOut<T> out, const double *clock, int N, double dt, double inv_dx2, double lambda, double T0sq3,
+                int prs, int form, int fresh) {
+    typedef typename Cplx<T>::type C;
+    const StepCoefs<T> c = block_coefs<T>(clock, dt, 0.5 * dt, inv_dx2, lambda, T0sq3, prs, form);
+    const int nbx = (N + 31) / 32;
+    const int x = (int)(blockIdx.x % nbx) * 32 + (threadIdx.x & 31), y = (int)(blockIdx.x / nbx) * 8 + (threadIdx.x >> 5);
+    const int64_t NN = (int64_t)N * N, col = x < N && y < N ? y * N + x : 0;
+    zcol_march<T, R>(psi, pih, N, fresh, c, [&](int, int z, const C &zc, const C &, const C &p, const C *) {
+        const int64_t m = z * NN + col;
+        if constexpr (SOA) {
+            out.f[0][m] = zc.x;
+            out.f[1][m] = zc.y;
+            out.f[2][m] = p.x;
+            out.f[3][m] = p.y;
+        } else {
+            reinterpret_cast<C *>(out.f[0])[m] = p;
+        }
+    });
+}
+
+// The same for 2D: one thread per site of 32 x 8 tiles, the neighbours from
+// L1/L2 (the lattice fits L2 up to 3000^2).
+template <typename T, int R, bool SOA>
+__global__ void __launch_bounds__(256)
+    k_sync_2d(const typename Cplx<T>::type *__restrict__ psi, const typename Cplx<T>::type *__restrict__ pih, SnapOut<T> out,
+              const double *clock, int N, double dt, double inv_dx2, double lambda, double T0sq3, int prs, int form,
+              int fresh) {
+    typedef typename Cplx<T>::type C;
+    const StepCoefs<T> c = block_coefs<T>(clock, dt, 0.5 * dt, inv_dx2, lambda, T0sq3, prs, form);
+    const int nbx = (N + 31) / 32, nt = nbx * ((N + 7) / 8);
+    for (int t = blockIdx.x; t < nt; t += gridDim.x) {
+        const int ty = t / nbx, x = (t - ty * nbx) * 32 + (threadIdx.x & 31), y = ty * 8 + (threadIdx.x >> 5);
+        if (x >= N || y >= N) continue;
+        const int m = y * N + x;
+        const C f = psi[m];
+        C p = pih[m];
+        if (!fresh) {   // stencil_at's sums: radius 1 as lap5, else the weights in order
+            T L1, L2;
+            if constexpr (R > 1) {
+                L1 = (T)stencil_coef(R - 1, 2, 0) * f.x;
+                L2 = (T)stencil_coef(R - 1, 2, 0) * f.y;
+            }
+#pragma unroll
+            for (int l = 1; l <= R; ++l) {
+                const C xm = psi[m - x + (x < l ? x - l + N : x - l)], xp = psi[m - x + (x + l >= N ? x + l - N : x + l)];
+                const C ym = psi[(y < l ? y - l + N : y - l) * N + x], yp = psi[(y + l >= N ? y + l - N : y + l) * N + x];
+                if constexpr (R == 1) {
+                    L1 = lap5<T>(f.x, xm.x, xp.x, ym.x, yp.x);
+                    L2 = lap5<T>(f.y, xm.y, xp.y, ym.y, yp.y);
+                } else {
+                    const T w = (T)stencil_coef(R - 1, 2, l);
+                    L1 = fma(w, nsum5<T>(xm.x, xp.x, ym.x, yp.x), L1);
+                    L2 = fma(w, nsum5<T>(xm.y, xp.y, ym.y, yp.y), L2);
+                }
+            }
+            sync_pi_site<T>(f.x, f.y, L1, L2, p.x, p.y, c);
+        }
+        if constexpr (SOA) {
+            out.f[0][m] = f.x;
+            out.f[1][m] = f.y;
+            out.f[2][m] = p.x;
+            out.f[3][m] = p.y;
+        } else {
+            reinterpret_cast<C *>(out.f[0])[m] = p;
+        }
+    }
+}
+
+template <typename T, int R, bool SOA>
+static void sync_fd_r(Lattice *L, const SnapOut<T> &out) {
+    typedef typename Cplx<T>::type C;
+    const axs_params &p = L->p;
+    const double dx = p.space_step, T0 = p.T_initial, dt = p.time_step, idx2 = 1.0 / (dx * dx), la = p.lambda;
+    const C *f = (const C *)L->psi[L->cur], *q = (const C *)L->pih;
+    const double *clk = L->dclock + L->cur;
+    if (p.NDIMS == 2) {
+        const int nt = ((p.N + 31) / 32) * ((p.N + 7) / 8);
+        k_sync_2d<T, R, SOA><<<std::min(nt, num_sms() * 8), 256, 0, L->stream>>>(f, q, out, clk, p.N, dt, idx2, la,
+                                                                                (T0 * T0) / 3.0, p.prs, p.form, L->fresh);
+    } else {
+        const size_t smem = ZMarch<T, R>::SMEM;
+        AXS_CUDA(cudaFuncSetAttribute(k_sync_zcol<T, R, SOA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k_sync_zcol<T, R, SOA><<<zcol_grid<T, R>(p.N), 256, smem, L->stream>>>(f, q, out, clk, p.N, dt, idx2, la,
+                                                                            (T0 * T0) / 3.0, p.prs, p.form, L->fresh);
+    }
+    AXS_CUDA(cudaGetLastError());
+    count_launches(1);
+}
+template <typename T, bool SOA>
+static void sync_fd(Lattice *L, const SnapOut<T> &out) {
+    switch (L->p.stencil_setting) {
+    case 0: sync_fd_r<T, 1, SOA>(L, out); break;
+    case 1: sync_fd_r<T, 2, SOA>(L, out); break;
+    case 2: sync_fd_r<T, 3, SOA>(L, out); break;
+    default: sync_fd_r<T, 4, SOA>(L, out); break;
+    }
+}
+void sync_pi_fd(Lattice *L) {
+    if (L->esz == 4) sync_fd<float, false>(L, SnapOut<float>{{(float *)L->scratch}});
+    else sync_fd<double, false>(L, SnapOut<double>{{(double *)L->scratch}});
+}
+void snapshot_fd(Lattice *L, void *const f[4]) {
+    if (L->esz == 4) sync_fd<float, true>(L, SnapOut<float>{{(float *)f[0], (float *)f[1], (float *)f[2], (float *)f[3]}});
+    else sync_fd<double, true>(L, SnapOut<double>{{(double *)f[0], (double *)f[1], (double *)f[2], (double *)f[3]}});
+}
+
 // The axion field of the kinetic spectrum for a stencil of radius R = 1..4:
 // 20 B per site from DRAM (psi, pih in, f out), against 44 B and per-site
-// 64-bit index arithmetic through k_sync_pi and scratch. (At radius 1 a
+// 64-bit index arithmetic through a synchronising pass and scratch. (At radius 1 a
 // march with the column's psi and pih loaded into registers two planes ahead
 // and the in-plane neighbours read from global memory ran 3.7 against 3.5 ms
 // at 1024^3.)
@@ -1470,10 +1616,10 @@ __global__ void __launch_bounds__(256, (ZMarch<T, R>::MINB)) k_axion_zcol_r(cons
                                                                  const typename Cplx<T>::type *__restrict__ pih,
                                                                  T *__restrict__ dst, const double *clock, int N,
                                                                  double dt, double inv_dx2, double lambda,
-                                                                 double T0sq3, int prs, int fresh, double tau) {
+                                                                 double T0sq3, int prs, int fresh, double itaud) {
     typedef typename Cplx<T>::type C;
-    const StepCoefs<T> c = make_coefs<T>(*clock, dt, 0.5 * dt, inv_dx2, lambda, T0sq3, prs, 0);
-    const T itau = (T)(1.0 / tau);
+    const StepCoefs<T> c = block_coefs<T>(clock, dt, 0.5 * dt, inv_dx2, lambda, T0sq3, prs, 0);
+    const T itau = (T)itaud;
     const int nbx = (N + 31) / 32;
     const int x = (int)(blockIdx.x % nbx) * 32 + (threadIdx.x & 31), y = (int)(blockIdx.x / nbx) * 8 + (threadIdx.x >> 5);
     const int64_t NN = (int64_t)N * N;
@@ -1495,16 +1641,15 @@ static void axion_zcol_t(Lattice *L) {
     T *dst = (T *)L->fft_in;
     const double *clk = L->dclock + L->cur;
     const double dt = p.time_step, idx2 = 1.0 / (dx * dx), la = p.lambda, t3 = (T0 * T0) / 3.0;
-    const int g = ((N + 31) / 32) * ((N + 7) / 8);   // blocks of 32 x 8 columns
-    auto radius = [&](auto kern, size_t smem) {
+    auto radius = [&](auto kern, size_t smem, dim3 g) {
         AXS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<g, 256, smem, L->stream>>>(f, q, dst, clk, N, dt, idx2, la, t3, p.prs, L->fresh, L->tau);
+        kern<<<g, 256, smem, L->stream>>>(f, q, dst, clk, N, dt, idx2, la, t3, p.prs, L->fresh, 1.0 / L->tau);
     };
     switch (p.stencil_setting) {
-    case 0: radius(k_axion_zcol_r<T, 1>, ZMarch<T, 1>::SMEM); break;
-    case 1: radius(k_axion_zcol_r<T, 2>, ZMarch<T, 2>::SMEM); break;
-    case 2: radius(k_axion_zcol_r<T, 3>, ZMarch<T, 3>::SMEM); break;
-    default: radius(k_axion_zcol_r<T, 4>, ZMarch<T, 4>::SMEM); break;
+    case 0: radius(k_axion_zcol_r<T, 1>, ZMarch<T, 1>::SMEM, zcol_grid<T, 1>(N)); break;
+    case 1: radius(k_axion_zcol_r<T, 2>, ZMarch<T, 2>::SMEM, zcol_grid<T, 2>(N)); break;
+    case 2: radius(k_axion_zcol_r<T, 3>, ZMarch<T, 3>::SMEM, zcol_grid<T, 3>(N)); break;
+    default: radius(k_axion_zcol_r<T, 4>, ZMarch<T, 4>::SMEM, zcol_grid<T, 4>(N)); break;
     }
 }
 
@@ -1981,7 +2126,7 @@ __device__ __forceinline__ void load_pair(const double2 *__restrict__ a, int64_t
 // plus the local part of the half kick and the host adds dt/2 W/dx^2 mean(psi).
 // That equals the mean of the per-site pi_n up to rounding (FP64: within
 // 1e-12 of the oracle's per-site sums) and reads 16 B per site instead of
-// k_sync_pi's 24 B plus 16 B. Two sites per trip
+// a synchronising pass's 24 B plus 16 B. Two sites per trip
 // (N^d is even), their terms added before one compensated add; the grid is
 // one wave of resident blocks.
 template <typename T>
@@ -2088,7 +2233,7 @@ __global__ void __launch_bounds__(256) k_energies(const typename Cplx<T>::type *
 // Energy densities of a 3D radius-1 lattice in one pass over psi and pih
 // (the kinetic term is quadratic in pi_n, so unlike the background means it
 // needs the full half kick per site). pi_n is formed per site with
-// k_sync_pi's arithmetic and never stored, and each thread marches one (x, y)
+// sync_pi_site and never stored, and each thread marches one (x, y)
 // column through z: psi's z-neighbours stay in registers
 // and the in-plane neighbours (also the x+1, y+1 forward differences of the
 // gradient energy; z+1 is the next plane in registers) come from the

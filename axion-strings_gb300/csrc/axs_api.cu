@@ -309,6 +309,17 @@ template <typename S>
 static void download_fields(Lattice *L, S *f0, S *f1, S *f2, S *f3) {
     S *dst[4] = {f0, f1, f2, f3};
     const int is_d = sizeof(S) == 8;
+    // a whole state in the lattice's precision into arrays that the device
+    // reaches: one pass over psi and pih, without scratch
+    void *dev[4] = {nullptr, nullptr, nullptr, nullptr};
+    bool direct = f0 && f1 && f2 && f3 && (int)sizeof(S) == L->esz && L->p.laplacian == 0;
+    for (int f = 0; f < 4 && direct; ++f) direct = (dev[f] = device_alias(dst[f])) != nullptr;
+    if (direct) {
+        snapshot_fd(L, dev);
+        AXS_CUDA(cudaStreamSynchronize(L->stream));
+        check_device_errors(L);
+        return;
+    }
     if (f2 || f3) launch_sync_pi(L);
     for (int pr = 0; pr < 2; ++pr) {
         const void *src = pr == 1 ? L->scratch : L->psi[L->cur];

@@ -271,6 +271,10 @@ void energies(Lattice *L, double out[3]);
 int check_finite(Lattice *L);
 void field_distance(Lattice *A, Lattice *B, double out[8]);
 void analysis_release(Lattice *L);
+// finite-difference lattices: pi_n into scratch; psi and pi_n into four arrays
+// of the lattice's precision that the device reaches
+void sync_pi_fd(Lattice *L);
+void snapshot_fd(Lattice *L, void *const f[4]);
 
 // helpers
 inline int64_t lattice_length(const axs_params &p) {

@@ -12,7 +12,7 @@
 // so one pass reads psi (with stencil halo) and pih and writes both: 4 reals
 // read + 4 written per site, no stored kernel arrays. The synchronised
 // momentum the reference holds between steps is pi_n = pih_{n-1} + dt/2 K_n,
-// produced on demand by k_sync_pi.
+// produced on demand (k_sync_zcol, k_sync_2d, k_sync_pi_spectral).
 //
 // Device layout: psi and pih are complex-interleaved arrays (re = field 1,
 // im = field 2) in the reference's site order; psi is double-buffered.
@@ -128,23 +128,6 @@ __global__ void __launch_bounds__(256) k_step_generic(const typename Cplx<T>::ty
         out[m] = o;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) *clock_out = tau + dt;
-}
-
-// Synchronised momentum pi_n = pih_{n-1} + dt/2 K(psi_n, tau_n) into `dst`.
-template <typename T, int ND, int R>
-__global__ void k_sync_pi(const typename Cplx<T>::type *__restrict__ psi, const typename Cplx<T>::type *__restrict__ pih,
-                          typename Cplx<T>::type *__restrict__ dst, const double *clock, int N, int64_t len, double dt,
-                          double inv_dx2, double lambda, double T0sq3, int prs, int setting, int form) {
-    StepCoefs<T> c = make_coefs<T>(*clock, dt, 0.5 * dt, inv_dx2, lambda, T0sq3, prs, form);
-    int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; m < len; m += stride) {
-        T L1, L2;
-        typename Cplx<T>::type ctr;
-        stencil_at<T, ND, R>(psi, m, N, setting, L1, L2, ctr);
-        auto p = pih[m];
-        sync_pi_site<T>(ctr.x, ctr.y, L1, L2, p.x, p.y, c);
-        dst[m] = p;
-    }
 }
 
 // ---- spectral Laplacian (compute_laplacian_fft, s_integrate.cpp:179-296)
@@ -2876,7 +2859,11 @@ void lattice_autotune(Lattice *L) {
         log.push_back({c, ms});
         if (ms < best_ms) { best_ms = ms; best = c; }
     }
-    const int zchunks[] = {32, 64, 128, 256};
+    // chunks of 8 and 16 planes for lattices whose tiles are too few for the SMs
+    // otherwise (128^3 has 32 tiles of 64 x 8 sites)
+    std::vector<int> zchunks{32, 64, 128, 256};
+    if (L->p.N <= 160) zchunks.insert(zchunks.begin(), 16);
+    if (L->p.N <= 80) zchunks.insert(zchunks.begin(), 8);
     auto trial = [&](int v, int zc, int nrep, int nwarm) {
         const bool oop = out_of_place(v, L);
         StepConfig c;
@@ -3179,26 +3166,6 @@ void ensemble_evolve(Ensemble *E, int nsteps) {
     }
 }
 // ---------------------------------------------------------------- helpers
-template <typename T, int ND, int R>
-static void sync_pi_t(Lattice *L) {
-    typedef typename Cplx<T>::type C;
-    double dx = L->p.space_step, T0 = L->p.T_initial;
-    k_sync_pi<T, ND, R><<<grid_for(L->length), 256, 0, L->stream>>>(
-        (const C *)L->psi[L->cur], (const C *)L->pih, (C *)L->scratch, L->dclock + L->cur, L->p.N, L->length,
-        (double)L->p.time_step, 1.0 / (dx * dx), (double)L->p.lambda, (T0 * T0) / 3.0, L->p.prs, L->p.stencil_setting,
-        L->p.form);
-    AXS_CUDA(cudaGetLastError());
-    count_launches(1);
-}
-template <typename T>
-static void sync_pi_dispatch(Lattice *L) {
-    int R = L->p.stencil_setting + 1;
-    if (L->p.NDIMS == 2) {
-        if (R == 1) sync_pi_t<T, 2, 1>(L); else if (R == 2) sync_pi_t<T, 2, 2>(L); else if (R == 3) sync_pi_t<T, 2, 3>(L); else sync_pi_t<T, 2, 4>(L);
-    } else {
-        if (R == 1) sync_pi_t<T, 3, 1>(L); else if (R == 2) sync_pi_t<T, 3, 2>(L); else if (R == 3) sync_pi_t<T, 3, 3>(L); else sync_pi_t<T, 3, 4>(L);
-    }
-}
 void launch_sync_pi(Lattice *L) {
     if (L->fresh) {   // pih holds pi_0 and the reference's ker_curr is zero
         AXS_CUDA(cudaMemcpyAsync(L->scratch, L->pih, (size_t)L->length * 2 * L->esz, cudaMemcpyDeviceToDevice, L->stream));
@@ -3220,8 +3187,7 @@ void launch_sync_pi(Lattice *L) {
         count_launches(1);
         return;
     }
-    if (L->esz == 4) sync_pi_dispatch<float>(L);
-    else sync_pi_dispatch<double>(L);
+    sync_pi_fd(L);
 }
 
 template <typename T, int ND, int R>

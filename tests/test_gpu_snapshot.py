@@ -1,0 +1,61 @@
+"""The whole state in one pass (axs_download into arrays the device reaches)
+gives the bits of the copy through host staging, for 2D and 3D, every stencil
+radius, both precisions, fresh and stepped states, at sizes around the march's
+32 x 8 columns and its shortest z-chunks."""
+import numpy as np
+import pytest
+
+from gpu_util import params
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("nd,N,stencil", [(2, 4, 0), (2, 30, 0), (2, 34, 1), (2, 70, 2), (2, 66, 3),
+                                          (3, 4, 0), (3, 6, 1), (3, 8, 2), (3, 10, 3), (3, 18, 0), (3, 34, 0),
+                                          (3, 64, 0), (3, 66, 1), (3, 40, 2), (3, 36, 3), (3, 130, 0)])
+def test_direct_snapshot_equals_staged(axs, precision, nd, N, stencil):
+    p = params(axs, nd=nd, N=N, precision=precision, stencil_setting=stencil)
+    dt = np.float64 if precision == 64 else np.float32
+    with axs.Lattice(p) as L:
+        rng = np.random.default_rng(2)
+        L.upload(*[rng.standard_normal(L.shape) for _ in range(4)])
+        for steps in (0, 3):
+            L.evolve(steps)
+            want = L.download(dtype=dt)
+            out = [axs.PinnedBuffer(L.shape, dt) for _ in range(4)]
+            fn = axs._lib.axs_download if precision == 64 else axs._lib.axs_download_f32
+            axs._check(fn(L._h, *[o.array.ctypes.data for o in out]))
+            for a, b in zip(out, want):
+                assert np.array_equal(a.array, b), steps
+            for o in out:
+                o.free()
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("N", [4, 6, 18, 64])
+def test_axion_spectrum_of_small_lattices(axs, oracle, precision, N):
+    """The march's planes wrap more than once on the smallest lattices (its ring runs A = 5 planes ahead)."""
+    from gpu_util import orc
+    p = params(axs, nd=3, N=N, precision=precision)
+    f = oracle.init_thermal(orc(p), 4)
+    with axs.Lattice(p) as L:
+        L.upload(*f)
+        L.evolve(4)
+        k, pk, c = L.axion_spectrum(8)
+        g = L.download()
+        tau = L.time[0]
+    ref = (g[1] * g[2] - g[0] * g[3]) / (tau * np.hypot(g[0], g[1]))
+    F = np.abs(np.fft.fftn(ref)) ** 2
+    n = np.fft.fftfreq(N, 1.0 / N)
+    n2 = (n[:, None, None] ** 2 + n[None, :, None] ** 2 + n[None, None, :] ** 2).round().astype(int)
+    ratio = np.sqrt(3.0) * N / 2
+    edges = [0] + [int(np.ceil(np.exp(np.log(ratio) * b / 8) ** 2)) for b in range(1, 8)]
+    at = np.searchsorted(edges, n2, side="right") - 1
+    at[n2 == 0] = -1
+    norm = (N * 0.5) ** 3 / float(N ** 3) ** 2
+    for b in range(8):
+        assert c[b] == (at == b).sum()
+        if c[b]:
+            # the tests of both precisions against the oracle: 1e-10 and 1e-4
+            assert abs(pk[b] - norm * F[at == b].mean()) <= (1e-10 if precision == 64 else 1e-4) * pk[b]
