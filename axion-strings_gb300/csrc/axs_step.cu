@@ -101,33 +101,99 @@ __device__ __forceinline__ void stencil_at(const typename Cplx<T>::type *__restr
     L2 = a2;
 }
 
-// One 3D step, one thread per site (grid-stride). Used for lattice shapes the
-// z-march kernels do not tile, and where it is the fastest candidate.
+// One 3D step of any N and stencil radius: a thread per (x, y) column of a
+// z-chunk, blocks of 32 x 8 columns. psi's z-neighbours stay in registers, the
+// in-plane neighbours come from L1/L2 (the neighbouring threads' loads), the
+// in-plane offsets are fixed for the column, and one thread forms the block's
+// time coefficients. FP64 steps are bound by the FP64 pipe (nine operations per
+// site at radius 1) with the neighbour sums' integer work under them, so this
+// kernel without barriers beats the TMA march there: 45 / 290 us per step at
+// 128^3 / 256^3 (37 / 298 at 18.5 cycles per operation and SM), where the march
+// takes 62 / 400 and one thread per site with 64-bit index divisions took 60 /
+// 371. FP32 lattices that lie in L2 take it too (64^3: 5.0 us per step where the
+// two-step march takes 6.5, 144^3: 19.3 and 20.6), beyond that where no tile fits.
 template <typename T, int R>
 __global__ void __launch_bounds__(256) k_step_generic(const typename Cplx<T>::type *__restrict__ psi,
                                                       typename Cplx<T>::type *__restrict__ out,
                                                       typename Cplx<T>::type *__restrict__ pih,
-                                                      const double *clock_in, double *clock_out, int N, int64_t len,
-                                                      double dt, double inv_dx2, double lambda, double T0sq3, int prs,
-                                                      int setting, int form) {
-    double tau = *clock_in;
-    StepCoefs<T> c = make_coefs<T>(tau, dt, dt, inv_dx2, lambda, T0sq3, prs, form);
-    constexpr bool FOLD = sizeof(T) == 8 && R == 1;
-    constexpr int ND = 3;
-    const T kctr = c.kdt_idx2 * (T)(-2 * ND);
-    int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; m < len; m += stride) {
-        T L1, L2;
-        typename Cplx<T>::type ctr;
-        stencil_at<T, ND, R, FOLD>(psi, m, N, setting, L1, L2, ctr);
-        auto p = pih[m];
-        typename Cplx<T>::type o;
-        if constexpr (FOLD) site_update_fold<T>(ctr.x, ctr.y, L1, L2, p.x, p.y, o.x, o.y, c, kctr);
-        else site_update<T>(ctr.x, ctr.y, L1, L2, p.x, p.y, o.x, o.y, c);
-        pih[m] = p;
-        out[m] = o;
+                                                      const double *clock_in, double *clock_out, int N, double dt,
+                                                      double inv_dx2, double lambda, double T0sq3, int prs, int form) {
+    typedef typename Cplx<T>::type C;
+    __shared__ StepCoefs<T> sc;
+    __shared__ T skctr;
+    if (threadIdx.x == 0) {
+        const double tau = *clock_in;
+        sc = make_coefs<T>(tau, dt, dt, inv_dx2, lambda, T0sq3, prs, form);
+        skctr = sc.kdt_idx2 * (T)-6;
+        if (blockIdx.x == 0 && blockIdx.y == 0) *clock_out = tau + dt;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *clock_out = tau + dt;
+    const int nbx = (N + 31) / 32;
+    const int x = (int)(blockIdx.x % nbx) * 32 + (threadIdx.x & 31), y = (int)(blockIdx.x / nbx) * 8 + (threadIdx.x >> 5);
+    const int za = (int)((int64_t)blockIdx.y * N / gridDim.y), zb = (int)((int64_t)(blockIdx.y + 1) * N / gridDim.y);
+    __syncthreads();
+    if (x >= N || y >= N) return;
+    const StepCoefs<T> c = sc;
+    const T kctr = skctr;
+    const int64_t NN = (int64_t)N * N;
+    const int col = y * N + x;
+    int xo[2 * R], yo[2 * R];   // in-plane offsets of the neighbours at distances 1..R, minus and plus
+#pragma unroll
+    for (int l = 1; l <= R; ++l) {
+        xo[l - 1] = (x < l ? N : 0) - l;
+        xo[R + l - 1] = (x + l >= N ? -N : 0) + l;
+        yo[l - 1] = ((y < l ? N : 0) - l) * N;
+        yo[R + l - 1] = ((y + l >= N ? -N : 0) + l) * N;
+    }
+    C zr[2 * R + 1];   // planes z-R .. z+R
+#pragma unroll
+    for (int d = 0; d < 2 * R; ++d) {
+        const int pl = za + d - R;
+        zr[d] = psi[(int64_t)(pl < 0 ? pl + N : (pl >= N ? pl - N : pl)) * NN + col];
+    }
+    const C *cur = psi + (int64_t)za * NN + col;
+    C *pp = pih + (int64_t)za * NN + col, *po = out + (int64_t)za * NN + col;
+    const C *ahead = psi + (int64_t)(za + R >= N ? za + R - N : za + R) * NN + col;
+    for (int z = za; z < zb; ++z) {
+        zr[2 * R] = *ahead;
+        C p = *pp, xm[R], xp[R], ym[R], yp[R];
+#pragma unroll
+        for (int l = 0; l < R; ++l) {
+            xm[l] = cur[xo[l]];
+            xp[l] = cur[xo[R + l]];
+            ym[l] = cur[yo[l]];
+            yp[l] = cur[yo[R + l]];
+        }
+        ahead = z + R + 1 == N ? psi + col : ahead + NN;
+        const C ctr = zr[R];
+        C o;
+        if constexpr (R == 1) {
+            if constexpr (sizeof(T) == 8) {   // the centre weight folded (site_update_fold)
+                const T S1 = nsum7<T>(xm[0].x, xp[0].x, ym[0].x, yp[0].x, zr[0].x, zr[2].x);
+                const T S2 = nsum7<T>(xm[0].y, xp[0].y, ym[0].y, yp[0].y, zr[0].y, zr[2].y);
+                site_update_fold<T>(ctr.x, ctr.y, S1, S2, p.x, p.y, o.x, o.y, c, kctr);
+            } else {
+                const T L1 = lap7<T>(ctr.x, xm[0].x, xp[0].x, ym[0].x, yp[0].x, zr[0].x, zr[2].x);
+                const T L2 = lap7<T>(ctr.y, xm[0].y, xp[0].y, ym[0].y, yp[0].y, zr[0].y, zr[2].y);
+                site_update<T>(ctr.x, ctr.y, L1, L2, p.x, p.y, o.x, o.y, c);
+            }
+        } else {   // stencil_at's order
+            T a1 = (T)stencil_coef(R - 1, 3, 0) * ctr.x, a2 = (T)stencil_coef(R - 1, 3, 0) * ctr.y;
+#pragma unroll
+            for (int l = 1; l <= R; ++l) {
+                const T w = (T)stencil_coef(R - 1, 3, l);
+                a1 = fma(w, nsum7<T>(xm[l - 1].x, xp[l - 1].x, ym[l - 1].x, yp[l - 1].x, zr[R - l].x, zr[R + l].x), a1);
+                a2 = fma(w, nsum7<T>(xm[l - 1].y, xp[l - 1].y, ym[l - 1].y, yp[l - 1].y, zr[R - l].y, zr[R + l].y), a2);
+            }
+            site_update<T>(ctr.x, ctr.y, a1, a2, p.x, p.y, o.x, o.y, c);
+        }
+        *pp = p;
+        *po = o;
+        cur += NN;
+        pp += NN;
+        po += NN;
+#pragma unroll
+        for (int d = 0; d < 2 * R; ++d) zr[d] = zr[d + 1];
+    }
 }
 
 // ---- spectral Laplacian (compute_laplacian_fft, s_integrate.cpp:179-296)
@@ -1951,7 +2017,7 @@ static int radius(const ZVariant &v) { return v.r > 0 ? v.r : 1; }
 
 std::string StepConfig::describe() const {
     char b[200];
-    if (kind == 0) snprintf(b, sizeof b, "generic per-site kernel");   // 2D: axs_step_2d.cu
+    if (kind == 0) snprintf(b, sizeof b, "generic kernel (3D: z-march by columns, 2D: steps per launch)");
     else if (two_step(variant))
         snprintf(b, sizeof b, "TMA z-march variant %d (two steps per pass, halo depth 2%s; odd step on variant %d), tx=%d, zchunk=%d",
                  variant, kZVariants[variant].lean ? ", lean" : "", kZVariants[variant].partner, tx, zchunk);
@@ -2499,15 +2565,18 @@ void step_release(Lattice *L) {
     L->dcounter = nullptr;
 }
 
+// About 16 blocks per SM (their work evens out over the SMs), in chunks of at
+// least 4 planes.
 template <typename T, int R>
 static void launch_generic_t(Lattice *L, const double *cin, double *cout) {
     typedef typename Cplx<T>::type C;
     const axs_params &p = L->p;
-    double dx = p.space_step;
-    double T0 = p.T_initial;
-    k_step_generic<T, R><<<grid_for(L->length), 256, 0, L->stream>>>(
-        (const C *)L->psi[L->cur], (C *)L->psi[L->cur ^ 1], (C *)L->pih, cin, cout, p.N, L->length,
-        (double)p.time_step, 1.0 / (dx * dx), (double)p.lambda, (T0 * T0) / 3.0, p.prs, p.stencil_setting, p.form);
+    const double dx = p.space_step, T0 = p.T_initial;
+    const int cols = ((p.N + 31) / 32) * ((p.N + 7) / 8);
+    const dim3 grid(cols, std::max(1, std::min((16 * num_sms() + cols - 1) / cols, p.N / 4)));
+    k_step_generic<T, R><<<grid, 256, 0, L->stream>>>(
+        (const C *)L->psi[L->cur], (C *)L->psi[L->cur ^ 1], (C *)L->pih, cin, cout, p.N, (double)p.time_step,
+        1.0 / (dx * dx), (double)p.lambda, (T0 * T0) / 3.0, p.prs, p.form);
     AXS_CUDA(cudaGetLastError());
     count_launches(1);
 }
@@ -2860,10 +2929,10 @@ void lattice_autotune(Lattice *L) {
         if (ms < best_ms) { best_ms = ms; best = c; }
     }
     // chunks of 8 and 16 planes for lattices whose tiles are too few for the SMs
-    // otherwise (128^3 has 32 tiles of 64 x 8 sites)
+    // otherwise (128^3 has 32 tiles of 64 x 8 sites: 18.6 us per step with chunks of
+    // 32, 13.4 with 16)
     std::vector<int> zchunks{32, 64, 128, 256};
-    if (L->p.N <= 160) zchunks.insert(zchunks.begin(), 16);
-    if (L->p.N <= 80) zchunks.insert(zchunks.begin(), 8);
+    if (L->p.N <= 160) zchunks.insert(zchunks.begin(), {8, 16});
     auto trial = [&](int v, int zc, int nrep, int nwarm) {
         const bool oop = out_of_place(v, L);
         StepConfig c;
