@@ -114,10 +114,11 @@ static void lattice_init(Lattice *L, const axs_params &p, cudaStream_t shared) {
     L->psi[1] = dalloc(cbytes);
     L->pih = dalloc(cbytes);
     L->scratch = dalloc(cbytes);
-    L->dclock = (double *)dalloc(2 * sizeof(double));
-    L->derr = (int *)dalloc(sizeof(int));
+    // one small allocation: the clock's two slots, the error flag, 2D: the coefficient tables
+    L->dclock = (double *)dalloc(256 + (p.NDIMS == 2 ? 2 * kStep2dSlot : 0));
+    L->derr = (int *)(L->dclock + 2);
     if (p.NDIMS == 2) {
-        L->dstep2d = dalloc(2 * kStep2dSlot);
+        L->dstep2d = (char *)L->dclock + 256;
         AXS_CUDA(cudaMemsetAsync(L->dstep2d, 0xff, 2 * kStep2dSlot, L->stream));   // NaN tags: no table yet
     }
     AXS_CUDA(cudaMemsetAsync(L->psi[0], 0, cbytes, L->stream));
@@ -144,9 +145,7 @@ static void lattice_free(Lattice *L) {
     dfree(L->psi[1]);
     dfree(L->pih);
     dfree(L->scratch);
-    dfree(L->dclock);
-    dfree(L->dstep2d);
-    dfree(L->derr);
+    dfree(L->dclock);   // with the error flag and the tables
     dfree(L->dstage);
     if (L->own_stream && L->stream) cudaStreamDestroy(L->stream);
     L->stream = nullptr;

@@ -117,7 +117,8 @@ struct GraphEntry {
 };
 
 // Shape of a multi-step 2D launch (axs_step_2d.cu): sites per lane, rows per
-// warp, warps, steps, tiles across and in all, and its estimated time.
+// warp, warps (0: the one-step march), steps, tiles across and in all, and its
+// estimated time.
 struct Plan2d {
     int xs = 0, v = 0, nw = 0, k = 1, ntx = 0, ntiles = 0;
     double us = 1e30;

@@ -22,16 +22,17 @@
 // same bits.
 //
 // Measured (GB300, graph of launches, us per step): FP32 radius 1 at 128^2 /
-// 512^2 / 1500^2 / 4096^2: 0.58 / 1.03 / 4.9 / 34 with 10 / 6 / 6 / 6 steps
-// per launch, against 5 / 11 / 26 / 99 with one thread per site and one step per
+// 512^2 / 1500^2 / 4096^2: 0.48 / 1.03 / 5.0 / 34 with 8 / 6 / 4 / 6 steps
+// per launch, against 3.2 / 10 / 23 / 99 with one thread per site and one step per
 // launch; FP64 (bound by its FP64 pipe, 9 operations per site and step)
-// 1.8 / 7.2 / 49 / 340 against 6 / 17 / 70 / 520. A launch costs about 3 us
+// 1.8 / 7.0 / 44 / 300 against 4 / 16 / 77 / 520 (from 470^2 the march below). A launch costs about 3 us
 // before its first step; it was 0.6 us more when every block formed the time
 // coefficients (FP64 divisions, one dependent chain): an extra block now forms
 // those of the next launch while the others step. Programmatic dependent
 // launch gained nothing (the next launch's blocks take slots from this one's).
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "axs_internal.h"
 
@@ -146,16 +147,50 @@ __device__ __forceinline__ void store_sites(typename Cplx<T>::type *p, const typ
     }
 }
 
+// The coefficients n steps from tau (advanced as single steps advance it), and FP64's centre weight.
+template <typename T>
+__device__ __forceinline__ StepCoefs<T> make_step_coefs(const Step2dArgs &A, double tau, int n, T &kctr) {
+    for (int s = 0; s < n; ++s) tau = tau + A.dt;
+    const StepCoefs<T> c = make_coefs<T>(tau, A.dt, A.dt, A.inv_dx2, A.lambda, A.T0sq3, A.prs, A.form);
+    kctr = sizeof(T) == 8 ? c.kdt_idx2 * (T)-4 : (T)0;
+    return c;
+}
+// Those of step n of this launch, from the table when its tag is this clock and step.
+template <typename T>
+__device__ __forceinline__ StepCoefs<T> step_coefs(const Step2dArgs &A, int n, T &kctr) {
+    const Step2dTable<T> *t = reinterpret_cast<const Step2dTable<T> *>(A.tab_in);
+    const double tau = *A.clock_in;
+    const bool made = t->tau == tau && t->dt == A.dt;
+    const StepCoefs<T> c = t->c[n];
+    kctr = t->kctr[n];
+    return made ? c : make_step_coefs<T>(A, tau, n, kctr);
+}
+// The launch's extra block: the next clock and its table.
+template <typename T>
+__device__ __forceinline__ void next_table(const Step2dArgs &A) {
+    const int tid = threadIdx.x;
+    if (tid >= kStep2dMaxK) return;
+    double tau = *A.clock_in;
+    for (int s = 0; s < A.k; ++s) tau = tau + A.dt;
+    Step2dTable<T> *t = reinterpret_cast<Step2dTable<T> *>(A.tab_out);
+    t->c[tid] = make_step_coefs<T>(A, tau, tid, t->kctr[tid]);
+    if (tid == 0) {
+        t->tau = tau;
+        t->dt = A.dt;
+        *A.clock_out = tau;
+    }
+}
+
 // XS sites per lane, V rows per warp; the block's warps (1 .. 16, at run time)
 // lie above one another. R <= V.
 template <typename T, int R, int XS, int V>
 __global__ void __launch_bounds__(V <= 2 ? 512 : 256) k_step2d(const Step2dArgs A) {
     typedef typename Cplx<T>::type C;
-    static_assert(R <= V, "the halo rows come from the next warps");
     constexpr int RX = 32 * XS;
+    constexpr int E = V < 2 * R ? V : 2 * R;   // rows a warp publishes: its first and last R, or all
     constexpr int LN = (R + XS - 1) / XS;   // lanes to either side that hold x neighbours
     extern __shared__ __align__(16) unsigned char smem[];
-    // the first and last R rows of each warp, two buffers: [2][warps][2R][RX]
+    // the first and last R rows of each warp (all, if fewer than 2R), two buffers: [2][warps][E][RX]
     C *edge = reinterpret_cast<C *>(smem);
     __shared__ StepCoefs<T> coefs[kStep2dMaxK];
     __shared__ T kctrs[kStep2dMaxK];
@@ -165,37 +200,13 @@ __global__ void __launch_bounds__(V <= 2 ? 512 : 256) k_step2d(const Step2dArgs 
     const int TX = RX - 2 * HX, TY = RY - 2 * H;
     const C *psi = reinterpret_cast<const C *>(A.psi), *pih = reinterpret_cast<const C *>(A.pih);
     C *po = reinterpret_cast<C *>(A.psi_out), *qo = reinterpret_cast<C *>(A.pih_out);
-    auto make = [&](double tau, int n, StepCoefs<T> &c, T &kc) {   // step n from tau, advanced as single steps advance it
-        for (int s = 0; s < n; ++s) tau = tau + A.dt;
-        c = make_coefs<T>(tau, A.dt, A.dt, A.inv_dx2, A.lambda, A.T0sq3, A.prs, A.form);
-        kc = sizeof(T) == 8 ? c.kdt_idx2 * (T)-4 : (T)0;
-    };
-    if (blockIdx.x == gridDim.x - 1) {   // the last block: the next clock and its table
-        if (tid < kStep2dMaxK) {
-            double tau = *A.clock_in;
-            for (int s = 0; s < k; ++s) tau = tau + A.dt;
-            Step2dTable<T> *t = reinterpret_cast<Step2dTable<T> *>(A.tab_out);
-            StepCoefs<T> c;
-            T kc;
-            make(tau, tid, c, kc);
-            t->c[tid] = c;
-            t->kctr[tid] = kc;
-            if (tid == 0) {
-                t->tau = tau;
-                t->dt = A.dt;
-                *A.clock_out = tau;
-            }
-        }
+    if (blockIdx.x == gridDim.x - 1) {
+        next_table<T>(A);
         return;
     }
     if (tid < k) {
-        const Step2dTable<T> *t = reinterpret_cast<const Step2dTable<T> *>(A.tab_in);
-        const double tau = *A.clock_in;
-        const bool made = t->tau == tau && t->dt == A.dt;
-        StepCoefs<T> c = t->c[tid];
-        T kc = t->kctr[tid];
-        if (!made) make(tau, tid, c, kc);
-        coefs[tid] = c;
+        T kc;
+        coefs[tid] = step_coefs<T>(A, tid, kc);
         if (sizeof(T) == 8) kctrs[tid] = kc;
     }
     for (int tile = blockIdx.x; tile < A.ntiles; tile += gridDim.x - 1) {
@@ -215,23 +226,22 @@ __global__ void __launch_bounds__(V <= 2 ? 512 : 256) k_step2d(const Step2dArgs 
             }
         }
         for (int s = 0; s < k; ++s) {
-            C *eb = edge + (s & 1) * nw * 2 * R * RX;
+            C *eb = edge + (s & 1) * nw * E * RX;
+            // rows 0 .. R-1 of the warp at 0 .. R-1, rows V-R .. V-1 at the end (E < 2R: row r at r)
 #pragma unroll
-            for (int l = 0; l < R; ++l) {
-                store_sites<T, XS>(eb + (w * 2 * R + l) * RX + x, a[l]);
-                store_sites<T, XS>(eb + (w * 2 * R + R + l) * RX + x, a[V - R + l]);
-            }
+            for (int e = 0; e < E; ++e) store_sites<T, XS>(eb + (w * E + e) * RX + x, a[e < R ? e : V - E + e]);
             __syncthreads();
             Site2d<T, R> st;
             st.c = coefs[s];
             st.kctr = sizeof(T) == 8 ? kctrs[s] : (T)0;
             const int lo = R * (s + 1), hi = RY - lo;   // rows with all their neighbours
             C up[R][XS], dn[R][XS];   // rows y - 1 .. y - R before this step; rows past the warp's last
-            const int wu = max(w - 1, 0), wd = min(w + 1, nw - 1);
+            // row y0 - 1 - l is the l-th of the warp above from its end (l < V), of the one above that, ...
 #pragma unroll
             for (int l = 0; l < R; ++l) {
-                load_sites<T, XS>(eb + (wu * 2 * R + 2 * R - 1 - l) * RX + x, up[l]);
-                load_sites<T, XS>(eb + (wd * 2 * R + l) * RX + x, dn[l]);
+                const int wu = max(w - 1 - l / V, 0), wd = min(w + 1 + l / V, nw - 1);
+                load_sites<T, XS>(eb + (wu * E + E - 1 - l % V) * RX + x, up[l]);
+                load_sites<T, XS>(eb + (wd * E + l % V) * RX + x, dn[l]);
             }
 #pragma unroll
             for (int v = 0; v < V; ++v) {
@@ -285,64 +295,158 @@ __global__ void __launch_bounds__(V <= 2 ? 512 : 256) k_step2d(const Step2dArgs 
     }
 }
 
+// One FP64 step of a large lattice: a thread per column of a y-chunk, the y
+// neighbours in registers, the x neighbours from L1. FP64 is bound by its pipe,
+// so here the tiles' halo columns (2 R k of 32 lanes) cost more than a launch per
+// step (kMarch2dSites).
+template <int R>
+__global__ void __launch_bounds__(128) k_march2d(const Step2dArgs A) {
+    typedef double2 C;
+    __shared__ StepCoefs<double> sc;
+    __shared__ double skctr;
+    const int N = A.N, x = blockIdx.x * 128 + threadIdx.x;
+    const int chunks = gridDim.y - 1;   // the last row of blocks forms the next launch's coefficients
+    if ((int)blockIdx.y == chunks) {
+        if (blockIdx.x == 0) next_table<double>(A);
+        return;
+    }
+    if (threadIdx.x == 0) sc = step_coefs<double>(A, 0, skctr);
+    const int ya = (int)((int64_t)blockIdx.y * N / chunks), yb = (int)((int64_t)(blockIdx.y + 1) * N / chunks);
+    __syncthreads();
+    if (x >= N) return;
+    Site2d<double, R> st;
+    st.c = sc;
+    st.kctr = skctr;
+    const C *psi = reinterpret_cast<const C *>(A.psi), *pih = reinterpret_cast<const C *>(A.pih);
+    C *po = reinterpret_cast<C *>(A.psi_out), *qo = reinterpret_cast<C *>(A.pih_out);
+    int xl[R], xr[R];
+#pragma unroll
+    for (int l = 0; l < R; ++l) {
+        xl[l] = x - 1 - l < 0 ? x - 1 - l + N : x - 1 - l;
+        xr[l] = x + 1 + l >= N ? x + 1 + l - N : x + 1 + l;
+    }
+    C yr[2 * R + 1];   // rows y-R .. y+R
+#pragma unroll
+    for (int d = 0; d < 2 * R; ++d) {
+        const int y = ya + d - R;
+        yr[d] = psi[(y < 0 ? y + N : (y >= N ? y - N : y)) * N + x];
+    }
+    for (int y = ya; y < yb; ++y) {
+        const int row = y * N;
+        yr[2 * R] = psi[(y + R >= N ? y + R - N : y + R) * N + x];
+        C p = pih[row + x], a = yr[R], xm[R], xp[R], ym[R], yp[R];
+#pragma unroll
+        for (int l = 0; l < R; ++l) {
+            xm[l] = psi[row + xl[l]];
+            xp[l] = psi[row + xr[l]];
+            ym[l] = yr[R - 1 - l];
+            yp[l] = yr[R + 1 + l];
+        }
+        st.update(a, p, xm, xp, ym, yp);
+        po[row + x] = a;
+        qo[row + x] = p;
+#pragma unroll
+        for (int d = 0; d < 2 * R; ++d) yr[d] = yr[d + 1];
+    }
+}
+// About 16 blocks per SM, in chunks of at least 2 rows (4 from 800^2: 1000^2 takes
+// 19.8 us with 4, 20.6 with 2; 512^2 7.4 and 7.0).
+template <int R>
+static void launch_march2d(const Step2dArgs &a, cudaStream_t st) {
+    const int cols = (a.N + 127) / 128;
+    const dim3 grid(cols, std::max(1, std::min((16 * num_sms() + cols - 1) / cols, a.N / (a.N < 800 ? 2 : 4))) + 1);
+    k_march2d<R><<<grid, 128, 0, st>>>(a);
+    AXS_CUDA(cudaGetLastError());
+    count_launches(1);
+}
+// Sites from which FP64 takes it, by radius: us per step of the march and of the
+// tiles at radius 1, 426^2 6.5 and 5.9, 512^2 7.0 and 8.3, 1000^2 19.8 and 26,
+// 3000^2 158 and 216; radius 2, 256^2 5.5 and 5.4, 340^2 7.1 and 9.1; radius 3, 256^2
+// 6.0 and 7.3; radius 4, 126^2 5.5 and 5.9, 64^2 5 and 3.9.
+constexpr double kMarch2dSites[4] = {220000.0, 75000.0, 32000.0, 12000.0};
+
 // ---------------------------------------------------------------- dispatch
 //
 // The shape of a launch (sites per lane, rows per warp, warps, steps) follows
-// from a cost estimate over the shapes below, in SM cycles fitted to
-// measurements: a launch costs t0 plus a barrier's latency per step; an SM takes
-// ceil(tiles / SMs) tiles, each as many 32-site rows as its shrinking region
-// has over the steps, at the cost of a row (FP32 9 cycles at radius 1, FP64
-// 18.5 per FP64 operation); and the tiles' loads and stores go at L2's rate while
-// the state fits it, else HBM's. More steps per launch amortise t0 and the
-// memory traffic, and cost halo: at 128^2 ten to twelve steps per launch win
-// in FP32, at 1500^2 four to six, in FP64 one to four.
+// from an estimate of its time over the shapes below: a launch costs t0; an SM
+// takes ceil(tiles / SMs) tiles, in rounds of as many as are resident, a
+// round at a load's latency plus a barrier's per step; a tile costs the 32-site
+// rows that its shrinking region has over the steps times the cycles of a row
+// (a lone block's rows count as its fullest scheduler's, four to the SM); and
+// loads and stores go at L2's rate while the state fits half of it (each die's
+// share), else HBM's. The
+// constants are fitted to 1300 measured launches (N = 64 .. 1500, all radii):
+// 5 % rms in FP32, 9 % in FP64, and the shape chosen is within 12 % of the best
+// measured one in FP32 and 20 % (one case 32 %) in FP64. More steps per launch
+// amortise t0, latency and traffic and cost halo: at 128^2 eight steps per
+// launch win in FP32, at 1500^2 four to six; FP64, bound by its pipe, takes one
+// to four.
 struct Shape2d {
-    int xs, v, nwmin, nwmax, nwstep;
+    int xs, v;
+    double row;   // SM cycles per 32-site row
 };
 
 template <typename T, int R>
 static int shapes2d(const Shape2d *&s) {
-    static constexpr Shape2d f1[] = {{2, 2, 4, 8, 4}, {2, 4, 4, 8, 4}, {2, 8, 4, 8, 4}};
-    static constexpr Shape2d f2[] = {{2, 4, 4, 8, 4}, {2, 8, 4, 8, 4}};
-    static constexpr Shape2d f4[] = {{2, 4, 4, 8, 4}};
-    static constexpr Shape2d d1[] = {{1, 1, 4, 16, 1}, {1, 2, 3, 12, 1}, {1, 4, 4, 8, 1}};
-    static constexpr Shape2d d2[] = {{1, 2, 4, 12, 1}, {1, 4, 4, 8, 1}};
-    static constexpr Shape2d d4[] = {{1, 4, 4, 8, 1}};
+    static constexpr Shape2d f1[] = {{1, 2, 5.4}, {2, 2, 4.8}, {2, 4, 6.8}, {2, 8, 8.5}};
+    static constexpr Shape2d f2[] = {{1, 2, 15.6}, {2, 2, 14.4}, {2, 4, 14.7}, {2, 8, 14.1}};
+    static constexpr Shape2d f3[] = {{1, 2, 28.2}, {2, 2, 25.0}, {2, 4, 21.4}};
+    static constexpr Shape2d f4[] = {{1, 2, 42.0}, {2, 2, 35.7}, {2, 4, 29.7}};
+    static constexpr Shape2d d1[] = {{1, 1, 92.6}, {1, 2, 126.0}, {1, 4, 138.9}};
+    static constexpr Shape2d d2[] = {{1, 1, 233.5}, {1, 2, 281.2}};
+    static constexpr Shape2d d3[] = {{1, 1, 377.5}, {1, 2, 374.9}};
+    static constexpr Shape2d d4[] = {{1, 1, 552.2}, {1, 2, 512.1}};
     if constexpr (sizeof(T) == 4) {
-        if constexpr (R == 1) { s = f1; return 3; }
-        else if constexpr (R == 2) { s = f2; return 2; }
-        else { s = f4; return 1; }
+        s = R == 1 ? f1 : R == 2 ? f2 : R == 3 ? f3 : f4;
+        return R <= 2 ? 4 : 3;
     } else {
-        if constexpr (R == 1) { s = d1; return 3; }
-        else if constexpr (R == 2) { s = d2; return 2; }
-        else { s = d4; return 1; }
+        s = R == 1 ? d1 : R == 2 ? d2 : R == 3 ? d3 : d4;
+        return R == 1 ? 3 : 2;
     }
 }
+
+// Resident blocks per SM of a shape with nw warps.
+template <typename T, int R>
+static int resident2d(const Shape2d &s, int nw);
 
 template <typename T, int R>
 static Plan2d plan2d_k(int N, int k, int sms) {
     const Shape2d *sh = nullptr;
     const int n = shapes2d<T, R>(sh);
     const bool f32 = sizeof(T) == 4;
-    const double row = f32 ? 9.0 * (0.4 + 0.6 * R) : 18.5 * (R == 1 ? 9 : 11 + 2 * R);
-    const double ghz = 1.92, t0 = 3.0, step = f32 ? 0.12 : 0.5;
+    const double t0 = f32 ? 1.8 : 1.9, lat = f32 ? 0.25 : 0.08, step = f32 ? 0.19 : 0.77;   // us
     const double csz = 2.0 * sizeof(T);
-    const double bw = 4.0 * N * N * csz < 100e6 ? 10e6 : 6.5e6;   // bytes per us
+    const double bw = 4.0 * N * N * csz < 60e6 ? (f32 ? 15.8e6 : 13.9e6) : 6.5e6;   // bytes per us
     Plan2d best;
-    for (int i = 0; i < n; ++i)
-        for (int nw = sh[i].nwmin; nw <= sh[i].nwmax; nw += sh[i].nwstep) {
-            const int rx = 32 * sh[i].xs, ry = sh[i].v * nw, h = k * R, hx = (h + sh[i].xs - 1) / sh[i].xs * sh[i].xs;
+    for (int i = 0; i < n; ++i) {
+        const int V = sh[i].v, xs = sh[i].xs;
+        for (int nw = 4; nw <= (V <= 2 ? 16 : 8); nw += f32 ? 4 : 2) {
+            const int rx = 32 * xs, ry = V * nw, h = k * R, hx = (h + xs - 1) / xs * xs;
             const int tx = rx - 2 * hx, ty = ry - 2 * h;
             if (tx < 8 || ty < 2) continue;
             const int ntx = (N + tx - 1) / tx;
-            const double tiles = (double)ntx * ((N + ty - 1) / ty);
-            const double rows = (double)k * ry - R * (double)k * (k + 1);   // sum of ry - 2 R s
-            const double per_sm = tiles / sms <= 8.0 ? std::ceil(tiles / sms) : tiles / sms;
-            const double us = t0 + step * k + per_sm * rows * sh[i].xs * row / (ghz * 1e3) +
+            const double tiles = (double)ntx * ((N + ty - 1) / ty), per = tiles / sms;
+            // few rows per warp are for lattices of few tiles: with more, their loads are
+            // not under other blocks' steps (1500^2 FP32: 5.9 us per step, V = 4 and 8 5.1)
+            if (f32 && V == 2 && per > 2.0) continue;
+            const int occ = resident2d<T, R>(sh[i], nw);
+            double rows = 0.0;
+            for (int s = 1; s <= k; ++s) {
+                const int a = ry - 2 * R * s;
+                int r = a;
+                if (per <= 1.0) {
+                    const int warps = (a + V - 1) / V + ((R * s) % V && a > V ? 1 : 0);
+                    r = std::max(a, 4 * V * ((warps + 3) / 4));
+                }
+                rows += r;
+            }
+            const double rounds = per <= 8.0 * occ ? std::ceil(per / occ) : per / occ;
+            const double us = t0 + rounds * (lat + step * k) +
+                              (per <= 8.0 ? std::ceil(per) : per) * rows * xs * sh[i].row / 1920.0 +
                               tiles * ((double)rx * ry + (double)tx * ty) * 2.0 * csz / bw;
             if (us < best.us) {
-                best.xs = sh[i].xs;
-                best.v = sh[i].v;
+                best.xs = xs;
+                best.v = V;
                 best.nw = nw;
                 best.k = k;
                 best.ntx = ntx;
@@ -350,6 +454,7 @@ static Plan2d plan2d_k(int N, int k, int sms) {
                 best.us = us;
             }
         }
+    }
     return best;
 }
 
@@ -359,51 +464,69 @@ template <typename T, int R>
 static Plan2d plan2d(int N, int max_steps) {
     const int sms = num_sms();
     Plan2d best;
+    if (sizeof(T) == 8 && (double)N * N >= kMarch2dSites[R - 1]) return best;   // one step by k_march2d
     for (int k = 1; k <= std::min(12, max_steps); ++k) {
         const Plan2d p = plan2d_k<T, R>(N, k, sms);
         if (p.nw && p.us / k < best.us / best.k) best = p;
     }
     const int launches = (max_steps + best.k - 1) / best.k, k = (max_steps + launches - 1) / launches;
-    return k == best.k ? best : plan2d_k<T, R>(N, k, sms);
+    if (k == best.k) return best;
+    const Plan2d p = plan2d_k<T, R>(N, k, sms);
+    return p.nw ? p : best;
+}
+
+template <typename T, int R, int XS, int V>
+static int resident2d_t(int nw) {
+    typedef typename Cplx<T>::type C;
+    constexpr int E = V < 2 * R ? V : 2 * R;
+    constexpr int per_warp = 2 * E * 32 * XS * (int)sizeof(C);
+    static PerDevice occ[17];   // the kernel's shared-memory attribute and occupancy belong to the device
+    return occ[nw].get([nw] {
+        AXS_CUDA(cudaFuncSetAttribute(k_step2d<T, R, XS, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (V <= 2 ? 16 : 8) * per_warp));
+        int o = 0;
+        AXS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_step2d<T, R, XS, V>, 32 * nw, nw * per_warp));
+        return std::max(1, o);
+    });
 }
 
 template <typename T, int R, int XS, int V>
 static void launch2d_t(const Step2dArgs &a, int nw, cudaStream_t st) {
     typedef typename Cplx<T>::type C;
-    const int smem = 2 * nw * 2 * R * 32 * XS * (int)sizeof(C);
-    constexpr int smax = 2 * (V <= 2 ? 16 : 8) * 2 * R * 32 * XS * (int)sizeof(C);
-    static PerDevice ready;   // the kernel's shared-memory attribute belongs to the device
-    ready.get([] {
-        AXS_CUDA(cudaFuncSetAttribute(k_step2d<T, R, XS, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
-        return 1;
-    });
-    static PerDevice occ[17];
-    const int per = occ[nw].get([nw, smem] {
-        int o = 0;
-        AXS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_step2d<T, R, XS, V>, 32 * nw, smem));
-        return std::max(1, o);
-    });
-    const int grid = (int)std::min<int64_t>(a.ntiles, (int64_t)per * num_sms()) + 1;   // and the next launch's coefficients
+    constexpr int E = V < 2 * R ? V : 2 * R;
+    const int smem = nw * 2 * E * 32 * XS * (int)sizeof(C);
+    // one more block for the next launch's coefficients
+    const int grid = (int)std::min<int64_t>(a.ntiles, (int64_t)resident2d_t<T, R, XS, V>(nw) * num_sms()) + 1;
     k_step2d<T, R, XS, V><<<grid, 32 * nw, smem, st>>>(a);
     AXS_CUDA(cudaGetLastError());
     count_launches(1);
 }
 
+// fn<XS, V>() for the shape (xs, v) of shapes2d
+template <typename T, int R, class Fn>
+static void with_shape2d(int xs, int v, Fn fn) {
+    if constexpr (sizeof(T) == 4) {
+        if (xs == 1) fn(std::integral_constant<int, 1>(), std::integral_constant<int, 2>());
+        else if (v == 2) fn(std::integral_constant<int, 2>(), std::integral_constant<int, 2>());
+        else if (v == 4) fn(std::integral_constant<int, 2>(), std::integral_constant<int, 4>());
+        else if constexpr (R <= 2) fn(std::integral_constant<int, 2>(), std::integral_constant<int, 8>());
+    } else {
+        if (v == 1) fn(std::integral_constant<int, 1>(), std::integral_constant<int, 1>());
+        else if (v == 2) fn(std::integral_constant<int, 1>(), std::integral_constant<int, 2>());
+        else if constexpr (R == 1) fn(std::integral_constant<int, 1>(), std::integral_constant<int, 4>());
+    }
+}
+template <typename T, int R>
+static int resident2d(const Shape2d &s, int nw) {
+    int o = 1;
+    with_shape2d<T, R>(s.xs, s.v, [&](auto xs, auto v) { o = resident2d_t<T, R, xs(), v()>(nw); });
+    return o;
+}
 template <typename T, int R>
 static void launch2d(const Step2dArgs &a, const Plan2d &p, cudaStream_t st) {
-    if constexpr (sizeof(T) == 4) {
-        if constexpr (R == 1)
-            if (p.v == 2) return launch2d_t<T, R, 2, 2>(a, p.nw, st);
-        if constexpr (R <= 2)
-            if (p.v == 8) return launch2d_t<T, R, 2, 8>(a, p.nw, st);
-        launch2d_t<T, R, 2, 4>(a, p.nw, st);
-    } else {
-        if constexpr (R == 1)
-            if (p.v == 1) return launch2d_t<T, R, 1, 1>(a, p.nw, st);
-        if constexpr (R <= 2)
-            if (p.v == 2) return launch2d_t<T, R, 1, 2>(a, p.nw, st);
-        launch2d_t<T, R, 1, 4>(a, p.nw, st);
-    }
+    if constexpr (sizeof(T) == 8)
+        if (p.nw == 0) return launch_march2d<R>(a, st);
+    with_shape2d<T, R>(p.xs, p.v, [&](auto xs, auto v) { launch2d_t<T, R, xs(), v()>(a, p.nw, st); });
 }
 
 template <typename T, int R>

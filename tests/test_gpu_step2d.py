@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("precision", [64, 32])
 @pytest.mark.parametrize("stencil,N", [(0, 4), (0, 6), (0, 26), (0, 30), (0, 62), (0, 64), (0, 66), (0, 128), (0, 502),
-                                       (1, 6), (1, 60), (1, 130), (2, 8), (2, 54), (3, 10), (3, 58), (3, 200)])
+                                       (1, 6), (1, 60), (1, 130), (1, 276), (2, 8), (2, 54), (2, 180), (3, 10), (3, 58),
+                                       (3, 108), (3, 110), (3, 200)])
 def test_steps_per_launch_bit_identical(axs, oracle, precision, stencil, N):
     p = params(axs, nd=2, N=N, precision=precision, stencil_setting=stencil)
     f = oracle.init_thermal(orc(p), 3)
