@@ -59,3 +59,29 @@ def test_axion_spectrum_of_small_lattices(axs, oracle, precision, N):
         if c[b]:
             # the tests of both precisions against the oracle: 1e-10 and 1e-4
             assert abs(pk[b] - norm * F[at == b].mean()) <= (1e-10 if precision == 64 else 1e-4) * pk[b]
+
+
+@pytest.mark.parametrize("fields", [(0, 1), (0, 1, 2, 3), (1,), (2,)])
+def test_large_pageable_downloads(axs, fields):
+    """Destinations large enough to be touched ahead of the copies (several chunks, not page-aligned) get the values of
+    the pinned ones, and nothing outside them is written."""
+    p = params(axs, nd=3, N=202, precision=64)
+    with axs.Lattice(p) as L:
+        L.init_flat(7, 1.0)
+        L.evolve(3)
+        pins = [axs.PinnedBuffer(L.shape, np.float64) for _ in range(4)]
+        axs._check(axs._lib.axs_download(L._h, *[o.array.ctypes.data for o in pins]))
+        raw = [np.full(L.length + 24, -7.0) for _ in fields]
+        got = {f: r[13:13 + L.length] for f, r in zip(fields, raw)}
+        axs._check(axs._lib.axs_download(L._h, *[got[f].ctypes.data if f in got else None for f in range(4)]))
+        for f in fields:
+            assert np.array_equal(got[f].reshape(L.shape), pins[f].array)
+        for r in raw:
+            assert (r[:13] == -7.0).all() and (r[13 + L.length:] == -7.0).all()
+        c = L.checkpoint()
+        with axs.Lattice(p) as M:
+            M.restore(c)
+            for a, b in zip(M.download(), pins):
+                assert np.array_equal(a, b.array)
+        for o in pins:
+            o.free()
