@@ -134,11 +134,22 @@ __device__ __noinline__ int cell3_exact(Corner<T, FROM_THETA> cn, int64_t x, int
     return (ta > accept || tb > accept || tc > accept) ? 1 : 0;
 }
 
-template <typename T, int ND, bool FROM_THETA>
-__global__ void __launch_bounds__(256) k_cores(const typename Cplx<T>::type *__restrict__ psi,
-                                               const double *__restrict__ theta, uint8_t *__restrict__ mask, int N,
+// The same for the 2D cell (i, j) = (x, y): corners (i,j), (i+1,j), (i+1,j+1), (i,j+1).
+template <typename T>
+__device__ __noinline__ int cell2_exact(Corner<T, false> cn, int x, int y, int N, double accept) {
+    const int xp = x + 1 == N ? 0 : x + 1, yp = y + 1 == N ? 0 : y + 1;
+    const double n1 = cn.nd((int64_t)y * N + x), n2 = cn.nd((int64_t)y * N + xp), n3 = cn.nd((int64_t)yp * N + xp),
+                 n4 = cn.nd((int64_t)yp * N + x);
+    return sum3(circd(n1, n2), circd(n2, n3), circd(n3, n4)) > accept ? 1 : 0;
+}
+
+// The finder on a caller's theta.
+template <int ND>
+__global__ void __launch_bounds__(256) k_cores(const double *__restrict__ theta, uint8_t *__restrict__ mask, int N,
                                                int64_t len, double accept, unsigned long long *count) {
-    Corner<T, FROM_THETA> cn{psi, theta};
+    typedef double T;
+    constexpr bool FROM_THETA = true;
+    Corner<T, FROM_THETA> cn{nullptr, theta};
     const float acc_f = (float)accept;
     unsigned long long local = 0;
     const int64_t NN = (int64_t)N * N;
@@ -210,6 +221,7 @@ __global__ void __launch_bounds__(256) k_cores(const typename Cplx<T>::type *__r
 // whose twelve sums all lie above the margin (nearly every thread: flagged
 // cells are rare) writes four zero bytes without forming the flag bits.
 static constexpr int kCX = 64, kCY = 16, kCZ = 32;   // cells per block tile; 256 threads x 4 cells
+static constexpr int kChunk = 4096;                  // cells per chunk of the list's compaction
 static constexpr int kHalo = kCX + kCY + 1;          // the tile's +y row and +x column (with the corner)
 
 // 1/2 - |b - a| for angles in turns (see above)
@@ -225,7 +237,7 @@ static constexpr int kRS = kCX + 4;                   // shared row stride: 16-b
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3)
     k_cores3_tiled(const typename Cplx<T>::type *__restrict__ psi, uint8_t *__restrict__ mask, int N, double accept,
-                   unsigned long long *count) {
+                   unsigned long long *count, int32_t *__restrict__ chunks, unsigned *ticket, int64_t *hout) {
     typedef typename Cplx<T>::type C;
     __shared__ __align__(16) float nsm[2][kCY + 1][kRS];
     Corner<T, false> cn{psi, nullptr};
@@ -366,6 +378,15 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3)
             word &= vbytes;   // cells past the lattice's edge
             und &= vmask;
             local += __popc(word);
+            if (chunks && word) {
+                if (VEC) {
+                    atomicAdd(&chunks[mo / kChunk], __popc(word));   // 4 divides mo and kChunk
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if ((word >> (8 * j)) & 1u) atomicAdd(&chunks[(mo + j) / kChunk], 1);
+                }
+            }
             if (und) unc[(z - z0) >> 3][tid] |= und << (4 * ((z - z0) & 7));
         }
         if (VEC) {
@@ -400,101 +421,263 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3)
             u &= u - 1;
             const int zz = z0 + (b >> 2), j = b & 3;
             if (cell3_exact<T, false>(cn, gx + j, gy, zz, N, accept)) {
-                mask[(int64_t)zz * NN + (int64_t)gy * N + gx + j] = 1;
+                const int64_t m = (int64_t)zz * NN + (int64_t)gy * N + gx + j;
+                mask[m] = 1;
+                if (chunks) atomicAdd(&chunks[m / kChunk], 1);
                 ++local;
             }
         }
     }
     for (int o = 16; o > 0; o >>= 1) local += __shfl_down_sync(0xffffffffu, local, o);
     if ((threadIdx.x & 31) == 0 && local) atomicAdd(count, (unsigned long long)local);
+    if (hout && last_block(ticket) && tid == 0) {   // the count to the host, the counter to 0 for the next search
+        *hout = (int64_t)__ldcg(count);
+        *count = 0;
+    }
 }
 
-// ---- ordered compaction of the mask: chunk counts, scan, ordered write
-static constexpr int kChunk = 4096;   // cells per block
-
-__global__ void k_chunk_counts(const uint8_t *__restrict__ mask, int64_t len, int64_t *__restrict__ counts) {
-    int64_t base = (int64_t)blockIdx.x * kChunk;
-    int c = 0;
-    for (int q = threadIdx.x; q < kChunk; q += blockDim.x) {
-        int64_t m = base + q;
-        if (m < len) c += mask[m];
+// 2D finder from psi: 64 x 16 cells per block, four along x per thread, the
+// angles (turns) once per site through shared memory, as in k_cores3_tiled.
+// A thread per cell took four fast_atan2 and 64-bit divisions each. At small
+// sizes the launches and synchronisations bound the call: a search and its
+// list at 352^2 FP32 go from 112 to 73 us with this, k_pairs2 and the results in
+// page-locked memory.
+template <typename T>
+__global__ void __launch_bounds__(256) k_cores2_tiled(const typename Cplx<T>::type *__restrict__ psi,
+                                                      uint8_t *__restrict__ mask, int N, double accept,
+                                                      unsigned long long *count) {
+    __shared__ __align__(16) float ns[kCY + 1][kRS];
+    Corner<T, false> cn{psi, nullptr};
+    const float acc_f = (float)accept;
+    const float t_flag = 1.5f - acc_f - kMargin, t_undecided = 1.5f - acc_f + kMargin;
+    const int tid = threadIdx.x, x0 = blockIdx.x * kCX, y0 = blockIdx.y * kCY;
+    const int lx = 4 * (tid & 15), ly = tid >> 4, gx = x0 + lx, gy = y0 + ly;
+    // a site at x = N or y = N is site 0 of that axis; sites past that belong to no cell
+    auto site = [&](int x, int y) {
+        if (x > N || y > N) return 0.0f;
+        const auto v = psi[(int64_t)(y == N ? 0 : y) * N + (x == N ? 0 : x)];
+        return fast_turns((float)v.x, (float)v.y);
+    };
+    float a[5];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) a[j] = site(gx + j, gy);
+    *reinterpret_cast<float4 *>(&ns[ly][lx]) = make_float4(a[0], a[1], a[2], a[3]);
+    if (tid < kHalo) {   // the +y row, then the +x column with the corner
+        const bool row = tid < kCX;
+        const float h = row ? site(x0 + tid, y0 + kCY) : site(x0 + kCX, y0 + tid - kCX);
+        if (row) ns[kCY][tid] = h;
+        else ns[tid - kCX][kCX] = h;
     }
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    __shared__ int ws[8];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = c;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int64_t s = 0;
-        for (int w = 0; w < 8; ++w) s += ws[w];
-        counts[blockIdx.x] = s;
-    }
-}
-
-// Exclusive scan of n counts by one block of 1024 threads.
-__global__ void k_scan(int64_t *__restrict__ counts, int64_t n, int64_t *__restrict__ total) {
-    __shared__ int64_t part[1024];
-    int64_t per = (n + 1023) / 1024;
-    int64_t b = threadIdx.x * per, e = b + per < n ? b + per : n;
-    int64_t s = 0;
-    for (int64_t i = b; i < e; ++i) s += counts[i];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int64_t run = 0;
-        for (int i = 0; i < 1024; ++i) { int64_t v = part[i]; part[i] = run; run += v; }
-        *total = run;
-    }
-    __syncthreads();
-    int64_t run = part[threadIdx.x];
-    for (int64_t i = b; i < e; ++i) { int64_t v = counts[i]; counts[i] = run; run += v; }
-}
-
-__global__ void k_chunk_write(const uint8_t *__restrict__ mask, int64_t len, const int64_t *__restrict__ offsets,
-                              int64_t *__restrict__ list) {
-    __shared__ int wsum[8];
-    int64_t base = (int64_t)blockIdx.x * kChunk;
-    int64_t out = offsets[blockIdx.x];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int q0 = 0; q0 < kChunk; q0 += blockDim.x) {
-        int64_t m = base + q0 + threadIdx.x;
-        int f = (m < len) ? mask[m] : 0;
-        unsigned bal = __ballot_sync(0xffffffffu, f);
-        if (lane == 0) wsum[w] = __popc(bal);
-        __syncthreads();
-        int before = 0, tot = 0;
-        for (int i = 0; i < 8; ++i) { if (i < w) before += wsum[i]; tot += wsum[i]; }
-        if (f) list[out + before + __popc(bal & ((1u << lane) - 1))] = m;
-        out += tot;
-        __syncthreads();
-    }
-}
-
-// Neighbouring-plaquette pairs of s_run.cpp:101-109 over the ascending list.
-__global__ void k_pairs2(const int64_t *__restrict__ list, int64_t n, int N, unsigned long long *pairs) {
-    unsigned long long local = 0;
-    int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q + 1 < n; q += stride) {
-        int64_t a = list[q], b = list[q + 1];
-        int64_t dx = (b % N) - (a % N), dy = (b / N) - (a / N);
-        local += (dy == 0 && dx == 1) || (dy == 1 && dx == 0);
+    a[4] = ns[ly][lx + 4];
+    float b[5];
+    const float4 q = *reinterpret_cast<const float4 *>(&ns[ly + 1][lx]);
+    b[0] = q.x; b[1] = q.y; b[2] = q.z; b[3] = q.w; b[4] = ns[ly + 1][lx + 4];
+    unsigned local = 0, word = 0;
+    if (gy < N) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (gx + j >= N) continue;
+            // the edges (i,j)-(i+1,j)-(i+1,j+1)-(i,j+1), kept as |t| (see above)
+            const float tm = fabsf(half_gap(a[j], a[j + 1])) + fabsf(half_gap(a[j + 1], b[j + 1])) + fabsf(half_gap(b[j + 1], b[j]));
+            unsigned f = tm < t_flag ? 1u : 0u;
+            if (!f && tm <= t_undecided) f = (unsigned)cell2_exact<T>(cn, gx + j, gy, N, accept);
+            word |= f << (8 * j);
+        }
+        local = __popc(word);
+        uint8_t *m = mask + (int64_t)gy * N + gx;
+        if ((N & 3) == 0) {
+            if (gx < N) *reinterpret_cast<unsigned *>(m) = word;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (gx + j < N) m[j] = (uint8_t)(word >> (8 * j));
+        }
     }
     for (int o = 16; o > 0; o >>= 1) local += __shfl_down_sync(0xffffffffu, local, o);
-    if ((threadIdx.x & 31) == 0 && local) atomicAdd(pairs, local);
+    if ((tid & 31) == 0 && local) atomicAdd(count, (unsigned long long)local);
 }
 
-__global__ void k_positions(const int64_t *__restrict__ list, int64_t n, int N, int ndims, int32_t *__restrict__ pos) {
-    int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    int64_t NN = (int64_t)N * N;
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += stride) {
-        int64_t m = list[q];
-        if (ndims == 2) { pos[2 * q] = (int32_t)(m % N); pos[2 * q + 1] = (int32_t)(m / N); }
-        else { pos[3 * q] = (int32_t)(m / NN); pos[3 * q + 1] = (int32_t)((m / N) % N); pos[3 * q + 2] = (int32_t)(m % N); }
+// ---- the flagged cells' positions in ascending offset order: flagged cells per
+// chunk of kChunk cells (counted by the 3D finder as it writes the mask, else
+// by k_chunk_counts), an exclusive scan, and an ordered write by a warp per
+// chunk. At 512^3 with 383 thousand cells: 48 us, the 3D finder's own counts
+// included; byte loads and a block per chunk took 453.
+
+// 16 mask bytes (0 or 1) of cells m .. m + 15, zeros past len.
+__device__ __forceinline__ uint4 mask16(const uint8_t *__restrict__ mask, int64_t m, int64_t len) {
+    if (m + 16 <= len) return *reinterpret_cast<const uint4 *>(mask + m);   // m is a multiple of 16
+    unsigned w[4] = {0, 0, 0, 0};
+    for (int j = 0; j < 16 && m + j < len; ++j) w[j >> 2] |= (unsigned)mask[m + j] << (8 * (j & 3));
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+// bit j: byte j is 1
+__device__ __forceinline__ unsigned bits16(const uint4 &v) {
+    auto b4 = [](unsigned w) { return (w * 0x08040201u) >> 24 & 0xfu; };   // bytes 0, 1, 2, 3 to bits 3, 2, 1, 0
+    const unsigned r = b4(v.x) << 12 | b4(v.y) << 8 | b4(v.z) << 4 | b4(v.w);
+    return __brev(r) >> 16;
+}
+__device__ __forceinline__ int count16(const uint4 &v) { return __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w); }
+
+__global__ void __launch_bounds__(256) k_chunk_counts(const uint8_t *__restrict__ mask, int64_t len, int nch,
+                                                      int32_t *__restrict__ counts) {
+    const int c = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (c >= nch) return;
+    int n = 0;
+#pragma unroll
+    for (int it = 0; it < kChunk / 512; ++it) n += count16(mask16(mask, (int64_t)c * kChunk + it * 512 + lane * 16, len));
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (lane == 0) counts[c] = n;
+}
+
+// Exclusive scan in place, in blocks of 4096 counts; block b's total goes to
+// totals[b] and the last block scans those (a 32-bit sum: at most 2^31 cells are
+// listed, the reference's int).
+__global__ void __launch_bounds__(256) k_chunk_scan(int32_t *__restrict__ counts, int n, int64_t *__restrict__ totals,
+                                                    unsigned *ticket) {
+    __shared__ int ws[8];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, i0 = blockIdx.x * 4096 + tid * 16;
+    int v[16], s = 0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        v[j] = i0 + j < n ? counts[i0 + j] : 0;
+        s += v[j];
+    }
+    int inc = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    if (lane == 31) ws[w] = inc;
+    __syncthreads();
+    int run = inc - s;
+    for (int i = 0; i < w; ++i) run += ws[i];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        if (i0 + j < n) counts[i0 + j] = run;
+        run += v[j];
+    }
+    if (tid == 255) totals[blockIdx.x] = run;
+    if (last_block(ticket) && tid == 0) {
+        int64_t t = 0;
+        for (int b = 0; b < (int)gridDim.x; ++b) {
+            const int64_t x = __ldcg(totals + b);
+            totals[b] = t;
+            t += x;
+        }
     }
 }
 
+__global__ void __launch_bounds__(256) k_chunk_positions(const uint8_t *__restrict__ mask, int64_t len, int nch,
+                                                         const int32_t *__restrict__ starts,
+                                                         const int64_t *__restrict__ totals, int64_t total, int N, int ndims,
+                                                         int32_t *__restrict__ pos) {
+    // per warp: the flagged cells of 512, as offsets from the chunk's first, in order
+    __shared__ uint16_t cells[8][512];
+    const int w = threadIdx.x >> 5, c = blockIdx.x * 8 + w, lane = threadIdx.x & 31;
+    if (c >= nch) return;
+    int64_t out = totals[c >> 12] + starts[c];
+    const int64_t end = c + 1 < nch ? totals[(c + 1) >> 12] + starts[c + 1] : total;
+    if (out == end) return;
+    // the chunk's first cell; a cell d further on has x0 + d, carried by 32-bit divisions
+    const int64_t base = (int64_t)c * kChunk;
+    const unsigned n = (unsigned)N;
+    const unsigned row = (unsigned)(base / N), x0 = (unsigned)(base - (int64_t)row * N);   // rows: N^2 < 2^32
+    for (int it = 0; it < kChunk / 512 && out < end; ++it) {
+        const uint4 v = mask16(mask, base + it * 512 + lane * 16, len);
+        const int cnt = count16(v);
+        int inc = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        const int tot = __shfl_sync(0xffffffffu, inc, 31);
+        if (tot == 0) continue;   // the same in the whole warp
+        int q = inc - cnt;
+        for (unsigned bits = bits16(v); bits; bits &= bits - 1)
+            cells[w][q++] = (uint16_t)(it * 512 + lane * 16 + __ffs((int)bits) - 1);
+        __syncwarp();
+        for (int e = lane; e < tot; e += 32) {
+            const unsigned xx = x0 + cells[w][e], cy = xx / n, x = xx - cy * n, r = row + cy;
+            int32_t *o = pos + (out + e) * ndims;
+            if (ndims == 2) {
+                o[0] = (int32_t)x;
+                o[1] = (int32_t)r;
+            } else {
+                const unsigned z = r / n;
+                o[0] = (int32_t)z;
+                o[1] = (int32_t)(r - z * n);
+                o[2] = (int32_t)x;
+            }
+        }
+        __syncwarp();
+        out += tot;
+    }
+}
+
+// Neighbouring-plaquette pairs of s_run.cpp:101-109, consecutive entries a, b of
+// the ascending list with b = a + 1 in the same row or b = a + N, straight from
+// the mask: the entry after a is a + 1 if that is flagged; otherwise it is a + N if that is
+// flagged and nothing between is (the warp looks at those cells together).
+// (The list it was counted from before took a count, a scan, a write and two
+// more synchronisations per search: 29 us of kernels at 128^2, against 6.) The last
+// block hands the counts of flagged cells and pairs to the host.
+__global__ void __launch_bounds__(256) k_pairs2(const uint8_t *__restrict__ mask, int64_t len, int N,
+                                                unsigned long long *tally, unsigned *ticket, int64_t *hout) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nwarp = (int64_t)gridDim.x * 8;
+    int local = 0;
+    for (int64_t u = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); u * 512 < len; u += nwarp) {
+        const int64_t m0 = u * 512 + lane * 16;
+        unsigned bits = bits16(mask16(mask, m0, len));
+        // bit 16: the cell after this lane's sixteen
+        const unsigned after = __shfl_down_sync(0xffffffffu, bits, 1) & 1u;
+        unsigned next = bits >> 1 | (lane < 31 ? after : (bits >> 15 && m0 + 16 < len ? (unsigned)mask[m0 + 16] : 0u)) << 15;
+        for (unsigned b = bits & next; b; b &= b - 1)   // a and a + 1
+            if ((m0 + __ffs((int)b)) % N != 0) ++local;   // (a + 1) % N: the same row
+        unsigned alone = bits & ~next;
+        while (__any_sync(0xffffffffu, alone)) {
+            int64_t a = -1;   // the lane's next flagged cell whose successor is not: is a + N flagged?
+            if (alone) {
+                a = m0 + __ffs((int)alone) - 1;
+                alone &= alone - 1;
+                if (a + N >= len || !mask[a + N]) a = -1;
+            }
+            for (unsigned cand = __ballot_sync(0xffffffffu, a >= 0); cand; cand &= cand - 1) {
+                const int64_t from = __shfl_sync(0xffffffffu, a, __ffs((int)cand) - 1);
+                int between = 0;
+                for (int64_t o = from + 1 + lane; o < from + N; o += 32) between |= mask[o];
+                if (!__any_sync(0xffffffffu, between) && lane == 0) ++local;
+            }
+        }
+    }
+    local = __reduce_add_sync(0xffffffffu, local);
+    if (lane == 0 && local) atomicAdd(&tally[1], (unsigned long long)local);
+    if (last_block(ticket) && threadIdx.x == 0) {
+        hout[0] = (int64_t)__ldcg(&tally[0]);
+        hout[1] = (int64_t)__ldcg(&tally[1]);
+        tally[0] = tally[1] = 0;
+    }
+}
+
+// The counters of a search on a caller's theta to the host, for the 3D case.
+__global__ void k_take_tally(unsigned long long *tally, int64_t *hout) {
+    hout[0] = (int64_t)tally[0];
+    tally[0] = tally[1] = 0;
+}
+
+double *host_slot(Lattice *L) {
+    if (!L->hslot) AXS_CUDA(cudaHostAlloc((void **)&L->hslot, kHostSlot * sizeof(double), cudaHostAllocDefault));
+    return L->hslot;
+}
+
+static int64_t chunk_count(const Lattice *L) { return (L->length + kChunk - 1) / kChunk; }
 static void ensure_mask(Lattice *L) {
     if (!L->dmask) L->dmask = (uint8_t *)dalloc((size_t)L->length);
-    if (!L->dcount) L->dcount = (int64_t *)dalloc(4 * sizeof(int64_t));
+    // counts, then the scan's block totals
+    if (!L->dchunk) L->dchunk = (int32_t *)dalloc((size_t)chunk_count(L) * 4 + 16 + (size_t)(chunk_count(L) / 4096 + 1) * 8);
 }
 
 // A work buffer of at least `bytes` in the lattice's slot (allocated once, grown
@@ -510,49 +693,47 @@ static void *lattice_tmp(Lattice *L, int slot, size_t bytes) {
     return L->tmp[slot];
 }
 
-// Build the ascending list of flagged offsets from the device mask.
-static int64_t compact(Lattice *L) {
-    int64_t nch = (L->length + kChunk - 1) / kChunk;
-    int64_t *counts = (int64_t *)lattice_tmp(L, 0, (size_t)nch * sizeof(int64_t));
-    int64_t total = 0;
-    {
-        k_chunk_counts<<<(unsigned)nch, 256, 0, L->stream>>>(L->dmask, L->length, counts);
-        k_scan<<<1, 1024, 0, L->stream>>>(counts, nch, L->dcount + 2);
-        count_launches(2);
-        AXS_CUDA(cudaGetLastError());
-        AXS_CUDA(cudaMemcpyAsync(&total, L->dcount + 2, sizeof(int64_t), cudaMemcpyDeviceToHost, L->stream));
-        AXS_CUDA(cudaStreamSynchronize(L->stream));
-        if (total > L->list_cap) {
-            dfree(L->dlist);
-            L->dlist = nullptr;
-            L->list_cap = std::max<int64_t>(total, 1024);
-            L->dlist = (int32_t *)dalloc((size_t)L->list_cap * sizeof(int64_t));
-        }
-        k_chunk_write<<<(unsigned)nch, 256, 0, L->stream>>>(L->dmask, L->length, counts, (int64_t *)L->dlist);
-        count_launches(1);
-        AXS_CUDA(cudaGetLastError());
-        AXS_CUDA(cudaStreamSynchronize(L->stream));
+// The flagged cells' positions into dlist, ascending.
+static void list_positions(Lattice *L) {
+    const int64_t total = L->last_nplaq;
+    const int nch = (int)chunk_count(L), nd = L->p.NDIMS, blocks = (nch + 7) / 8;
+    int64_t *totals = (int64_t *)((char *)L->dchunk + ((size_t)nch * 4 + 15) / 16 * 16);
+    if (total * nd > L->list_cap) {
+        dfree(L->dlist);
+        L->dlist = nullptr;
+        L->list_cap = 0;
+        const int64_t cap = std::max<int64_t>(total * nd + total * nd / 4, 4096);
+        L->dlist = (int32_t *)dalloc((size_t)cap * sizeof(int32_t));
+        L->list_cap = cap;
     }
+    if (!L->chunks_valid) {
+        k_chunk_counts<<<blocks, 256, 0, L->stream>>>(L->dmask, L->length, nch, L->dchunk);
+        count_launches(1);
+    }
+    L->chunks_valid = false;   // scanned in place
+    k_chunk_scan<<<(nch + 4095) / 4096, 256, 0, L->stream>>>(L->dchunk, nch, totals, L->dticket);
+    k_chunk_positions<<<blocks, 256, 0, L->stream>>>(L->dmask, L->length, nch, L->dchunk, totals, total, L->p.N, nd, L->dlist);
+    AXS_CUDA(cudaGetLastError());
+    count_launches(2);
     L->list_valid = true;
-    return total;
 }
 
+// The search from psi. chunks: the 3D finder's counts per chunk (or nullptr);
+// hout: where the 3D finder's last block puts the count (or nullptr).
 template <typename T>
-static void launch_cores(Lattice *L, bool from_theta, double accept, unsigned long long *cnt) {
+static void launch_cores(Lattice *L, double accept, int32_t *chunks, int64_t *hout) {
     typedef typename Cplx<T>::type C;
     const C *psi = (const C *)L->psi[L->cur];
-    int g = grid_cap(L->length, 256, 8);
-    int N = L->p.N;
+    const int N = L->p.N;
     if (L->p.NDIMS == 2) {
-        if (from_theta) k_cores<T, 2, true><<<g, 256, 0, L->stream>>>(psi, L->dtheta, L->dmask, N, L->length, accept, cnt);
-        else k_cores<T, 2, false><<<g, 256, 0, L->stream>>>(psi, nullptr, L->dmask, N, L->length, accept, cnt);
+        const dim3 grid((N + kCX - 1) / kCX, (N + kCY - 1) / kCY);
+        k_cores2_tiled<T><<<grid, 256, 0, L->stream>>>(psi, L->dmask, N, accept, L->dtally);
     } else {
-        if (from_theta) k_cores<T, 3, true><<<g, 256, 0, L->stream>>>(psi, L->dtheta, L->dmask, N, L->length, accept, cnt);
-        else {
-            dim3 grid((N + kCX - 1) / kCX, (N + kCY - 1) / kCY, (N + kCZ - 1) / kCZ);
-            if ((N & 3) == 0) k_cores3_tiled<T, true><<<grid, 256, 0, L->stream>>>(psi, L->dmask, N, accept, cnt);
-            else k_cores3_tiled<T, false><<<grid, 256, 0, L->stream>>>(psi, L->dmask, N, accept, cnt);
-        }
+        const dim3 grid((N + kCX - 1) / kCX, (N + kCY - 1) / kCY, (N + kCZ - 1) / kCZ);
+        if ((N & 3) == 0)
+            k_cores3_tiled<T, true><<<grid, 256, 0, L->stream>>>(psi, L->dmask, N, accept, L->dtally, chunks, L->dticket, hout);
+        else
+            k_cores3_tiled<T, false><<<grid, 256, 0, L->stream>>>(psi, L->dmask, N, accept, L->dtally, chunks, L->dticket, hout);
     }
     AXS_CUDA(cudaGetLastError());
     count_launches(1);
@@ -560,60 +741,47 @@ static void launch_cores(Lattice *L, bool from_theta, double accept, unsigned lo
 
 void find_strings(Lattice *L, const double *theta_host, uint8_t *mask_host, int64_t *nplaq, int64_t *ncores) {
     ensure_mask(L);
-    bool from_theta = theta_host != nullptr;
-    if (from_theta) {
+    int64_t *h = (int64_t *)host_slot(L);
+    const double accept = (double)(0.5f * (1.0f - L->p.thr / 100.0f));   // string_finding.cpp:8,40
+    const int N = L->p.N, nd = L->p.NDIMS;
+    L->chunks_valid = false;
+    if (theta_host) {
         if (!L->dtheta) L->dtheta = (double *)dalloc((size_t)L->length * sizeof(double));
         AXS_CUDA(cudaMemcpyAsync(L->dtheta, theta_host, (size_t)L->length * sizeof(double), cudaMemcpyHostToDevice,
                                  L->stream));
+        const int g = grid_cap(L->length, 256, 8);
+        if (nd == 2) k_cores<2><<<g, 256, 0, L->stream>>>(L->dtheta, L->dmask, N, L->length, accept, L->dtally);
+        else k_cores<3><<<g, 256, 0, L->stream>>>(L->dtheta, L->dmask, N, L->length, accept, L->dtally);
+        if (nd == 3) k_take_tally<<<1, 1, 0, L->stream>>>(L->dtally, h);
+        AXS_CUDA(cudaGetLastError());
+        count_launches(nd == 3 ? 2 : 1);
+    } else {
+        if (nd == 3) AXS_CUDA(cudaMemsetAsync(L->dchunk, 0, (size_t)chunk_count(L) * sizeof(int32_t), L->stream));
+        if (L->esz == 4) launch_cores<float>(L, accept, L->dchunk, h);
+        else launch_cores<double>(L, accept, L->dchunk, h);
+        L->chunks_valid = nd == 3;
     }
-    int thr = L->p.thr;
-    double accept = (double)(0.5f * (1.0f - thr / 100.0f));   // string_finding.cpp:8,40
-    AXS_CUDA(cudaMemsetAsync(L->dcount, 0, 2 * sizeof(int64_t), L->stream));
-    unsigned long long *cnt = (unsigned long long *)L->dcount;
-    if (L->esz == 4) launch_cores<float>(L, from_theta, accept, cnt);
-    else launch_cores<double>(L, from_theta, accept, cnt);
-    int64_t n = 0;
-    AXS_CUDA(cudaMemcpyAsync(&n, L->dcount, sizeof(int64_t), cudaMemcpyDeviceToHost, L->stream));
+    if (nd == 2) {
+        k_pairs2<<<grid_cap(L->length, 4096, 4), 256, 0, L->stream>>>(L->dmask, L->length, N, L->dtally, L->dticket, h);
+        AXS_CUDA(cudaGetLastError());
+        count_launches(1);
+    }
     if (mask_host) AXS_CUDA(cudaMemcpyAsync(mask_host, L->dmask, (size_t)L->length, cudaMemcpyDeviceToHost, L->stream));
     AXS_CUDA(cudaStreamSynchronize(L->stream));
-    L->last_nplaq = n;
+    L->last_nplaq = h[0];
     L->list_valid = false;
-    int64_t cores = n;
-    if (L->p.NDIMS == 2) {
-        int64_t total = compact(L);
-        AXS_CUDA(cudaMemsetAsync(L->dcount + 1, 0, sizeof(int64_t), L->stream));
-        k_pairs2<<<grid_cap(std::max<int64_t>(total, 1), 256, 4), 256, 0, L->stream>>>(
-            (const int64_t *)L->dlist, total, L->p.N, (unsigned long long *)(L->dcount + 1));
-        count_launches(1);
-        AXS_CUDA(cudaGetLastError());
-        int64_t pairs = 0;
-        AXS_CUDA(cudaMemcpyAsync(&pairs, L->dcount + 1, sizeof(int64_t), cudaMemcpyDeviceToHost, L->stream));
-        AXS_CUDA(cudaStreamSynchronize(L->stream));
-        cores = n - pairs;
-    }
-    if (nplaq) *nplaq = n;
-    if (ncores) *ncores = cores;
+    if (nplaq) *nplaq = h[0];
+    if (ncores) *ncores = nd == 2 ? h[0] - h[1] : h[0];   // s_run.cpp:101-109, 112-131
 }
 
 void string_positions(Lattice *L, int32_t *pos, int64_t cap, int64_t *n) {
     if (L->last_nplaq < 0) fail(AXS_ERR_STATE, "axs_string_positions needs a preceding axs_find_strings");
-    int64_t total = L->list_valid ? L->last_nplaq : compact(L);
+    const int64_t total = L->last_nplaq, w = std::min<int64_t>(cap, total);
     if (n) *n = total;
-    int64_t w = std::min<int64_t>(cap, total);
     if (w <= 0 || !pos) return;
-    int nd = L->p.NDIMS;
-    int32_t *dpos = (int32_t *)dalloc((size_t)w * nd * sizeof(int32_t));
-    try {
-        k_positions<<<grid_cap(w, 256, 4), 256, 0, L->stream>>>((const int64_t *)L->dlist, w, L->p.N, nd, dpos);
-        count_launches(1);
-        AXS_CUDA(cudaGetLastError());
-        AXS_CUDA(cudaMemcpyAsync(pos, dpos, (size_t)w * nd * sizeof(int32_t), cudaMemcpyDeviceToHost, L->stream));
-        AXS_CUDA(cudaStreamSynchronize(L->stream));
-    } catch (...) {
-        dfree(dpos);
-        throw;
-    }
-    dfree(dpos);
+    if (!L->list_valid) list_positions(L);
+    AXS_CUDA(cudaMemcpyAsync(pos, L->dlist, (size_t)w * L->p.NDIMS * sizeof(int32_t), cudaMemcpyDeviceToHost, L->stream));
+    AXS_CUDA(cudaStreamSynchronize(L->stream));
 }
 
 // ============================================================== spectra
@@ -1371,14 +1539,8 @@ struct ZStage {
 template <typename T, int R, int W, int TW>
 __device__ __forceinline__ void tile_stencil(const typename Cplx<T>::type *t, const typename Cplx<T>::type (&zr)[W],
                                              int g, T &L1, T &L2) {
+    static_assert(R > 1, "radius 1: sync_pi_r1");
     const auto &ctr = zr[g % W];
-    if constexpr (R == 1) {   // lap7's order, as stencil_at forms radius 1
-        const auto xm = t[-1], xp = t[1], ym = t[-TW], yp = t[TW];
-        const auto &zm = zr[(g + W - 1) % W], &zp = zr[(g + 1) % W];
-        L1 = lap7<T>(ctr.x, xm.x, xp.x, ym.x, yp.x, zm.x, zp.x);
-        L2 = lap7<T>(ctr.y, xm.y, xp.y, ym.y, yp.y, zm.y, zp.y);
-        return;
-    }
     T a1 = (T)stencil_coef(R - 1, 3, 0) * ctr.x, a2 = (T)stencil_coef(R - 1, 3, 0) * ctr.y;
 #pragma unroll
     for (int l = 1; l <= R; ++l) {
@@ -1425,6 +1587,7 @@ __device__ __forceinline__ void zcol_march(const typename Cplx<T>::type *__restr
         st.issue(psi, pih, (int64_t)((za + a) % N) * NN, a, tiles, pown, active, col);
         cp_async_commit();
     }
+    const T kctr = c.kdt_idx2 * (T)-6;
     C zr[W];   // at a trip's start z0: zr[j] = plane z0 - R - 1 + j
 #pragma unroll
     for (int j = 1; j < W; ++j) zr[j] = psi[(int64_t)((za + N + j - R - 1) % N) * NN + col];
@@ -1451,9 +1614,13 @@ __device__ __forceinline__ void zcol_march(const typename Cplx<T>::type *__restr
                     C p = pown[slot * 256 + threadIdx.x];
                     const C zc = zr[(h + R + 1) % W], zp = zr[(h + R + 2) % W];
                     if (!fresh) {   // a fresh state holds pi_0 itself (the reference's ker is zero)
-                        T L1, L2;
-                        tile_stencil<T, R, W, M::TW>(ts, zr, h + R + 1, L1, L2);
-                        sync_pi_site<T>(zc.x, zc.y, L1, L2, p.x, p.y, c);
+                        if constexpr (R == 1) {
+                            sync_pi_r1<T, 3>(zc, vnsum(ts[-1], ts[1], ts[-M::TW], ts[M::TW], zr[(h + R) % W], zp), p, c, kctr);
+                        } else {
+                            T L1, L2;
+                            tile_stencil<T, R, W, M::TW>(ts, zr, h + R + 1, L1, L2);
+                            sync_pi_site<T>(zc.x, zc.y, L1, L2, p.x, p.y, c);
+                        }
                     }
                     site(h, z, zc, zp, p, ts);
                 }
@@ -1519,13 +1686,51 @@ __global__ void __launch_bounds__(256, (ZMarch<T, R>::MINB))
     });
 }
 
-// The same for 2D: one thread per site of 32 x 8 tiles, the neighbours from
-// L1/L2 (the lattice fits L2 up to 3000^2).
-template <typename T, int R, bool SOA>
+// pi_n of the 2D site (x, y) with psi f, its neighbours from L1/L2 (the lattice
+// fits L2 up to 2000^2); xp and yp are the forward neighbours.
+template <typename T, int R>
+__device__ __forceinline__ typename Cplx<T>::type sync_site_2d(const typename Cplx<T>::type *__restrict__ psi,
+                                                               const typename Cplx<T>::type *__restrict__ pih, int N, int x,
+                                                               int y, const typename Cplx<T>::type &f, int fresh,
+                                                               const StepCoefs<T> &c, typename Cplx<T>::type &xp1,
+                                                               typename Cplx<T>::type &yp1) {
+    typedef typename Cplx<T>::type C;
+    const int row = y * N;
+    C p = pih[row + x];
+    T L1 = 0, L2 = 0;
+    if constexpr (R > 1) {
+        L1 = (T)stencil_coef(R - 1, 2, 0) * f.x;
+        L2 = (T)stencil_coef(R - 1, 2, 0) * f.y;
+    }
+#pragma unroll
+    for (int l = 1; l <= R; ++l) {
+        const C xm = psi[row + (x < l ? x - l + N : x - l)], xp = psi[row + (x + l >= N ? x + l - N : x + l)];
+        const C ym = psi[(y < l ? y - l + N : y - l) * N + x], yp = psi[(y + l >= N ? y + l - N : y + l) * N + x];
+        if (l == 1) {
+            xp1 = xp;
+            yp1 = yp;
+        }
+        if constexpr (R == 1) {
+            if (!fresh) sync_pi_r1<T, 2>(f, vnsum(xm, xp, ym, yp), p, c, c.kdt_idx2 * (T)-4);
+        } else {
+            const T w = (T)stencil_coef(R - 1, 2, l);
+            L1 = fma(w, nsum5<T>(xm.x, xp.x, ym.x, yp.x), L1);
+            L2 = fma(w, nsum5<T>(xm.y, xp.y, ym.y, yp.y), L2);
+        }
+    }
+    if constexpr (R > 1)
+        if (!fresh) sync_pi_site<T>(f.x, f.y, L1, L2, p.x, p.y, c);
+    return p;
+}
+
+// The snapshot and pi_n alone for 2D, and the axion field (MODE 0: pi_n as
+// complex values into out.f[0], 1: all four fields, 2: the axion field into
+// out.f[0]): one thread per site of 32 x 8 tiles.
+template <typename T, int R, int MODE>
 __global__ void __launch_bounds__(256)
     k_sync_2d(const typename Cplx<T>::type *__restrict__ psi, const typename Cplx<T>::type *__restrict__ pih, SnapOut<T> out,
               const double *clock, int N, double dt, double inv_dx2, double lambda, double T0sq3, int prs, int form,
-              int fresh) {
+              int fresh, double itau) {
     typedef typename Cplx<T>::type C;
     const StepCoefs<T> c = block_coefs<T>(clock, dt, 0.5 * dt, inv_dx2, lambda, T0sq3, prs, form);
     const int nbx = (N + 31) / 32, nt = nbx * ((N + 7) / 8);
@@ -1534,67 +1739,66 @@ __global__ void __launch_bounds__(256)
         if (x >= N || y >= N) continue;
         const int m = y * N + x;
         const C f = psi[m];
-        C p = pih[m];
-        if (!fresh) {   // stencil_at's sums: radius 1 as lap5, else the weights in order
-            T L1, L2;
-            if constexpr (R > 1) {
-                L1 = (T)stencil_coef(R - 1, 2, 0) * f.x;
-                L2 = (T)stencil_coef(R - 1, 2, 0) * f.y;
-            }
-#pragma unroll
-            for (int l = 1; l <= R; ++l) {
-                const C xm = psi[m - x + (x < l ? x - l + N : x - l)], xp = psi[m - x + (x + l >= N ? x + l - N : x + l)];
-                const C ym = psi[(y < l ? y - l + N : y - l) * N + x], yp = psi[(y + l >= N ? y + l - N : y + l) * N + x];
-                if constexpr (R == 1) {
-                    L1 = lap5<T>(f.x, xm.x, xp.x, ym.x, yp.x);
-                    L2 = lap5<T>(f.y, xm.y, xp.y, ym.y, yp.y);
-                } else {
-                    const T w = (T)stencil_coef(R - 1, 2, l);
-                    L1 = fma(w, nsum5<T>(xm.x, xp.x, ym.x, yp.x), L1);
-                    L2 = fma(w, nsum5<T>(xm.y, xp.y, ym.y, yp.y), L2);
-                }
-            }
-            sync_pi_site<T>(f.x, f.y, L1, L2, p.x, p.y, c);
-        }
-        if constexpr (SOA) {
+        C xp, yp;
+        const C p = sync_site_2d<T, R>(psi, pih, N, x, y, f, fresh, c, xp, yp);
+        if constexpr (MODE == 1) {
             out.f[0][m] = f.x;
             out.f[1][m] = f.y;
             out.f[2][m] = p.x;
             out.f[3][m] = p.y;
-        } else {
+        } else if constexpr (MODE == 0) {
             reinterpret_cast<C *>(out.f[0])[m] = p;
+        } else {
+            out.f[0][m] = axion_f<T>(f.x, f.y, p.x, p.y, (T)itau);
         }
     }
 }
 
-template <typename T, int R, bool SOA>
-static void sync_fd_r(Lattice *L, const SnapOut<T> &out) {
+template <typename T, int R, int MODE>
+static void sync_2d_r(Lattice *L, const SnapOut<T> &out) {
     typedef typename Cplx<T>::type C;
     const axs_params &p = L->p;
-    const double dx = p.space_step, T0 = p.T_initial, dt = p.time_step, idx2 = 1.0 / (dx * dx), la = p.lambda;
-    const C *f = (const C *)L->psi[L->cur], *q = (const C *)L->pih;
-    const double *clk = L->dclock + L->cur;
-    if (p.NDIMS == 2) {
-        const int nt = ((p.N + 31) / 32) * ((p.N + 7) / 8);
-        k_sync_2d<T, R, SOA><<<std::min(nt, num_sms() * 8), 256, 0, L->stream>>>(f, q, out, clk, p.N, dt, idx2, la,
-                                                                                (T0 * T0) / 3.0, p.prs, p.form, L->fresh);
-    } else {
-        const size_t smem = ZMarch<T, R>::SMEM;
-        AXS_CUDA(cudaFuncSetAttribute(k_sync_zcol<T, R, SOA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_sync_zcol<T, R, SOA><<<zcol_grid<T, R>(p.N), 256, smem, L->stream>>>(f, q, out, clk, p.N, dt, idx2, la,
-                                                                            (T0 * T0) / 3.0, p.prs, p.form, L->fresh);
+    const double dx = p.space_step, T0 = p.T_initial;
+    const int nt = ((p.N + 31) / 32) * ((p.N + 7) / 8);
+    k_sync_2d<T, R, MODE><<<std::min(nt, num_sms() * 8), 256, 0, L->stream>>>(
+        (const C *)L->psi[L->cur], (const C *)L->pih, out, L->dclock + L->cur, p.N, (double)p.time_step, 1.0 / (dx * dx),
+        (double)p.lambda, (T0 * T0) / 3.0, p.prs, p.form, L->fresh, 1.0 / L->tau);
+}
+template <typename T, int MODE>
+static void sync_2d(Lattice *L, const SnapOut<T> &out) {
+    switch (L->p.stencil_setting) {
+    case 0: sync_2d_r<T, 1, MODE>(L, out); break;
+    case 1: sync_2d_r<T, 2, MODE>(L, out); break;
+    case 2: sync_2d_r<T, 3, MODE>(L, out); break;
+    default: sync_2d_r<T, 4, MODE>(L, out); break;
     }
-    AXS_CUDA(cudaGetLastError());
-    count_launches(1);
+}
+
+template <typename T, int R, bool SOA>
+static void sync_3d_r(Lattice *L, const SnapOut<T> &out) {
+    typedef typename Cplx<T>::type C;
+    const axs_params &p = L->p;
+    const double dx = p.space_step, T0 = p.T_initial;
+    const size_t smem = ZMarch<T, R>::SMEM;
+    AXS_CUDA(cudaFuncSetAttribute(k_sync_zcol<T, R, SOA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_sync_zcol<T, R, SOA><<<zcol_grid<T, R>(p.N), 256, smem, L->stream>>>(
+        (const C *)L->psi[L->cur], (const C *)L->pih, out, L->dclock + L->cur, p.N, (double)p.time_step, 1.0 / (dx * dx),
+        (double)p.lambda, (T0 * T0) / 3.0, p.prs, p.form, L->fresh);
 }
 template <typename T, bool SOA>
 static void sync_fd(Lattice *L, const SnapOut<T> &out) {
-    switch (L->p.stencil_setting) {
-    case 0: sync_fd_r<T, 1, SOA>(L, out); break;
-    case 1: sync_fd_r<T, 2, SOA>(L, out); break;
-    case 2: sync_fd_r<T, 3, SOA>(L, out); break;
-    default: sync_fd_r<T, 4, SOA>(L, out); break;
+    if (L->p.NDIMS == 2) {
+        sync_2d<T, SOA ? 1 : 0>(L, out);
+    } else {
+        switch (L->p.stencil_setting) {
+        case 0: sync_3d_r<T, 1, SOA>(L, out); break;
+        case 1: sync_3d_r<T, 2, SOA>(L, out); break;
+        case 2: sync_3d_r<T, 3, SOA>(L, out); break;
+        default: sync_3d_r<T, 4, SOA>(L, out); break;
+        }
     }
+    AXS_CUDA(cudaGetLastError());
+    count_launches(1);
 }
 void sync_pi_fd(Lattice *L) {
     if (L->esz == 4) sync_fd<float, false>(L, SnapOut<float>{{(float *)L->scratch}});
@@ -1685,7 +1889,7 @@ struct BinPending {
 
 template <typename B>
 static BinPending bin_spectrum_enqueue(Lattice *L, const B &binner, int kind, const std::vector<int> &edges, int nbins,
-                                       double *host) {
+                                       double *host, bool pinned) {
     const Lattice::BinGeom *geom = nullptr;
     for (const Lattice::BinGeom &g : L->bin_geom)
         if (g.kind == kind && g.edges == edges) geom = &g;
@@ -1724,7 +1928,7 @@ static BinPending bin_spectrum_enqueue(Lattice *L, const B &binner, int kind, co
     const int64_t units = groups * ((nh + seg - 1) / seg);
     if (units >= ((int64_t)1 << 31)) fail(AXS_ERR_ARG, "spectrum of N = %d: too many row groups", N);
     int nblk = (int)std::min<int64_t>((int64_t)num_sms() * per_sm, (units + 3) / 4);   // whole units per warp
-    double *part = (double *)lattice_tmp(L, 1, (size_t)nblk * 3 * nbp * sizeof(double) + (size_t)3 * nbp * sizeof(double));
+    double *part = (double *)lattice_tmp(L, 0, (size_t)nblk * 3 * nbp * sizeof(double) + (size_t)3 * nbp * sizeof(double));
     double *out = part + (size_t)nblk * 3 * nbp;
     auto kern = L->esz == 4 ? (ks ? (const void *)k_bin_runs<float, B, true> : (const void *)k_bin_runs<float, B, false>)
                             : (ks ? (const void *)k_bin_runs<double, B, true> : (const void *)k_bin_runs<double, B, false>);
@@ -1739,13 +1943,15 @@ static BinPending bin_spectrum_enqueue(Lattice *L, const B &binner, int kind, co
             else k_bin_runs<double, B, false><<<nblk, 128, sm, L->stream>>>((const double2 *)L->fft_out, N, L->p.NDIMS, binner, nbins, seg, b0, nb, part, L->derr);
         }
         AXS_CUDA(cudaGetLastError());
-        k_bin_final3<<<nb, 256, 0, L->stream>>>(part, nblk, nb, out);
+        // rows (power, |n|, count) of this pass at host[3 b0 ..], which the kernel
+        // writes itself when host is page-locked; otherwise the next pass
+        // overwrites `out` only after this copy (stream order)
+        k_bin_final3<<<nb, 256, 0, L->stream>>>(part, nblk, nb, pinned ? host + 3 * (size_t)b0 : out);
         AXS_CUDA(cudaGetLastError());
         count_launches(2);
-        // rows (power, |n|, count) of this pass at host[3 b0 ..]; the next pass
-        // overwrites `out` only after this copy (stream order)
-        AXS_CUDA(cudaMemcpyAsync(host + 3 * (size_t)b0, out, 3 * (size_t)nb * sizeof(double), cudaMemcpyDeviceToHost,
-                                 L->stream));
+        if (!pinned)
+            AXS_CUDA(cudaMemcpyAsync(host + 3 * (size_t)b0, out, 3 * (size_t)nb * sizeof(double), cudaMemcpyDeviceToHost,
+                                     L->stream));
     }
     // the lattice's error flag into the slot after the rows (host holds 3 nbins + 1 doubles)
     AXS_CUDA(cudaMemcpyAsync(host + 3 * (size_t)nbins, L->derr, sizeof(int), cudaMemcpyDeviceToHost, L->stream));
@@ -1803,13 +2009,22 @@ static void bin_spectrum_finish(Lattice *L, const BinPending &pd, std::vector<do
     cnt = geom->cnt;
 }
 
+// Where a call's rows and error flag land: the lattice's page-locked slot when
+// they fit it, else `own` (a pageable destination makes each copy complete
+// before the call returns).
+static double *rows_host(Lattice *L, int nbins, std::vector<double> &own) {
+    if (3 * (size_t)nbins + 1 <= (size_t)kHostSlot) return host_slot(L);
+    own.resize(3 * (size_t)nbins + 1);
+    return own.data();
+}
+
 // Bin the current fft_out; returns per-bin sums (pk, |n|) and weighted counts.
-// A pageable destination makes each copy complete before the call returns.
 template <typename B>
 static void bin_spectrum(Lattice *L, const B &binner, int kind, const std::vector<int> &edges, int nbins,
                          std::vector<double> &psum, std::vector<double> &nsum, std::vector<unsigned long long> &cnt) {
-    std::vector<double> h(3 * (size_t)nbins + 1);   // rows, then the error flag
-    const BinPending pd = bin_spectrum_enqueue(L, binner, kind, edges, nbins, h.data());
+    std::vector<double> own;
+    double *h = rows_host(L, nbins, own);
+    const BinPending pd = bin_spectrum_enqueue(L, binner, kind, edges, nbins, h, own.empty());
     AXS_CUDA(cudaStreamSynchronize(L->stream));
     bin_spectrum_finish(L, pd, psum, nsum, cnt);
 }
@@ -1853,13 +2068,16 @@ struct AxionPending {
     std::vector<int> thr;
 };
 
-static AxionPending axion_spectrum_enqueue(Lattice *L, int nbins, double *host, int *thr_host) {
+static AxionPending axion_spectrum_enqueue(Lattice *L, int nbins, double *host, int *thr_host, bool pinned) {
     if (nbins < 1) fail(AXS_ERR_ARG, "nbins must be >= 1");
     if (L->p.form != 0) fail(AXS_ERR_STATE, "the axion kinetic spectrum is defined on the field-rescaled variables (form 0)");
     ensure_fft(L);
     if (L->p.NDIMS == 3 && L->p.laplacian == 0) {
         if (L->esz == 4) axion_zcol_t<float>(L);
         else axion_zcol_t<double>(L);
+    } else if (L->p.laplacian == 0) {
+        if (L->esz == 4) sync_2d<float, 2>(L, SnapOut<float>{{(float *)L->fft_in}});
+        else sync_2d<double, 2>(L, SnapOut<double>{{(double *)L->fft_in}});
     } else {
         launch_sync_pi(L);
         int g = grid_cap(L->length, 256, 16);
@@ -1881,15 +2099,19 @@ static AxionPending axion_spectrum_enqueue(Lattice *L, int nbins, double *host, 
     AxionPending pd;
     pd.thr.assign(nbins, 0);
     for (int b = 1; b < nbins; ++b) { double t = exp(log(ratio) * (double)b / (double)nbins); pd.thr[b] = (int)ceil(t * t); }
-    int *de2 = (int *)lattice_tmp(L, 2, nbins * sizeof(int));
-    const int *src = pd.thr.data();
-    if (thr_host) {
-        memcpy(thr_host, pd.thr.data(), nbins * sizeof(int));
-        src = thr_host;
+    int *de2 = (int *)lattice_tmp(L, 1, nbins * sizeof(int));
+    if (L->thr_on_device != pd.thr) {   // the thresholds stay on the device while the binning is the same
+        L->thr_on_device.clear();
+        const int *src = pd.thr.data();
+        if (thr_host) {
+            memcpy(thr_host, pd.thr.data(), nbins * sizeof(int));
+            src = thr_host;
+        }
+        AXS_CUDA(cudaMemcpyAsync(de2, src, nbins * sizeof(int), cudaMemcpyHostToDevice, L->stream));
+        L->thr_on_device = pd.thr;
     }
-    AXS_CUDA(cudaMemcpyAsync(de2, src, nbins * sizeof(int), cudaMemcpyHostToDevice, L->stream));
     pd.bin = bin_spectrum_enqueue(L, LogBinsI{de2, nbins, (float)((double)nbins / log2(ratio * ratio))}, 1, pd.thr,
-                                  nbins, host);
+                                  nbins, host, pinned);
     return pd;
 }
 
@@ -1913,8 +2135,9 @@ static void axion_spectrum_finish(Lattice *L, const AxionPending &pd, double *km
 }
 
 void axion_spectrum(Lattice *L, int nbins, double *kmean, double *pk, int64_t *count) {
-    std::vector<double> h(3 * (size_t)std::max(nbins, 1) + 1);   // rows, then the error flag
-    const AxionPending pd = axion_spectrum_enqueue(L, nbins, h.data(), nullptr);
+    std::vector<double> own;
+    double *h = rows_host(L, std::max(nbins, 1), own);
+    const AxionPending pd = axion_spectrum_enqueue(L, nbins, h, nullptr, own.empty());
     AXS_CUDA(cudaStreamSynchronize(L->stream));
     axion_spectrum_finish(L, pd, kmean, pk, count);
 }
@@ -1995,17 +2218,14 @@ void ensemble_find_strings(Ensemble *E, int64_t *nplaq, int64_t *ncores) {
     ensemble_fan_out(E, [&](Lattice *L, size_t i) {
         ensure_mask(L);
         const double accept = (double)(0.5f * (1.0f - L->p.thr / 100.0f));   // string_finding.cpp:8,40
-        AXS_CUDA(cudaMemsetAsync(L->dcount, 0, 2 * sizeof(int64_t), L->stream));
-        unsigned long long *cnt = (unsigned long long *)L->dcount;
-        if (L->esz == 4) launch_cores<float>(L, false, accept, cnt);
-        else launch_cores<double>(L, false, accept, cnt);
-        AXS_CUDA(cudaMemcpyAsync(&hc[i], L->dcount, sizeof(int64_t), cudaMemcpyDeviceToHost, L->stream));
+        if (L->esz == 4) launch_cores<float>(L, accept, nullptr, &hc[i]);
+        else launch_cores<double>(L, accept, nullptr, &hc[i]);
     });
     AXS_CUDA(cudaStreamSynchronize(E->stream));
     for (size_t i = 0; i < n; ++i) {
         Lattice *L = E->members[i];
         L->last_nplaq = hc[i];
-        L->list_valid = false;
+        L->list_valid = L->chunks_valid = false;
         nplaq[i] = hc[i];
         ncores[i] = hc[i];   // 3D: every flagged plaquette counts (s_run.cpp:112-131)
     }
@@ -2021,7 +2241,7 @@ void ensemble_axion_spectrum(Ensemble *E, int nbins, double *kmean, double *pk, 
     ensemble_fan_out(E, [&](Lattice *L, size_t i) {
         double *h = (double *)(base + i * per);
         int *t = (int *)(base + i * per + (3 * (size_t)nbins + 2) * sizeof(double));
-        pend[i] = axion_spectrum_enqueue(L, nbins, h, t);
+        pend[i] = axion_spectrum_enqueue(L, nbins, h, t, true);
     });
     AXS_CUDA(cudaStreamSynchronize(E->stream));
     for (size_t i = 0; i < n; ++i)
@@ -2054,53 +2274,62 @@ template <> struct Acc<double> {
 __device__ __forceinline__ float abs_theta(float a, float b) { return fabsf(fast_atan2(a, b)); }
 // FP64 fields: |atan2(a, b)| and |(a, b)| to double precision at a fraction
 // of the library's FP64 cost (GB300's FP64 pipe bounds the FP64 means). The
-// float angle picks the nearest of the angles k pi/128 (k = -128 .. 128); the
-// vector (b, a) is rotated by -k pi/128 with that angle's double cosine and
+// float angle picks the nearest of the angles k pi/512 (k = -512 .. 512); the
+// vector (b, a) is rotated by -k pi/512 with that angle's double cosine and
 // sine (formed on the host) to (x, y), a small angle from the x axis. With
-// u = y/x (the reciprocal from the float one by two Newton-Raphson steps,
-// within an ulp), |u| < 0.0125: the remainder angle atan(u) is the Taylor
-// series to u^7 and |(a, b)| = x sqrt(1 + u^2) the binomial series to u^6
-// (truncations below 3e-17). Vectors outside that (a zero, tiny, huge or
-// non-finite component) take the library's atan2 and square root. The angle
-// is brought back to [-pi, pi] before its magnitude.
-__device__ double2 g_theta_rot[257];   // (cos, sin) of k pi/128 at index k + 128
-__device__ __forceinline__ void abs_phi_theta(double a, double b, double &aphi, double &ath) {
-    const float t0 = fast_atan2((float)a, (float)b);
-    const int k = __float2int_rn(t0 * 40.743665431525205f);   // 128 / pi
-    const double2 cs = g_theta_rot[k + 128];
-    const double x = fma(b, cs.x, a * cs.y), y = fma(a, cs.x, -(b * cs.y));
-    if (x > 1e-30 && x < 1e30) {
-        double r = (double)__frcp_rn((float)x);
-        r = fma(r, fma(-x, r, 1.0), r);
-        r = fma(r, fma(-x, r, 1.0), r);
-        const double u = y * r;
-        if (fabs(u) < 0.0125) {
-            const double u2 = u * u;
-            double q = fma(u2, -1.0 / 7.0, 1.0 / 5.0);
-            q = fma(u2, q, -1.0 / 3.0);
-            double t = fma(u * u2, q, u) + (double)k * (3.141592653589793 / 128.0);
-            if (t > 3.141592653589793) t -= 6.283185307179586;
-            else if (t < -3.141592653589793) t += 6.283185307179586;
-            ath = fabs(t);
-            double w = fma(u2, 1.0 / 16.0, -1.0 / 8.0);
-            w = fma(u2, w, 0.5);
-            aphi = x * fma(u2, w, 1.0);
-            return;
-        }
-    }
+// u = y/x (the reciprocal from the float one by one Newton-Raphson step, within
+// 2^-44: u is below 0.0031, so its error is below 2^-52.4, and of either sign),
+// the remainder angle
+// atan(u) is the Taylor series to u^5 (truncated below 4e-19) and |(a, b)| =
+// x sqrt(1 + u^2) the binomial series to u^4 (6e-17 of it at most). |theta| is
+// the table's |k| pi/512 plus atan(u) with k's sign: for k = +-512 the angle
+// past pi counts back from it, |theta| = pi - |atan(u)|. Signs are set in the
+// high words, ranges and conversions read from the bits (no FP64 instructions):
+// 13 FP64 operations. Vectors outside that (a zero, tiny, huge or non-finite
+// component) take the library's atan2 and square root.
+static constexpr int kRot = 512;
+struct ThetaRot {
+    double c, s, angle, pad;   // cosine and sine of k pi/512, |k| pi/512
+};
+__device__ ThetaRot g_theta_rot[2 * kRot + 1];
+__device__ __noinline__ void abs_phi_theta_lib(double a, double b, double &aphi, double &ath) {
     ath = fabs(atan2(a, b));
     aphi = sqrt(a * a + b * b);
+}
+__device__ __forceinline__ void abs_phi_theta(double a, double b, double &aphi, double &ath) {
+    const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu, eb = ((unsigned)__double2hiint(b) >> 20) & 0x7ffu;
+    const unsigned top = max(ea, eb), low = min(ea, eb);
+    if (top < 1023 + 90 && low > 1023 - 90) {   // both magnitudes within float's range, neither zero
+        const float t0 = fast_atan2(float_bits(a), float_bits(b));
+        const int k = __float2int_rn(t0 * 162.97466172610083f);   // 512 / pi
+        const ThetaRot &r = g_theta_rot[k + kRot];
+        const double x = fma(b, r.c, a * r.s), y = fma(a, r.c, -(b * r.s));   // x > 0: within a step of the axis
+        double i = double_bits(__frcp_rn(float_bits(x)));
+        i = fma(i, fma(-x, i, 1.0), i);
+        const double u = y * i, u2 = u * u;
+        double q = fma(u2, 1.0 / 5.0, -1.0 / 3.0);
+        const double t = fma(u * u2, q, u);   // atan(u)
+        // + t for k > 0, - t for k < 0, |t| for k = 0, -|t| for k = +-512
+        unsigned hi = (unsigned)__double2hiint(t);
+        if (k == 0 || k == kRot || k == -kRot) hi &= 0x7fffffffu;
+        if (k < 0 || k == kRot) hi ^= 0x80000000u;
+        ath = r.angle + __hiloint2double((int)hi, __double2loint(t));
+        q = fma(u2, -1.0 / 8.0, 0.5);
+        aphi = fma(x * u2, q, x);
+        return;
+    }
+    abs_phi_theta_lib(a, b, aphi, ath);
 }
 // the rotation table of abs_phi_theta, once per device
 static void ensure_theta_table() {
     static PerDevice done;
     done.get([] {
-        double2 tab[257];
-        for (int k = -128; k <= 128; ++k) {
-            const double t = (double)k * (3.141592653589793 / 128.0);
-            tab[k + 128] = make_double2(cos(t), sin(t));
+        std::vector<ThetaRot> tab(2 * kRot + 1);
+        for (int k = -kRot; k <= kRot; ++k) {
+            const double t = (double)k * (3.141592653589793 / kRot);
+            tab[k + kRot] = ThetaRot{cos(t), sin(t), fabs(t), 0.0};
         }
-        AXS_CUDA(cudaMemcpyToSymbol(g_theta_rot, tab, sizeof(tab)));
+        AXS_CUDA(cudaMemcpyToSymbol(g_theta_rot, tab.data(), tab.size() * sizeof(ThetaRot)));
         return 1;
     });
 }
@@ -2134,38 +2363,32 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_background(cons
                                                        const typename Cplx<T>::type *__restrict__ pih,
                                                        const double *clock, int64_t len, double dt, double lambda,
                                                        double T0sq3, int prs, int form, int fresh,
-                                                       double *__restrict__ partials) {
+                                                       double *__restrict__ partials, unsigned *ticket,
+                                                       double *__restrict__ hout) {
     typedef typename Cplx<T>::type C;
-    const StepCoefs<T> c = make_coefs<T>(*clock, dt, 0.5 * dt, 0.0, lambda, T0sq3, prs, form);
+    const StepCoefs<T> c = block_coefs<T>(clock, dt, 0.5 * dt, 0.0, lambda, T0sq3, prs, form);
     Acc<T> a[6];
     const int64_t npair = len >> 1;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    auto trip = [&](C (&f)[2], C (&p)[2]) {
-        T t[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) t[k] = 0;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (!fresh) sync_pi_site<T>(f[h].x, f[h].y, (T)0, (T)0, p[h].x, p[h].y, c);   // a fresh pih is pi_0
-            t[0] += f[h].x;
-            t[1] += f[h].y;
-            t[2] += p[h].x;
-            t[3] += p[h].y;
-            if constexpr (sizeof(T) == 8) {
-                double ap, at;
-                abs_phi_theta(f[h].x, f[h].y, ap, at);
-                t[4] += at;
-                t[5] += ap;
-            } else {
-                t[4] += abs_theta(f[h].x, f[h].y);
-                t[5] += sqrt(f[h].x * f[h].x + f[h].y * f[h].y);
-            }
+    // the six terms of one site (the half kick's local part only, see above)
+    auto terms = [&](const C &f, C p, T (&t)[6]) {
+        if (!fresh) {   // a fresh pih is pi_0
+            const T g = c.kdt_coef * fma(f.x, f.x, fma(f.y, f.y, c.c0));
+            p.x = fma(g, f.x, p.x);
+            p.y = fma(g, f.y, p.y);
         }
-#pragma unroll
-        for (int k = 0; k < 6; ++k) a[k].add(t[k]);
+        t[0] = f.x;
+        t[1] = f.y;
+        t[2] = p.x;
+        t[3] = p.y;
+        if constexpr (sizeof(T) == 8) {
+            abs_phi_theta(f.x, f.y, t[5], t[4]);
+        } else {
+            t[4] = abs_theta(f.x, f.y);
+            t[5] = sqrt(f.x * f.x + f.y * f.y);
+        }
     };
-    // the loads of two trips are in flight before either is summed (the same
-    // trips in the same order as one at a time: the same sums)
+    // the loads of two trips (two sites each) are in flight before either is summed
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (; i + stride < npair; i += 2 * stride) {
         C f0[2], p0[2], f1[2], p1[2];
@@ -2173,24 +2396,41 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_background(cons
         load_pair(pih, i, p0);
         load_pair(psi, i + stride, f1);
         load_pair(pih, i + stride, p1);
-        trip(f0, p0);
-        trip(f1, p1);
+        T t[4][6];
+        terms(f0[0], p0[0], t[0]);
+        terms(f0[1], p0[1], t[1]);
+        terms(f1[0], p1[0], t[2]);
+        terms(f1[1], p1[1], t[3]);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            if constexpr (sizeof(T) == 8) {   // four sites by one sum off the FP64 pipe
+                a[k].add(nsum5<T>(t[0][k], t[1][k], t[2][k], t[3][k]));
+            } else {
+                a[k].add(t[0][k] + t[1][k]);
+                a[k].add(t[2][k] + t[3][k]);
+            }
+        }
     }
     if (i < npair) {
         C f[2], p[2];
         load_pair(psi, i, f);
         load_pair(pih, i, p);
-        trip(f, p);
+        T t[2][6];
+        terms(f[0], p[0], t[0]);
+        terms(f[1], p[1], t[1]);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) a[k].add(t[0][k] + t[1][k]);
     }
     double v[6];
     for (int k = 0; k < 6; ++k) v[k] = a[k].value();
-    block_reduce_store<6>(v, partials);
+    grid_reduce<6>(v, partials, ticket, hout);
 }
 
 template <typename T, int ND>
 __global__ void __launch_bounds__(256) k_energies(const typename Cplx<T>::type *__restrict__ psi,
                                                   const typename Cplx<T>::type *__restrict__ pi, int N, int64_t len,
-                                                  double tau, double dx, double lam_eff, double *__restrict__ partials) {
+                                                  double tau, double dx, double lam_eff, double *__restrict__ partials,
+                                                  unsigned *ticket, double *__restrict__ hout) {
     Acc<T> a[3];
     const T it = (T)(1.0 / tau), idx = (T)(1.0 / dx), q = (T)(0.25 * lam_eff);
     const int64_t NN = (int64_t)N * N;
@@ -2227,93 +2467,113 @@ __global__ void __launch_bounds__(256) k_energies(const typename Cplx<T>::type *
     }
     double v[3];
     for (int k = 0; k < 3; ++k) v[k] = a[k].value();
-    block_reduce_store<3>(v, partials);
+    grid_reduce<3>(v, partials, ticket, hout);
 }
+
+// The energies' terms of one site, from its pi_n, psi and forward neighbours:
+// (pi - psi/tau)^2 and the squared differences of psi per component, and
+// (|psi|^2/tau^2 - 1)^2; the constant factors are applied to the sums.
+template <typename T>
+struct EnergyAcc {
+    typedef typename Cplx<T>::type C;
+    C kin, grad;   // the running pair of sites
+    T pot;
+    Acc<T> k[2], g[2], v;
+    __device__ __forceinline__ void clear() {
+        kin = grad = C{T(0), T(0)};
+        pot = T(0);
+    }
+    __device__ __forceinline__ void site(const C &c, const C &p, const C &xp, const C &yp, const C *zp, T it, T it2) {
+        const C e = vfma(-it, c, p);
+        kin = vfma(e, e, kin);
+        const C gx = vsub(xp, c), gy = vsub(yp, c);
+        grad = vfma(gx, gx, grad);
+        grad = vfma(gy, gy, grad);
+        if (zp) {
+            const C gz = vsub(*zp, c);
+            grad = vfma(gz, gz, grad);
+        }
+        const T r = fma(it2, fma(c.x, c.x, c.y * c.y), (T)-1);
+        pot = fma(r, r, pot);
+    }
+    __device__ __forceinline__ void add() {   // into the compensated sums
+        if constexpr (sizeof(T) == 8) {
+            k[0].add(kin.x + kin.y);
+            g[0].add(grad.x + grad.y);
+        } else {
+            k[0].add(kin.x);
+            k[1].add(kin.y);
+            g[0].add(grad.x);
+            g[1].add(grad.y);
+        }
+        v.add(pot);
+        clear();
+    }
+    __device__ __forceinline__ void sums(double (&out)[3], double tau, double dx, double lam_eff) const {
+        out[0] = (k[0].value() + k[1].value()) * (0.5 / (tau * tau));
+        out[1] = (g[0].value() + g[1].value()) * (0.5 / (tau * tau * dx * dx));
+        out[2] = v.value() * (0.25 * lam_eff);
+    }
+};
 
 // Energy densities of a 3D radius-1 lattice in one pass over psi and pih
 // (the kinetic term is quadratic in pi_n, so unlike the background means it
-// needs the full half kick per site). pi_n is formed per site with
-// sync_pi_site and never stored, and each thread marches one (x, y)
-// column through z: psi's z-neighbours stay in registers
+// needs the full half kick per site). pi_n is formed per site by
+// sync_pi_r1 and never stored, and each thread marches one (x, y)
+// column of a z-chunk: psi's z-neighbours stay in registers
 // and the in-plane neighbours (also the x+1, y+1 forward differences of the
 // gradient energy; z+1 is the next plane in registers) come from the
 // neighbouring threads' loads of the same plane. 16 B from DRAM per site
 // instead of 40 B through scratch. Blocks are 256 threads over 32 x 8 columns
-// (threads past the edge add nothing); each block writes its partial sums at
-// its index, so the totals are deterministic.
+// (threads past the edge add nothing).
 //
-// The kernel is issue-bound, so the march is arranged for few instructions per
-// site: three column pointers advance a plane per site (wrapping once, near the
-// end), two sites per trip (N is even) so the register rotation is renaming,
-// the two sites' terms are added in plain T before one compensated add, and
-// the constant factors (1/2 tau^-2, 1/2 (tau dx)^-2, lambda/4) are applied to
-// the column sums: the sums are of (pi - psi/tau)^2, of the squared
-// differences of psi and of (|psi|^2/tau^2 - 1)^2. Float fields fit 64
-// registers (4 CTAs per SM). N >= 4.
+// The march is arranged for few instructions per site: plane addresses are uniform and
+// each load adds a fixed 32-bit offset, both components go through packed
+// FP32 operations, two sites per trip (a chunk has whole pairs) so the register
+// rotation is renaming, and two sites' terms are added before one compensated
+// add. 512^3 FP32: 443 us (4.9 TB/s), 476 without the packed operations and the
+// uniform addresses.
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_energies_zcol(const typename Cplx<T>::type *__restrict__ psi,
                                                          const typename Cplx<T>::type *__restrict__ pih,
                                                          double *__restrict__ partials, const double *clock, int N,
                                                          double dt, double inv_dx2, double lambda, double T0sq3,
                                                          int prs, int form, int fresh, double tau, double dx,
-                                                         double lam_eff) {
+                                                         double lam_eff, unsigned *ticket, double *__restrict__ hout) {
     typedef typename Cplx<T>::type C;
-    constexpr int K = 3;
-    Acc<T> acc[K];
+    const StepCoefs<T> c = block_coefs<T>(clock, dt, 0.5 * dt, inv_dx2, lambda, T0sq3, prs, form);
+    EnergyAcc<T> acc;
+    acc.clear();
     const int bx = (N + 31) / 32;
     const int x = (int)(blockIdx.x % bx) * 32 + (threadIdx.x & 31), y = (int)(blockIdx.x / bx) * 8 + (threadIdx.x >> 5);
-    if (x < N && y < N) {
-        const StepCoefs<T> c = make_coefs<T>(*clock, dt, 0.5 * dt, inv_dx2, lambda, T0sq3, prs, form);
-        const T it = (T)(1.0 / tau), it2 = (T)(1.0 / (tau * tau));
-        const int64_t NN = (int64_t)N * N, len = NN * N;
-        const int col = y * N + x;
-        const int xm = y * N + (x == 0 ? N - 1 : x - 1) - col, xp = y * N + (x == N - 1 ? 0 : x + 1) - col;
-        const int ym = (y == 0 ? N - 1 : y - 1) * N + x - col, yp = (y == N - 1 ? 0 : y + 1) * N + x - col;
-        // column values: psi planes z-1, z, z+1 in use, z+2 and z+3 in flight;
-        // pih plane z in use, z+1 and z+2 in flight; neighbours of plane z in
-        // use (loaded a site earlier), those of z+1 in flight
-        C zm = psi[(N - 1) * NN + col], zc = psi[col];
-        C zp = psi[NN + col], zq = psi[2 * NN + col];
-        C pc = pih[col], pq = pih[NN + col];
-        C a, b, d, e;
-        { a = psi[col + xm]; b = psi[col + xp]; d = psi[col + ym]; e = psi[col + yp]; }
-        const C *s3 = psi + 3 * NN + col, *p2 = pih + 2 * NN + col, *s1 = psi + NN + col;   // planes z+3, z+2, z+1
-        for (int z = 0; z < N; z += 2) {
-            T t[K];
-#pragma unroll
-            for (int k = 0; k < K; ++k) t[k] = 0;
+    const int za = 2 * (int)((int64_t)blockIdx.y * (N / 2) / gridDim.y);
+    const int zb = 2 * (int)((int64_t)(blockIdx.y + 1) * (N / 2) / gridDim.y);
+    if (x < N && y < N && za < zb) {
+        const T it = (T)(1.0 / tau), it2 = (T)(1.0 / (tau * tau)), kctr = c.kdt_idx2 * (T)-6;
+        const size_t plane = (size_t)N * N * sizeof(C);
+        // byte offsets within a plane (below 2^32: N <= 4096)
+        auto off = [&](int xx, int yy) { return (unsigned)((unsigned)yy * (unsigned)N + (unsigned)xx) * (unsigned)sizeof(C); };
+        const unsigned oc = off(x, y), oxm = off(x == 0 ? N - 1 : x - 1, y), oxp = off(x == N - 1 ? 0 : x + 1, y),
+                       oym = off(x, y == 0 ? N - 1 : y - 1), oyp = off(x, y == N - 1 ? 0 : y + 1);
+        auto at = [](const char *b, unsigned o) { return *reinterpret_cast<const C *>(b + o); };
+        auto pl = [&](const C *b, int z) { return reinterpret_cast<const char *>(b) + (size_t)(z >= N ? z - N : (z < 0 ? z + N : z)) * plane; };
+        // planes z-1, z, z+1 in use, z+2 and z+3 in flight; pih plane z in use, z+1
+        // and z+2 in flight; the in-plane neighbours of z in use, those of z+1 in flight
+        C zm = at(pl(psi, za - 1), oc), zc = at(pl(psi, za), oc), zp = at(pl(psi, za + 1), oc), zq = at(pl(psi, za + 2), oc);
+        C pc = at(pl(pih, za), oc), pq = at(pl(pih, za + 1), oc);
+        const char *b0 = pl(psi, za);
+        C xm = at(b0, oxm), xp = at(b0, oxp), ym = at(b0, oym), yp = at(b0, oyp);
+        for (int z = za; z < zb; z += 2) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int zz = z + h;
-                const C zr = *(zz + 3 < N ? s3 : s3 - len);
-                const C pr = *(zz + 2 < N ? p2 : p2 - len);
-                const C *q1 = zz + 1 < N ? s1 : s1 - len;
-                s3 += NN;
-                p2 += NN;
-                s1 += NN;
-                C na, nb, nd, ne;
-                { na = q1[xm]; nb = q1[xp]; nd = q1[ym]; ne = q1[yp]; }
+                const C zr = at(pl(psi, zz + 3), oc), pr = at(pl(pih, zz + 2), oc);
+                const char *b1 = pl(psi, zz + 1);
+                const C nxm = at(b1, oxm), nxp = at(b1, oxp), nym = at(b1, oym), nyp = at(b1, oyp);
                 C p = pc;
-                if (!fresh) {   // a fresh state holds pi_0 itself (the reference's ker is zero)
-                    const T L1 = lap7<T>(zc.x, a.x, b.x, d.x, e.x, zm.x, zp.x);
-                    const T L2 = lap7<T>(zc.y, a.y, b.y, d.y, e.y, zm.y, zp.y);
-                    sync_pi_site<T>(zc.x, zc.y, L1, L2, p.x, p.y, c);
-                }
-                {   // differences in the order x, y, z
-                    const T e1 = fma(-zc.x, it, p.x), e2 = fma(-zc.y, it, p.y);
-                    t[0] += fma(e1, e1, e2 * e2);
-                    T g1 = b.x - zc.x, g2 = b.y - zc.y;
-                    T g = fma(g1, g1, g2 * g2);
-                    g1 = e.x - zc.x;
-                    g2 = e.y - zc.y;
-                    g = fma(g1, g1, fma(g2, g2, g));
-                    g1 = zp.x - zc.x;
-                    g2 = zp.y - zc.y;
-                    t[1] += fma(g1, g1, fma(g2, g2, g));
-                    const T r = fma(it2, fma(zc.x, zc.x, zc.y * zc.y), (T)-1);
-                    t[2] += r * r;
-                }
-                a = na; b = nb; d = nd; e = ne;
+                if (!fresh) sync_pi_r1<T, 3>(zc, vnsum(xm, xp, ym, yp, zm, zp), p, c, kctr);
+                acc.site(zc, p, xp, yp, &zp, it, it2);
+                xm = nxm; xp = nxp; ym = nym; yp = nyp;
                 zm = zc;
                 zc = zp;
                 zp = zq;
@@ -2321,16 +2581,41 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_energies_zcol(c
                 pc = pq;
                 pq = pr;
             }
-#pragma unroll
-            for (int k = 0; k < K; ++k) acc[k].add(t[k]);
+            acc.add();
         }
     }
-    double v[K];
-    for (int k = 0; k < K; ++k) v[k] = acc[k].value();
-    v[0] *= 0.5 / (tau * tau);
-    v[1] *= 0.5 / (tau * tau * dx * dx);
-    v[2] *= 0.25 * lam_eff;
-    block_reduce_store<K>(v, partials);
+    double v[3];
+    acc.sums(v, tau, dx, lam_eff);
+    grid_reduce<3>(v, partials, ticket, hout);
+}
+
+// The same for 2D and every radius: one thread per site of 32 x 8 tiles, the
+// neighbours from L1/L2.
+template <typename T, int R>
+__global__ void __launch_bounds__(256) k_energies_2d(const typename Cplx<T>::type *__restrict__ psi,
+                                                     const typename Cplx<T>::type *__restrict__ pih,
+                                                     double *__restrict__ partials, const double *clock, int N, double dt,
+                                                     double inv_dx2, double lambda, double T0sq3, int prs, int form,
+                                                     int fresh, double tau, double dx, double lam_eff, unsigned *ticket,
+                                                     double *__restrict__ hout) {
+    typedef typename Cplx<T>::type C;
+    const StepCoefs<T> c = block_coefs<T>(clock, dt, 0.5 * dt, inv_dx2, lambda, T0sq3, prs, form);
+    const T it = (T)(1.0 / tau), it2 = (T)(1.0 / (tau * tau));
+    EnergyAcc<T> acc;
+    acc.clear();
+    const int nbx = (N + 31) / 32, nt = nbx * ((N + 7) / 8);
+    for (int t = blockIdx.x; t < nt; t += gridDim.x) {
+        const int ty = t / nbx, x = (t - ty * nbx) * 32 + (threadIdx.x & 31), y = ty * 8 + (threadIdx.x >> 5);
+        if (x >= N || y >= N) continue;
+        const C f = psi[y * N + x];
+        C xp, yp;
+        const C p = sync_site_2d<T, R>(psi, pih, N, x, y, f, fresh, c, xp, yp);
+        acc.site(f, p, xp, yp, nullptr, it, it2);
+        acc.add();
+    }
+    double v[3];
+    acc.sums(v, tau, dx, lam_eff);
+    grid_reduce<3>(v, partials, ticket, hout);
 }
 
 // k_energies_zcol for the radius-R stencils (R = 2..4), on k_axion_zcol_r's
@@ -2343,49 +2628,35 @@ __global__ void __launch_bounds__(256, (ZMarch<T, R>::MINB)) k_energies_zcol_r(c
                                                                     double *__restrict__ partials, const double *clock,
                                                                     int N, double dt, double inv_dx2, double lambda,
                                                                     double T0sq3, int prs, int form, int fresh,
-                                                                    double tau, double dx, double lam_eff) {
+                                                                    double tau, double dx, double lam_eff,
+                                                                    unsigned *ticket, double *__restrict__ hout) {
     typedef typename Cplx<T>::type C;
-    constexpr int K = 3, TW = ZMarch<T, R>::TW;
-    Acc<T> acc[K];
-    T t[K] = {0, 0, 0};
-    const StepCoefs<T> c = make_coefs<T>(*clock, dt, 0.5 * dt, inv_dx2, lambda, T0sq3, prs, form);
+    constexpr int TW = ZMarch<T, R>::TW;
+    EnergyAcc<T> acc;
+    acc.clear();
+    const StepCoefs<T> c = block_coefs<T>(clock, dt, 0.5 * dt, inv_dx2, lambda, T0sq3, prs, form);
     const T it = (T)(1.0 / tau), it2 = (T)(1.0 / (tau * tau));
     zcol_march<T, R>(psi, pih, N, fresh, c, [&](int h, int, const C &zc, const C &zp, const C &p, const C *ts) {
-        const C b = ts[1], e = ts[TW];   // differences in the order x, y, z
-        const T e1 = fma(-zc.x, it, p.x), e2 = fma(-zc.y, it, p.y);
-        t[0] += fma(e1, e1, e2 * e2);
-        T g1 = b.x - zc.x, g2 = b.y - zc.y;
-        T g = fma(g1, g1, g2 * g2);
-        g1 = e.x - zc.x;
-        g2 = e.y - zc.y;
-        g = fma(g1, g1, fma(g2, g2, g));
-        g1 = zp.x - zc.x;
-        g2 = zp.y - zc.y;
-        t[1] += fma(g1, g1, fma(g2, g2, g));
-        const T r = fma(it2, fma(zc.x, zc.x, zc.y * zc.y), (T)-1);
-        t[2] += r * r;
-        if (h & 1) {   // W is even, so sites pair up within a trip
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                acc[k].add(t[k]);
-                t[k] = 0;
-            }
-        }
+        acc.site(zc, p, ts[1], ts[TW], &zp, it, it2);
+        if (h & 1) acc.add();   // W is even and chunks are whole pairs
     });
-    double v[K];
-    for (int k = 0; k < K; ++k) v[k] = acc[k].value();
-    v[0] *= 0.5 / (tau * tau);
-    v[1] *= 0.5 / (tau * tau * dx * dx);
-    v[2] *= 0.25 * lam_eff;
-    block_reduce_store<K>(v, partials);
+    double v[3];
+    acc.sums(v, tau, dx, lam_eff);
+    grid_reduce<3>(v, partials, ticket, hout);
 }
 
 template <typename T>
-__global__ void k_finite(const T *__restrict__ a, int64_t n, int *flag) {
+__global__ void __launch_bounds__(256) k_finite(const T *__restrict__ a, const T *__restrict__ b, int64_t n,
+                                                unsigned long long *bad_blocks, unsigned *ticket, int64_t *hout) {
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
     int bad = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) bad |= !isfinite(a[i]);
-    if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(flag, 1);
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
+        bad |= !isfinite(a[i]) | !isfinite(b[i]);
+    if (__syncthreads_or(bad) && threadIdx.x == 0) atomicAdd(bad_blocks, 1ull);
+    if (last_block(ticket) && threadIdx.x == 0) {
+        *hout = (int64_t)__ldcg(bad_blocks);
+        *bad_blocks = 0;
+    }
 }
 
 static double *ensure_partials(Lattice *L, int nblocks, int K) {
@@ -2399,30 +2670,37 @@ static double *ensure_partials(Lattice *L, int nblocks, int K) {
     return L->dpartials;
 }
 
-// The z-column energies serve 3D lattices with a finite-difference Laplacian
-// (any radius); 2D and the spectral Laplacian form pi_n in scratch first.
-static bool energies_zcol(const Lattice *L) { return L->p.NDIMS == 3 && L->p.laplacian == 0; }
-
 template <typename T>
-static void energies_zcol_t(Lattice *L, double *part, int g, double lam) {
+static void energies_fd(Lattice *L, double lam, double *hout) {
     typedef typename Cplx<T>::type C;
     const axs_params &p = L->p;
     const double dx = p.space_step, T0 = p.T_initial;
     const C *f = (const C *)L->psi[L->cur], *q = (const C *)L->pih;
     const double *clk = L->dclock + L->cur;
     const double dt = p.time_step, idx2 = 1.0 / (dx * dx), la = p.lambda, t3 = (T0 * T0) / 3.0;
-    auto radius = [&](auto kern, size_t smem) {
-        AXS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<g, 256, smem, L->stream>>>(f, q, part, clk, p.N, dt, idx2, la, t3, p.prs, p.form, L->fresh, L->tau, dx, lam);
+    auto go = [&](auto kern, dim3 g, size_t smem) {
+        if (smem) AXS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        double *part = ensure_partials(L, (int)(g.x * g.y), 3);
+        kern<<<g, 256, smem, L->stream>>>(f, q, part, clk, p.N, dt, idx2, la, t3, p.prs, p.form, L->fresh, L->tau, dx, lam,
+                                          L->dticket, hout);
     };
+    if (p.NDIMS == 2) {
+        const dim3 g(std::min(((p.N + 31) / 32) * ((p.N + 7) / 8), num_sms() * 8));
+        switch (p.stencil_setting) {
+        case 0: go(k_energies_2d<T, 1>, g, 0); break;
+        case 1: go(k_energies_2d<T, 2>, g, 0); break;
+        case 2: go(k_energies_2d<T, 3>, g, 0); break;
+        default: go(k_energies_2d<T, 4>, g, 0); break;
+        }
+        return;
+    }
     switch (p.stencil_setting) {
-    case 0: k_energies_zcol<T><<<g, 256, 0, L->stream>>>(f, q, part, clk, p.N, dt, idx2, la, t3, p.prs, p.form, L->fresh, L->tau, dx, lam); break;
-    case 1: radius(k_energies_zcol_r<T, 2>, ZMarch<T, 2>::SMEM); break;
-    case 2: radius(k_energies_zcol_r<T, 3>, ZMarch<T, 3>::SMEM); break;
-    default: radius(k_energies_zcol_r<T, 4>, ZMarch<T, 4>::SMEM); break;
+    case 0: go(k_energies_zcol<T>, zcol_grid<T, 1>(p.N), 0); break;
+    case 1: go(k_energies_zcol_r<T, 2>, zcol_grid<T, 2>(p.N), ZMarch<T, 2>::SMEM); break;
+    case 2: go(k_energies_zcol_r<T, 3>, zcol_grid<T, 3>(p.N), ZMarch<T, 3>::SMEM); break;
+    default: go(k_energies_zcol_r<T, 4>, zcol_grid<T, 4>(p.N), ZMarch<T, 4>::SMEM); break;
     }
 }
-static int zcol_blocks(int N) { return ((N + 31) / 32) * ((N + 7) / 8); }
 
 void background(Lattice *L, double out[6]) {
     const axs_params &p = L->p;
@@ -2431,18 +2709,20 @@ void background(Lattice *L, double out[6]) {
     const int resident = L->esz == 4 ? 4 : 2;   // k_background's blocks per SM
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>((L->length / 2 + 255) / 256, (int64_t)num_sms() * resident));
     double *part = ensure_partials(L, g, 6);
+    double *s = host_slot(L);
     if (L->esz == 4)
         k_background<float><<<g, 256, 0, L->stream>>>((const float2 *)L->psi[L->cur], (const float2 *)L->pih,
                                                        L->dclock + L->cur, L->length, (double)p.time_step,
-                                                       (double)p.lambda, (T0 * T0) / 3.0, p.prs, p.form, L->fresh, part);
+                                                       (double)p.lambda, (T0 * T0) / 3.0, p.prs, p.form, L->fresh, part,
+                                                       L->dticket, s);
     else
         k_background<double><<<g, 256, 0, L->stream>>>((const double2 *)L->psi[L->cur], (const double2 *)L->pih,
                                                         L->dclock + L->cur, L->length, (double)p.time_step,
-                                                        (double)p.lambda, (T0 * T0) / 3.0, p.prs, p.form, L->fresh, part);
+                                                        (double)p.lambda, (T0 * T0) / 3.0, p.prs, p.form, L->fresh, part,
+                                                        L->dticket, s);
     AXS_CUDA(cudaGetLastError());
     count_launches(1);
-    double s[6];
-    sum_partials(part, g, 6, s, L->stream);
+    AXS_CUDA(cudaStreamSynchronize(L->stream));
     for (int k = 0; k < 6; ++k) out[k] = s[k] / (double)L->length;   // s_run.cpp:149
     if (!L->fresh && p.laplacian == 0) {   // the stencil's share of the half kick: W mean(psi)
         double W = (double)stencil_coef(p.stencil_setting, p.NDIMS, 0);
@@ -2459,59 +2739,55 @@ void energies(Lattice *L, double out[3]) {
     if (L->p.form != 0) fail(AXS_ERR_STATE, "the energies are defined on the field-rescaled variables (form 0)");
     double lam = (double)L->p.lambda * (L->p.prs ? 1.0 : L->tau * L->tau);
     double dx = L->p.space_step;
-    int g;
-    double *part;
-    if (energies_zcol(L)) {
-        g = zcol_blocks(L->p.N);
-        part = ensure_partials(L, g, 3);
-        if (L->esz == 4) energies_zcol_t<float>(L, part, g, lam);
-        else energies_zcol_t<double>(L, part, g, lam);
-    } else {
+    double *s = host_slot(L);
+    if (L->p.laplacian == 0) {
+        if (L->esz == 4) energies_fd<float>(L, lam, s);
+        else energies_fd<double>(L, lam, s);
+    } else {   // the spectral Laplacian: pi_n through scratch
         launch_sync_pi(L);
-        g = reduce_grid(L->length);
-        part = ensure_partials(L, g, 3);
-        const int N = L->p.N;
+        const int g = reduce_grid(L->length), N = L->p.N;
+        double *part = ensure_partials(L, g, 3);
         const int64_t n = L->length;
+        auto go = [&](auto kern, auto f, auto q) {
+            kern<<<g, 256, 0, L->stream>>>(f, q, N, n, L->tau, dx, lam, part, L->dticket, s);
+        };
         if (L->esz == 4) {
             const float2 *f = (const float2 *)L->psi[L->cur], *q = (const float2 *)L->scratch;
-            if (L->p.NDIMS == 2) k_energies<float, 2><<<g, 256, 0, L->stream>>>(f, q, N, n, L->tau, dx, lam, part);
-            else k_energies<float, 3><<<g, 256, 0, L->stream>>>(f, q, N, n, L->tau, dx, lam, part);
+            if (L->p.NDIMS == 2) go(k_energies<float, 2>, f, q);
+            else go(k_energies<float, 3>, f, q);
         } else {
             const double2 *f = (const double2 *)L->psi[L->cur], *q = (const double2 *)L->scratch;
-            if (L->p.NDIMS == 2) k_energies<double, 2><<<g, 256, 0, L->stream>>>(f, q, N, n, L->tau, dx, lam, part);
-            else k_energies<double, 3><<<g, 256, 0, L->stream>>>(f, q, N, n, L->tau, dx, lam, part);
+            if (L->p.NDIMS == 2) go(k_energies<double, 2>, f, q);
+            else go(k_energies<double, 3>, f, q);
         }
     }
     AXS_CUDA(cudaGetLastError());
     count_launches(1);
-    double s[3];
-    sum_partials(part, g, 3, s, L->stream);
+    AXS_CUDA(cudaStreamSynchronize(L->stream));
     for (int k = 0; k < 3; ++k) out[k] = s[k] / (double)L->length;
 }
 
 int check_finite(Lattice *L) {
-    int *flag = (int *)(L->dcount ? L->dcount : (L->dcount = (int64_t *)dalloc(4 * sizeof(int64_t)))) + 6;
-    AXS_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), L->stream));
-    int64_t n = L->length * 2;
-    int g = grid_cap(n, 256, 8);
-    if (L->esz == 4) {
-        k_finite<float><<<g, 256, 0, L->stream>>>((const float *)L->psi[L->cur], n, flag);
-        k_finite<float><<<g, 256, 0, L->stream>>>((const float *)L->pih, n, flag);
-    } else {
-        k_finite<double><<<g, 256, 0, L->stream>>>((const double *)L->psi[L->cur], n, flag);
-        k_finite<double><<<g, 256, 0, L->stream>>>((const double *)L->pih, n, flag);
-    }
+    int64_t *h = (int64_t *)host_slot(L);
+    const int64_t n = L->length * 2;
+    const int g = grid_cap(n, 256, 8);
+    if (L->esz == 4)
+        k_finite<float><<<g, 256, 0, L->stream>>>((const float *)L->psi[L->cur], (const float *)L->pih, n, L->dtally,
+                                                  L->dticket, h);
+    else
+        k_finite<double><<<g, 256, 0, L->stream>>>((const double *)L->psi[L->cur], (const double *)L->pih, n, L->dtally,
+                                                   L->dticket, h);
     AXS_CUDA(cudaGetLastError());
-    count_launches(2);
-    int h = 0;
-    AXS_CUDA(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, L->stream));
+    count_launches(1);
     AXS_CUDA(cudaStreamSynchronize(L->stream));
-    return h == 0;
+    return h[0] == 0;
 }
 
 void analysis_release(Lattice *L) {
     dfree(L->dmask); L->dmask = nullptr;
-    dfree(L->dcount); L->dcount = nullptr;
+    dfree(L->dchunk); L->dchunk = nullptr;
+    if (L->hslot) cudaFreeHost(L->hslot);
+    L->hslot = nullptr;
     dfree(L->dlist); L->dlist = nullptr;
     dfree(L->dtheta); L->dtheta = nullptr;
     dfree(L->fft_in); L->fft_in = nullptr;
@@ -2519,7 +2795,7 @@ void analysis_release(Lattice *L) {
     if (L->have_plan) cufftDestroy(L->plan_r2c);
     L->have_plan = false;
     dfree(L->dpartials); L->dpartials = nullptr;
-    for (int i = 0; i < 3; ++i) {
+    for (int i = 0; i < 2; ++i) {
         dfree(L->tmp[i]);
         L->tmp[i] = nullptr;
         L->tmp_cap[i] = 0;

@@ -119,9 +119,12 @@ static void lattice_init(Lattice *L, const axs_params &p, cudaStream_t shared) {
     L->psi[1] = dalloc(cbytes);
     L->pih = dalloc(cbytes);
     L->scratch = dalloc(cbytes);
-    // one small allocation: the clock's two slots, the error flag, 2D: the coefficient tables
+    // one small allocation: the clock's two slots, the error flag, the analysis' ticket and
+    // counters, 2D: the coefficient tables
     L->dclock = (double *)dalloc(256 + (p.NDIMS == 2 ? 2 * kStep2dSlot : 0));
     L->derr = (int *)(L->dclock + 2);
+    L->dticket = (unsigned *)(L->dclock + 4);
+    L->dtally = (unsigned long long *)(L->dclock + 8);
     if (p.NDIMS == 2) {
         L->dstep2d = (char *)L->dclock + 256;
         AXS_CUDA(cudaMemsetAsync(L->dstep2d, 0xff, 2 * kStep2dSlot, L->stream));   // NaN tags: no table yet
@@ -129,7 +132,7 @@ static void lattice_init(Lattice *L, const axs_params &p, cudaStream_t shared) {
     AXS_CUDA(cudaMemsetAsync(L->psi[0], 0, cbytes, L->stream));
     AXS_CUDA(cudaMemsetAsync(L->psi[1], 0, cbytes, L->stream));
     AXS_CUDA(cudaMemsetAsync(L->pih, 0, cbytes, L->stream));
-    AXS_CUDA(cudaMemsetAsync(L->derr, 0, sizeof(int), L->stream));
+    AXS_CUDA(cudaMemsetAsync(L->dclock, 0, 256, L->stream));
     L->cur = 0;
     L->fresh = 1;
     L->tau = p.tau_initial;
@@ -371,8 +374,7 @@ static void download_fields(Lattice *L, S *f0, S *f1, S *f2, S *f3) {
     for (int f = 0; f < 4 && direct; ++f) direct = (dev[f] = device_alias(dst[f])) != nullptr;
     if (direct) {
         snapshot_fd(L, dev);
-        AXS_CUDA(cudaStreamSynchronize(L->stream));
-        check_device_errors(L);
+        check_device_errors(L);   // after the one synchronisation
         return;
     }
     if (f2 || f3) launch_sync_pi(L);
@@ -392,8 +394,7 @@ static void download_fields(Lattice *L, S *f0, S *f1, S *f2, S *f3) {
             AXS_CUDA(cudaStreamSynchronize(L->stream));
         }
     }
-    AXS_CUDA(cudaStreamSynchronize(L->stream));
-    check_device_errors(L);
+    check_device_errors(L);   // after the stream's synchronisation
 }
 
 struct CkptHeader {

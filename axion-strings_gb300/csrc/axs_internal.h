@@ -157,11 +157,17 @@ struct Lattice {
     int64_t zitems = 0;
     // analysis buffers (lazily allocated)
     uint8_t *dmask = nullptr;
-    int64_t *dcount = nullptr;       // [4] scratch counters
-    int32_t *dlist = nullptr;        // ascending flagged offsets (compacted)
-    int64_t list_cap = 0;
+    int32_t *dchunk = nullptr;       // flagged cells per chunk of the mask, then their scan
+    bool chunks_valid = false;       // dchunk holds the counts of the last search
+    int32_t *dlist = nullptr;        // positions of the flagged cells, in ascending offset order
+    int64_t list_cap = 0;            // int32 values
     int64_t last_nplaq = -1;
     bool list_valid = false;
+    // page-locked results of the analysis calls, written by the kernels' last
+    // blocks (host_slot): a call is its launches and one synchronisation
+    double *hslot = nullptr;
+    unsigned *dticket = nullptr;     // device: blocks done of the running reduction (0 between launches), then
+    unsigned long long *dtally = nullptr;   // [2] counters, 0 between searches (both beside the clock)
     double *dtheta = nullptr;        // caller theta upload
     void *fft_in = nullptr;          // real, length
     void *fft_out = nullptr;         // complex, R2C half spectrum
@@ -171,9 +177,10 @@ struct Lattice {
     size_t partials_cap = 0;
     void *dstage = nullptr;          // transfer staging (length reals)
     // small per-call work buffers of the analysis, kept between calls (grow only):
-    // 0 = string-finder chunk counts, 1 = spectrum block partials, 2 = bin thresholds
-    void *tmp[3] = {nullptr, nullptr, nullptr};
-    size_t tmp_cap[3] = {0, 0, 0};
+    // 0 = spectrum block partials, 1 = bin thresholds (and their host copy)
+    void *tmp[2] = {nullptr, nullptr};
+    size_t tmp_cap[2] = {0, 0};
+    std::vector<int> thr_on_device;
     // per-bin |n| sums and mode counts of the spectrum binnings used so far:
     // they depend on N and the bin edges alone, so later spectra with the same
     // edges bin the power only (kind 0 = linear bins of output_powerspec,
@@ -257,7 +264,7 @@ void launch_pack2_drift(Lattice *L, const void *a, const void *b, int src_is_dou
                         cudaStream_t st);
 void launch_unpack2(Lattice *L, const void *src_cplx, void *a, void *b, int dst_is_double, int64_t n, cudaStream_t st);
 void check_device_errors(Lattice *L);
-void check_device_error_flag(int *derr, cudaStream_t s);
+void check_device_error_flag(int *derr, cudaStream_t s, int *pinned = nullptr);
 
 // ---- init module (axs_init.cu)
 void init_gaussian(Lattice *L, uint64_t seed, int thermal, double kcut);
@@ -272,6 +279,9 @@ void energies(Lattice *L, double out[3]);
 int check_finite(Lattice *L);
 void field_distance(Lattice *A, Lattice *B, double out[8]);
 void analysis_release(Lattice *L);
+// page-locked results of the lattice's calls, kHostSlot doubles (allocated on first use)
+constexpr int kHostSlot = 2048;
+double *host_slot(Lattice *L);
 // finite-difference lattices: pi_n into scratch; psi and pi_n into four arrays
 // of the lattice's precision that the device reaches
 void sync_pi_fd(Lattice *L);
@@ -492,6 +502,58 @@ __device__ __forceinline__ void sync_pi_site(T a, T b, T L1, T L2, T &p1, T &p2,
     p2 = fma(c.kdt_idx2, L2, fma(g, b, p2));
 }
 
+// Two floats in one 64-bit register pair: sm_100's packed FP32 operations
+// round each half as the scalar ones do.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 r;
+    asm("{.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 z, x, y;\n\t"
+        "mov.b64 {%0, %1}, z;}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 r;
+    asm("{.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+        "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
+
+// Both components of a complex value at once: packed for float, each half
+// rounded as the scalar operation.
+__device__ __forceinline__ float2 vfma(float a, float2 b, float2 c) { return fma2(make_float2(a, a), b, c); }
+__device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return fma2(a, b, c); }
+__device__ __forceinline__ float2 vsub(float2 a, float2 b) { return fma2(make_float2(-1.f, -1.f), b, a); }
+__device__ __forceinline__ double2 vfma(double a, double2 b, double2 c) { return make_double2(fma(a, b.x, c.x), fma(a, b.y, c.y)); }
+__device__ __forceinline__ double2 vfma(double2 a, double2 b, double2 c) { return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y)); }
+__device__ __forceinline__ double2 vsub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+// nsum5 / nsum7 of both components
+__device__ __forceinline__ float2 vnsum(float2 xm, float2 xp, float2 ym, float2 yp) { return add2(add2(xm, xp), add2(ym, yp)); }
+__device__ __forceinline__ float2 vnsum(float2 xm, float2 xp, float2 ym, float2 yp, float2 zm, float2 zp) {
+    return add2(add2(add2(xm, xp), add2(ym, yp)), add2(zm, zp));
+}
+__device__ __forceinline__ double2 vnsum(double2 xm, double2 xp, double2 ym, double2 yp) {
+    return make_double2(nsum5<double>(xm.x, xp.x, ym.x, yp.x), nsum5<double>(xm.y, xp.y, ym.y, yp.y));
+}
+__device__ __forceinline__ double2 vnsum(double2 xm, double2 xp, double2 ym, double2 yp, double2 zm, double2 zp) {
+    return make_double2(nsum7<double>(xm.x, xp.x, ym.x, yp.x, zm.x, zp.x), nsum7<double>(xm.y, xp.y, ym.y, yp.y, zm.y, zp.y));
+}
+// Synchronised momentum of a radius-1 site from its neighbours' sum S:
+// sync_pi_site on the Laplacian in float; in double the centre weight goes into
+// the local coefficient (kctr = kdt_idx2 * -2 ND), as in site_update_fold.
+template <typename T, int ND>
+__device__ __forceinline__ void sync_pi_r1(const typename Cplx<T>::type &f, const typename Cplx<T>::type &S,
+                                           typename Cplx<T>::type &p, const StepCoefs<T> &c, T kctr) {
+    const T r = fma(f.x, f.x, fma(f.y, f.y, c.c0));
+    if constexpr (sizeof(T) == 8) {
+        p = vfma(c.kdt_idx2, S, vfma(fma(c.kdt_coef, r, kctr), f, p));
+    } else {
+        p = vfma(c.kdt_idx2, vfma((T)(-2 * ND), f, S), vfma(c.kdt_coef * r, f, p));
+    }
+}
+
 // The axion field of the kinetic spectrum, f = |phi| dtheta/dtau =
 // (psi2 pi1 - psi1 pi2) / (tau |psi|), with itau = 1/tau.
 template <typename T>
@@ -507,16 +569,32 @@ __device__ __forceinline__ float axion_f<float>(float a, float b, float p1, floa
     const float r2 = a * a + b * b;
     return r2 > 0.f ? (b * p1 - a * p2) * itau * rsqrtf(r2) : 0.f;
 }
+// Whether a positive double lies in [2^(lo-1023), 2^(hi-1023)), by its high word:
+// comparisons and conversions of doubles run on the FP64 pipe (16 cycles per
+// warp and SM, 32 integer instructions' worth).
+__device__ __forceinline__ bool exponent_in(double x, unsigned lo, unsigned hi) {
+    return ((unsigned)__double2hiint(x) >> 20) - lo < hi - lo;   // a negative x has 2048 more
+}
+// A double of magnitude in float's normal range as a float, truncated, and a
+// normal float as a double (exact), by their bits.
+__device__ __forceinline__ float float_bits(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    return __uint_as_float((hi & 0x80000000u) | (((hi & 0x7fffffffu) - (896u << 20)) << 3) | (lo >> 29));
+}
+__device__ __forceinline__ double double_bits(float x) {
+    const unsigned u = __float_as_uint(x);
+    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))), (int)(u << 29));
+}
 // FP64 fields: 1/|psi| by two Newton-Raphson steps for the reciprocal square
 // root, y <- y (3/2 - s y^2 / 2), from the float rsqrtf (within 1-2 ulp of the
 // correctly rounded square root and division, at a third of their cost on
-// GB300's FP64 pipe); |psi|^2 outside float range takes those.
+// GB300's FP64 pipe); |psi|^2 outside [2^-120, 2^120) takes those.
 template <>
 __device__ __forceinline__ double axion_f<double>(double a, double b, double p1, double p2, double itau) {
     const double s = a * a + b * b;
-    if (s > 1e-36 && s < 1e36) {
+    if (exponent_in(s, 1023 - 120, 1023 + 120)) {
         const double hs = 0.5 * s;
-        double y = (double)rsqrtf((float)s);
+        double y = double_bits(rsqrtf(float_bits(s)));
         y = y * fma(-hs * y, y, 1.5);
         y = y * fma(-hs * y, y, 1.5);
         return (b * p1 - a * p2) * itau * y;
@@ -576,33 +654,63 @@ __device__ __forceinline__ double normal_draw(uint64_t seed, int a, int64_t m) {
 
 __device__ __forceinline__ int64_t wrapi(int64_t i, int64_t N) { return i < 0 ? i + N : (i >= N ? i - N : i); }
 
-// Deterministic block reduction of K doubles (fixed shuffle tree, warps summed
-// in order); thread 0 writes the block's K partial sums to out[blockIdx.x*K+k].
-// blockDim.x must be 256.
-template <int K>
-__device__ __forceinline__ void block_reduce_store(double (&v)[K], double *out) {
-    __shared__ double red[8][K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        double x = v[k];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        v[k] = x;
-    }
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < K; ++k) red[w][k] = v[k];
+// The block's ticket: true in every thread of the launch's last block to get
+// here, with all earlier blocks' global writes visible; the ticket is then 0
+// again for the next launch.
+__device__ __forceinline__ bool last_block(unsigned *ticket) {
+    __shared__ bool last;
+    __threadfence();   // this thread's writes, before the barrier and the ticket
     __syncthreads();
     if (threadIdx.x == 0) {
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            double s = 0.0;
-            for (int i = 0; i < 8; ++i) s += red[i][k];
-            out[(int64_t)blockIdx.x * K + k] = s;
-        }
+        last = atomicAdd(ticket, 1u) == gridDim.x * gridDim.y * gridDim.z - 1;
+        if (last) *ticket = 0;
     }
     __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+// Deterministic block reduction of K doubles; writes the block's K sums to
+// out[row * K + k]. Warp w sums quantities w, w + 8, ... of all 256 threads: eight
+// values per lane, then a fixed shuffle tree, 13 FP64 instructions per quantity
+// (summing each quantity in each warp first takes 40 of the FP64 pipe's 16-cycle
+// slots). blockDim.x must be 256.
+template <int K>
+__device__ __forceinline__ void block_reduce_store(double (&v)[K], double *out, int64_t row) {
+    __shared__ double red[K][256];
+    __syncthreads();   // a previous reduction's readers are done
+#pragma unroll
+    for (int k = 0; k < K; ++k) red[k][threadIdx.x] = v[k];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int k = threadIdx.x >> 5; k < K; k += 8) {
+        double x = red[k][lane];
+#pragma unroll
+        for (int i = 1; i < 8; ++i) x += red[k][lane + 32 * i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if (lane == 0) out[row * K + k] = x;
+    }
+}
+template <int K>
+__device__ __forceinline__ void block_reduce_store(double (&v)[K], double *out) {
+    block_reduce_store<K>(v, out, blockIdx.x);
+}
+// The grid's sum of v: block partials, which the last block adds (thread t
+// those of blocks t, t + 256, ..., then the fixed tree) into hout, page-locked
+// host memory. The order is fixed, so the sums are deterministic.
+template <int K>
+__device__ __forceinline__ void grid_reduce(double (&v)[K], double *partials, unsigned *ticket, double *hout) {
+    block_reduce_store<K>(v, partials, blockIdx.y * gridDim.x + blockIdx.x);
+    if (!last_block(ticket)) return;
+    const int n = gridDim.x * gridDim.y;
+    double s[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) s[k] = 0.0;
+    for (int b = threadIdx.x; b < n; b += 256)
+#pragma unroll
+        for (int k = 0; k < K; ++k) s[k] += __ldcg(partials + (int64_t)b * K + k);
+    block_reduce_store<K>(s, hout, 0);
 }
 
 }  // namespace axs

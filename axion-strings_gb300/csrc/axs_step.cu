@@ -3425,15 +3425,16 @@ void launch_unpack2(Lattice *L, const void *src_cplx, void *a, void *b, int dst_
     count_launches(1);
 }
 
-void check_device_error_flag(int *derr, cudaStream_t s) {
-    int h = 0;
-    AXS_CUDA(cudaMemcpyAsync(&h, derr, sizeof(int), cudaMemcpyDeviceToHost, s));
+void check_device_error_flag(int *derr, cudaStream_t s, int *pinned) {
+    int own = 0, *dst = pinned ? pinned : &own;
+    AXS_CUDA(cudaMemcpyAsync(dst, derr, sizeof(int), cudaMemcpyDeviceToHost, s));
     AXS_CUDA(cudaStreamSynchronize(s));
+    const int h = *dst;
     if (h & DEVERR_TIMEOUT) {
         AXS_CUDA(cudaMemsetAsync(derr, 0, sizeof(int), s));
         fail(AXS_ERR_TIMEOUT, "a step kernel gave up waiting for a TMA load; the step was not completed");
     }
 }
-void check_device_errors(Lattice *L) { check_device_error_flag(L->derr, L->stream); }
+void check_device_errors(Lattice *L) { check_device_error_flag(L->derr, L->stream, (int *)host_slot(L)); }
 
 }  // namespace axs

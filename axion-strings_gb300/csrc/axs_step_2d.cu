@@ -38,25 +38,6 @@
 
 namespace axs {
 
-// Two floats in one 64-bit register pair: sm_100's packed FP32 operations
-// round each half as the scalar ones do.
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    float2 r;
-    asm("{.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 z, x, y;\n\t"
-        "mov.b64 {%0, %1}, z;}"
-        : "=f"(r.x), "=f"(r.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 r;
-    asm("{.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
-        "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;}"
-        : "=f"(r.x), "=f"(r.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return r;
-}
-
 struct Step2dArgs {
     const void *psi;
     void *psi_out;
