@@ -17,7 +17,7 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libaxs.so")
 DRIVER = os.path.join(HERE, "host", "axs_run")
 
-CUDA_SOURCES = ["axs_step.cu", "axs_step_r.cu", "axs_step_2d.cu", "axs_init.cu", "axs_analysis.cu", "axs_api.cu"]
+CUDA_SOURCES = ["axs_step.cu", "axs_step_r.cu", "axs_step_2d.cu", "axs_step_k.cu", "axs_init.cu", "axs_analysis.cu", "axs_api.cu"]
 HOST_SOURCES = ["axs_params.cpp", "axs_fileio.cpp", "axs_run.cpp"]
 
 NVCC = os.environ.get("NVCC", "nvcc")

@@ -851,7 +851,7 @@ int axs_inject_wait_timeout(axs_lattice *h) {
     if (L->in_ensemble)
         fail(AXS_ERR_STATE, "timeout injection on an ensemble member is not supported; use a standalone lattice");
     if (!L->tuned) lattice_evolve(L, 0);   // the configuration the next step will use (tuned unless AXS_AUTOTUNE=0)
-    if (L->cfg.kind != 1 || L->p.laplacian != 0)
+    if (!use_waiting_kernel(L))
         fail(AXS_ERR_STATE, "the step kernel in use (%s) has no device-side waits",
              L->p.laplacian != 0 ? "spectral Laplacian step" : L->cfg.describe().c_str());
     L->debug_tx_excess = 16;

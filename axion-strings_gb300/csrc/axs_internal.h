@@ -77,7 +77,7 @@ struct ZLat {
     // buffer when the momentum is updated in place.
     void *pih[2];
     double *clock;           // [2] tau at the parity of psi
-    int N, tx, ntx, nty, nzc;
+    int N, tx, ty, ntx, nty, nzc;
     int a_index;             // which of psi[0]/psi[1] is "current" at launch parity 0
     int64_t item_base;
     double dt, inv_dx2, lambda, T0sq3;
@@ -229,6 +229,7 @@ struct Ensemble {
 void step_setup(Lattice *L);
 void step_release(Lattice *L);
 bool zmarch_supported(const axs_params &p);
+bool use_waiting_kernel(Lattice *L);
 int lattice_advance(Lattice *L, int max_steps);       // one launch (eager or inside capture); steps taken
 void clear_graphs(std::map<GraphKey, GraphEntry> &g);
 void lattice_evolve(Lattice *L, int nsteps);          // graph-cached
@@ -242,6 +243,10 @@ void ensemble_autotune(Ensemble *E);
 constexpr int kStep2dSlot = 1024;   // bytes of one coefficient table
 int step2d_launch(Lattice *L, int max_steps);
 int step2d_steps(Lattice *L, int max_steps);
+// k radius-1 FP32 steps per pass, the tile in the registers of nw warps
+// of vr rows (axs_step_k.cu); prepare sets up the kernels of 1 .. kmax steps
+void launch_zmarch_k(int nw, int vr, int k, const ZLat *d, int nlat, int64_t items, int *counters, int parity, cudaStream_t st);
+void prepare_zmarch_k(int nw, int vr, int kmax);
 // radius-R z-march kernels (axs_step_r.cu), by tile shape; zr = 1 keeps the
 // z-neighbours in registers with a ring of 2R + 2 or more slots
 void launch_zmarch_r(int esz, int ty, int txmax, int slots, int r, int zr, const ZLat *d, int nlat, int64_t items,

@@ -1996,23 +1996,32 @@ static const ZVariant kZVariants[] = {
     // 56-57: radius 4 on 8 x 64 with 9 slots, radius 2 on 4 x 128 with 9 (at
     // the shared-memory limit of two CTAs per SM)
     {4, 8, 64, 9, 8, -1, 4, 0},   {4, 4, 128, 9, 8, -1, 2, 1},
+    // 58-61: up to `slots` steps per pass with the tile in the registers of ncw warps
+    // of `lean` rows (axs_step_k.cu): regions of 64 x lean ncw sites, tiles without the halo of the
+    // most steps (columns rounded up to pairs)
+    {6, 42, 56, 3, 12, -1, 0, 4}, {6, 24, 56, 4, 8, -1, 0, 4},  {6, 28, 56, 4, 12, -1, 0, 3},
+    {6, 26, 56, 3, 8, -1, 0, 4},
 };
 static const int kNumZVariants = sizeof(kZVariants) / sizeof(kZVariants[0]);
 
 static bool two_step(int variant) { return variant >= 0 && variant < kNumZVariants && kZVariants[variant].gen == 3; }
 static bool three_step(int variant) { return variant >= 0 && variant < kNumZVariants && kZVariants[variant].gen == 5; }
+static bool reg_tile(int variant) { return variant >= 0 && variant < kNumZVariants && kZVariants[variant].gen == 6; }
 static int variant_tx(const ZVariant &v, int N, int esz);
 // the variant's tiles do not divide N: the last ones overlap their neighbours (variant_tx)
 static bool overlapped(const ZVariant &v, int N, int esz) {
+    if (v.gen == 6) return false;
     const int tx = variant_tx(v, N, esz);
     return tx > 0 && (N % tx != 0 || N % v.ty != 0);
 }
 // the momentum is written out of place (pih and scratch exchange after every launch)
 static bool out_of_place(int variant, const Lattice *L) {
-    return two_step(variant) || three_step(variant) ||
+    return two_step(variant) || three_step(variant) || reg_tile(variant) ||
            (variant >= 0 && variant < kNumZVariants && overlapped(kZVariants[variant], L->p.N, L->esz));
 }
-static int steps_per_pass(int variant) { return three_step(variant) ? 3 : (two_step(variant) ? 2 : 1); }
+static int steps_per_pass(int variant) {
+    return reg_tile(variant) ? kZVariants[variant].slots : three_step(variant) ? 3 : (two_step(variant) ? 2 : 1);
+}
 static int radius(const ZVariant &v) { return v.r > 0 ? v.r : 1; }
 
 std::string StepConfig::describe() const {
@@ -2024,6 +2033,9 @@ std::string StepConfig::describe() const {
     else if (three_step(variant))
         snprintf(b, sizeof b, "TMA z-march variant %d (three steps per pass, halo depth 3; last steps on variant %d), tx=%d, zchunk=%d",
                  variant, kZVariants[variant].partner, tx, zchunk);
+    else if (reg_tile(variant))
+        snprintf(b, sizeof b, "register-tile z-march variant %d (up to %d steps per pass, %d warps), tx=%d, zchunk=%d", variant,
+                 kZVariants[variant].slots, kZVariants[variant].ncw, tx, zchunk);
     else if (variant >= 0 && variant < kNumZVariants && kZVariants[variant].gen == 4)
         snprintf(b, sizeof b, "TMA z-march variant %d (stencil radius %d), tx=%d, zchunk=%d", variant,
                  kZVariants[variant].r, tx, zchunk);
@@ -2152,7 +2164,11 @@ static void launch_zmarch5_t(const ZLat *d, int nlat, int64_t items, int *counte
 }
 
 static void launch_zmarch(int esz, int variant, const ZLat *d, int nlat, int64_t items, int *counters, int parity,
-                          int *derr, cudaStream_t st, int ctas_per_sm) {
+                          int *derr, cudaStream_t st, int ctas_per_sm, int k = 0) {
+    if (reg_tile(variant)) {   // k steps (0: as many as the variant takes)
+        launch_zmarch_k(kZVariants[variant].ncw, kZVariants[variant].lean, k > 0 ? k : kZVariants[variant].slots, d, nlat, items, counters, parity, st);
+        return;
+    }
     if (variant >= 0 && variant < kNumZVariants && kZVariants[variant].gen == 4) {
         const ZVariant &v = kZVariants[variant];
         launch_zmarch_r(esz, v.ty, v.txmax, v.slots, v.r, v.lean, d, nlat, items, counters, parity, derr, st, ctas_per_sm);
@@ -2231,6 +2247,10 @@ static void launch_zmarch(int esz, int variant, const ZLat *d, int nlat, int64_t
 }
 
 static void prepare_zmarch(int esz, int variant) {
+    if (reg_tile(variant)) {
+        prepare_zmarch_k(kZVariants[variant].ncw, kZVariants[variant].lean, kZVariants[variant].slots);
+        return;
+    }
     if (variant >= 0 && variant < kNumZVariants && kZVariants[variant].gen == 4) {
         const ZVariant &v = kZVariants[variant];
         prepare_zmarch_r(esz, v.ty, v.txmax, v.slots, v.r, v.lean);
@@ -2385,6 +2405,7 @@ static int exact_tx(const ZVariant &v, int N, int esz) {
 // periodic edge: boxes are R rows or R sites (rounded up to 16 bytes) wide
 // and start at multiples of 2, so any N serves R <= 2, multiples of 4 the rest.
 static int variant_tx(const ZVariant &v, int N, int esz) {
+    if (v.gen == 6) return esz == 4 && N >= 16 ? v.txmax : 0;   // any N: sites past the edge are masked
     if (v.gen == 5) {
         // complex float, x-tiled (the kernel takes its x halo from strips),
         // without overlap (its halo boxes are three rows high)
@@ -2411,6 +2432,19 @@ static int variant_tx(const ZVariant &v, int N, int esz) {
 // A variant serves a lattice when its stencil radius is the lattice's and it tiles N.
 static bool variant_fits(const ZVariant &v, const axs_params &p, int esz) {
     return radius(v) == p.stencil_setting + 1 && variant_tx(v, p.N, esz) > 0;
+}
+
+// For the injected wait timeout: a kernel with device-side waits (TMA) in place
+// of one without, false when none serves the lattice.
+bool use_waiting_kernel(Lattice *L) {
+    if (L->p.laplacian != 0 || L->cfg.kind != 1) return false;
+    if (!reg_tile(L->cfg.variant)) return true;
+    for (int v = 0; v < kNumZVariants; ++v)
+        if (!reg_tile(v) && variant_fits(kZVariants[v], L->p, L->esz)) {
+            L->cfg.variant = v;
+            return true;
+        }
+    return false;
 }
 
 bool zmarch_supported(const axs_params &p) {
@@ -2470,7 +2504,11 @@ static int64_t fill_zlat(ZLat &z, Lattice *L, int variant, int zchunk, int64_t i
     void *pb[2];
     pb[L->cur] = L->pih;
     pb[L->cur ^ 1] = oop ? L->scratch : L->pih;
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < 2 && v.gen == 6; ++b) {   // no tensor maps
+        z.psi[b] = L->psi[b];
+        z.pih[b] = pb[b];
+    }
+    for (int b = 0; b < 2 && v.gen != 6; ++b) {
         encode_map(&z.tm_row[b], L->psi[b], N, L->esz, tx, R);     // R halo rows
         encode_map(&z.tm_main[b], L->psi[b], N, L->esz, tx, v.ty);
         encode_map(&z.tm_xh[b], L->psi[b], N, L->esz, rp, v.ty);   // x-halo strip
@@ -2494,6 +2532,7 @@ static int64_t fill_zlat(ZLat &z, Lattice *L, int variant, int zchunk, int64_t i
     z.clock = L->dclock;
     z.N = N;
     z.tx = tx;
+    z.ty = v.ty;
     z.ntx = (N + tx - 1) / tx;
     z.nty = (N + v.ty - 1) / v.ty;
     z.nzc = std::max(1, N / std::max(1, zchunk));
@@ -2657,6 +2696,12 @@ static void spectral_release(Lattice *L) {
     L->dksq = nullptr;
 }
 
+// The steps of an interval's next pass: its passes, of at most `most` steps, evened out.
+static int even_steps(int steps, int most) {
+    const int passes = (steps + most - 1) / most;
+    return (steps + passes - 1) / passes;
+}
+
 // Advances a lattice by one launch of at most max_steps (>= 1) steps and
 // returns the steps taken: two for a two-step variant when allowed, else one.
 // The handle's bookkeeping advances here; the kernels may run later inside a
@@ -2697,7 +2742,8 @@ int lattice_advance(Lattice *L, int max_steps) {
             if (max_steps >= 2) k = 2;
             else kv = kZVariants[kv].partner;
         }
-        launch_zmarch(L->esz, kv, L->dzlat, 1, L->zitems, L->dcounter, L->cur, L->derr, L->stream, L->cfg.ctas_per_sm);
+        if (reg_tile(kv)) k = even_steps(max_steps, steps_per_pass(kv));
+        launch_zmarch(L->esz, kv, L->dzlat, 1, L->zitems, L->dcounter, L->cur, L->derr, L->stream, L->cfg.ctas_per_sm, k);
         if (L->debug_tx_excess) {   // an injected stall lasts one launch: rebuild the table before the next
             L->debug_tx_excess = 0;
             L->zlat_variant = -1;
@@ -2957,8 +3003,12 @@ void lattice_autotune(Lattice *L) {
     std::vector<std::pair<double, int>> screen;
     if (zc0 > 0)
         for (int v = 0; v < kNumZVariants; ++v)
-            if (variant_fits(kZVariants[v], L->p, L->esz) && variant_resident(L->esz, v))
-                screen.push_back({trial(v, zc0, 1, 1).second, v});
+            if (variant_fits(kZVariants[v], L->p, L->esz) && variant_resident(L->esz, v)) {
+                // register tiles take the whole SM: small lattices need short chunks
+                double ms = trial(v, zc0, 1, 1).second;
+                if (reg_tile(v) && L->p.N <= 512 && zc0 > 32) ms = std::min(ms, trial(v, 32, 1, 1).second);
+                screen.push_back({ms, v});
+            }
     std::sort(screen.begin(), screen.end());
     for (size_t k = 0; k < screen.size() && k < 3; ++k)
         for (int zc : zchunks) {
@@ -3082,8 +3132,9 @@ static int ensemble_advance(Ensemble *E, int max_steps) {
         if (max_steps >= 2) k = 2;
         else kv = kZVariants[kv].partner;
     }
+    if (reg_tile(kv)) k = even_steps(max_steps, steps_per_pass(kv));
     launch_zmarch(E->members[0]->esz, kv, E->dzlat, (int)E->members.size(), E->zitems, E->dcounter, ensemble_parity(E),
-                  E->derr, E->stream, E->cfg.ctas_per_sm);
+                  E->derr, E->stream, E->cfg.ctas_per_sm, k);
     for (Lattice *m : E->members) {
         m->cur ^= 1;
         if (out_of_place(E->cfg.variant, m)) std::swap(m->pih, m->scratch);
@@ -3125,7 +3176,6 @@ void ensemble_autotune(Ensemble *E) {
     const int zchunks[] = {32, 64, 128, 256};   // 256: whole columns of every member up to 256^3
     for (int v = 0; v < kNumZVariants; ++v) {
         if (!ensemble_variant_ok(E, v) || !variant_resident(E->members[0]->esz, v)) continue;
-        const bool two = two_step(v);
         for (int zc : zchunks) {
             StepConfig c;
             c.kind = 1;
@@ -3142,7 +3192,7 @@ void ensemble_autotune(Ensemble *E) {
                     if (out_of_place(v, m)) std::swap(m->pih, m->scratch);
                 }
             });
-            if (two) ms *= 0.5;   // per step
+            ms /= steps_per_pass(v);   // per step
             if (ms < best_ms) { best_ms = ms; best = c; }
             if (env_flag("AXS_TUNE_LOG", false))
                 fprintf(stderr, "[axs autotune ensemble] %-60s %.4f ms/step\n", c.describe().c_str(), ms);
