@@ -3170,34 +3170,41 @@ void ensemble_autotune(Ensemble *E) {
         if (!check_finite(m)) return;
     std::vector<int> cur_save;
     for (Lattice *m : E->members) cur_save.push_back(m->cur);
-    int reps = 6;
     StepConfig best = E->cfg;
     double best_ms = 1e30;
-    const int zchunks[] = {32, 64, 128, 256};   // 256: whole columns of every member up to 256^3
-    for (int v = 0; v < kNumZVariants; ++v) {
-        if (!ensemble_variant_ok(E, v) || !variant_resident(E->members[0]->esz, v)) continue;
-        for (int zc : zchunks) {
-            StepConfig c;
-            c.kind = 1;
-            c.variant = v;
-            c.zchunk = zc;
-            c.tx = variant_tx(kZVariants[v], E->members[0]->p.N, E->members[0]->esz);
-            E->cfg = c;
-            ensemble_table(E, 0.f, true);
-            double ms = time_launches(E->stream, reps, [&] {
-                launch_zmarch(E->members[0]->esz, v, E->dzlat, (int)E->members.size(), E->zitems, E->dcounter,
-                              ensemble_parity(E), E->derr, E->stream, 0);
-                for (Lattice *m : E->members) {
-                    m->cur ^= 1;
-                    if (out_of_place(v, m)) std::swap(m->pih, m->scratch);
-                }
-            });
-            ms /= steps_per_pass(v);   // per step
-            if (ms < best_ms) { best_ms = ms; best = c; }
-            if (env_flag("AXS_TUNE_LOG", false))
-                fprintf(stderr, "[axs autotune ensemble] %-60s %.4f ms/step\n", c.describe().c_str(), ms);
-        }
-    }
+    auto trial = [&](int v, int zc, int reps, int warm) {
+        StepConfig c;
+        c.kind = 1;
+        c.variant = v;
+        c.zchunk = zc;
+        c.tx = variant_tx(kZVariants[v], E->members[0]->p.N, E->members[0]->esz);
+        E->cfg = c;
+        ensemble_table(E, 0.f, true);
+        double ms = time_launches(E->stream, reps, [&] {
+            launch_zmarch(E->members[0]->esz, v, E->dzlat, (int)E->members.size(), E->zitems, E->dcounter,
+                          ensemble_parity(E), E->derr, E->stream, 0);
+            for (Lattice *m : E->members) {
+                m->cur ^= 1;
+                if (out_of_place(v, m)) std::swap(m->pih, m->scratch);
+            }
+        }, warm);
+        ms /= steps_per_pass(v);   // per step
+        if (ms < best_ms) { best_ms = ms; best = c; }
+        if (env_flag("AXS_TUNE_LOG", false))
+            fprintf(stderr, "[axs autotune ensemble] %-60s %.4f ms/step\n", c.describe().c_str(), ms);
+        return ms;
+    };
+    // as for a single lattice: every variant screened with one launch at one
+    // z-chunk, the three fastest timed at every z-chunk (256: whole columns of every
+    // member up to 256^3). Each ensemble is tuned anew: timing every variant at every
+    // z-chunk took 450 ms for 24 members
+    std::vector<std::pair<double, int>> screen;
+    for (int v = 0; v < kNumZVariants; ++v)
+        if (ensemble_variant_ok(E, v) && variant_resident(E->members[0]->esz, v)) screen.push_back({trial(v, 64, 1, 1), v});
+    std::sort(screen.begin(), screen.end());
+    best_ms = 1e30;
+    for (size_t k = 0; k < screen.size() && k < 3; ++k)
+        for (int zc : {32, 64, 128, 256}) trial(screen[k].second, zc, 6, 2);
     for (size_t i = 0; i < E->members.size(); ++i) {
         Lattice *m = E->members[i];
         if (m->cur != cur_save[i]) {
