@@ -1633,13 +1633,14 @@ __device__ __forceinline__ void zcol_march(const typename Cplx<T>::type *__restr
 }
 
 // The grid of the staged marches: blocks of 32 x 8 columns, and as many
-// z-chunks as fill the resident blocks once, none shorter than 8 planes (a
+// z-chunks as fill the resident blocks once (FP64, bound by its pipe, four times:
+// the work evens out over the SMs), none shorter than 8 planes (a
 // chunk stages A planes more than it has; lattices small enough to be cut that
 // far lie in L2). At 128^3 whole columns are 64 blocks for 152 SMs.
 template <typename T, int R>
 static dim3 zcol_grid(int N) {
     const int cols = ((N + 31) / 32) * ((N + 7) / 8), slots = num_sms() * ZMarch<T, R>::MINB;
-    return dim3(cols, std::max(1, std::min((slots + cols / 2) / cols, N / 8)));
+    return dim3(cols, std::max(1, std::min((sizeof(T) == 8 ? 4 * slots : slots) / cols, N / 8)));
 }
 
 // One thread's coefficients for the block: GB300's FP64 pipe makes them cost
@@ -2532,7 +2533,8 @@ struct EnergyAcc {
 // FP32 operations, two sites per trip (a chunk has whole pairs) so the register
 // rotation is renaming, and two sites' terms are added before one compensated
 // add. 512^3 FP32: 443 us (4.9 TB/s), 476 without the packed operations and the
-// uniform addresses.
+// uniform addresses (two columns per lane with 16-byte loads and shuffles, at two
+// blocks per SM: 602).
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_energies_zcol(const typename Cplx<T>::type *__restrict__ psi,
                                                          const typename Cplx<T>::type *__restrict__ pih,
