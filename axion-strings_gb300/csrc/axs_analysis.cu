@@ -907,9 +907,12 @@ __global__ void __launch_bounds__(128) k_bin(const typename Cplx<T>::type *__res
 }
 
 // One block per bin: strided partial sums over the blocks in a fixed order,
-// then a fixed shuffle tree; out = [pk | |n| | count] rows of nbins.
-__global__ void k_bin_final3(const double *__restrict__ partials, int nblocks, int nbins, double *__restrict__ out) {
+// then a fixed shuffle tree; out = [pk | |n| | count] rows of nbins. The lattice's
+// error flag goes to `flag` if given (page-locked memory: one copy less per call).
+__global__ void k_bin_final3(const double *__restrict__ partials, int nblocks, int nbins, double *__restrict__ out,
+                             const int *__restrict__ derr, int *flag) {
     const int bn = blockIdx.x;
+    if (flag && bn == 0 && threadIdx.x == 0) *flag = *derr;
     double v[3] = {0.0, 0.0, 0.0};
     for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
 #pragma unroll
@@ -959,6 +962,11 @@ struct RefBinsI {
         if (b >= 0) return min((b + 2) * (b + 2), half * half);
         return n2 == 0 ? 1 : INT_MAX;   // the origin, or past the last bin for good
     }
+    // modes ix >= limit(c2) of a row are in no bin (the root is within 0.01: + 2 is past it)
+    __device__ __forceinline__ int limit(int c2) const {
+        const int m = half * half - c2;
+        return m <= 0 ? 0 : (int)sqrtf((float)m) + 2;
+    }
 };
 struct LogBinsI {
     const int *thr;   // thr[b] for b = 1..nbins-1 (thr[0] = 0)
@@ -990,6 +998,7 @@ struct LogBinsI {
         if (b >= 0) return b + 1 < nbins ? thr[b + 1] : INT_MAX;
         return 1;   // b < 0 only at the origin (n2 = 0)
     }
+    __device__ __forceinline__ int limit(int) const { return INT_MAX; }
 };
 
 // Float-float values (hi + lo, about 48 significant bits): the warp-level sums
@@ -1107,24 +1116,37 @@ __device__ __forceinline__ FF run_power(const float2 *s, int s0, int a, int e, i
     return v;
 }
 
-template <typename T> __device__ __forceinline__ FF mode_power(const typename Cplx<T>::type &f);
-template <> __device__ __forceinline__ FF mode_power<float>(const float2 &f) { return FF{fmaf(f.x, f.x, f.y * f.y), 0.0f}; }
-template <> __device__ __forceinline__ FF mode_power<double>(const double2 &f) {
-    const double v = f.x * f.x + f.y * f.y;
-    const float hi = __double2float_rn(v);
-    return FF{hi, __double2float_rn(v - (double)hi)};
+// Asynchronous copies of 8 or 16 bytes from global to shared memory.
+__device__ __forceinline__ void cp_async_ca(uint32_t dst, const void *src, int bytes) {
+    if (bytes == 16) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int P>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(P) : "memory"); }
 
-// Run-length binner over the rows of the half spectrum. Along a row |n|^2 =
-// ix^2 + c only grows, so the bins do too: each lane takes a contiguous slice
-// of the (shared-memory staged) row and sums runs of one bin in registers
-// (float-float). A run strictly inside a lane's slice belongs to that lane
-// alone and goes straight into the warp's histogram; a lane's first run may
-// continue runs of the lanes before it (equal bins sit in consecutive lanes:
+// Run-length binner over the rows of the half spectrum. A unit of a warp's work
+// is (group, segment). A group holds the rows whose frequencies are (+-gz, +-gy),
+// gz and gy in 0 .. N/2 (2D: +-gy): up to four rows with the same c = fy^2 +
+// fz^2, hence the same bin at every ix: the bins are looked up, the runs closed
+// and the histograms updated once for the group. FP32 modes are staged in shared
+// memory, `rb` rows at a time (each lane's copies all in flight at once), FP64
+// modes as their powers' sums over the group's rows, added in double on the way
+// in (hi + lo floats: one split for four modes off GB300's FP64 pipe). Modes past
+// the last bin are not read. Along the row |n|^2 = ix^2 + c only grows, so the
+// bins do too: each lane takes a contiguous slice and sums its runs of one bin
+// in registers (float-float). A run strictly inside a lane's slice belongs to
+// that lane alone and goes straight into the warp's histogram; a lane's first run
+// may continue runs of the lanes before it (equal bins sit in consecutive lanes:
 // one segmented scan of 5 shuffle steps), and its last run has a bin no other
-// lane's last run has. Every bin thus receives its sums in an order fixed by
-// the data: results are the same run to run and for an ensemble member alone.
-// Rows are taken in groups that share every bin boundary (see the unit loop).
+// lane's last run has. Every bin thus receives its sums in an order fixed by the
+// data: results are the same run to run and for an ensemble member alone.
+// Bound by the issue slots (65 to 73 % busy): 512^3 FP32, the 256 reference bins
+// 165 us (307 MB: the modes past the last bin are not read), 128 logarithmic ones
+// 164 us (539 MB: 3.3 TB/s). With each row of a group staged, looked up and closed by
+// itself: 443 and 245 us; staged together but taken from run to run: 308 and 183 us
+// (lanes wait for the longest run). Adding the rows' powers before the runs would
+// take 69 and 102 us, but moves the FP32 sums by 1e-8.
 // Per-warp histograms (float-float slots), block partial rows in double and
 // k_bin_final3 (three rows: power, |n|, count). With KS false only the power
 // row is summed and held (the |n| and count rows, which depend on N and the
@@ -1137,11 +1159,11 @@ template <> __device__ __forceinline__ FF mode_power<double>(const double2 &f) {
 // One segment per row and one pass is the common case.
 template <typename T, typename B, bool KS>
 __global__ void __launch_bounds__(128, 8) k_bin_runs(const typename Cplx<T>::type *__restrict__ F, int N, int ndims,
-                                                  B binner, int nbins, int seg, int b0, int nbp,
-                                                  double *__restrict__ partials, int *derr) {
+                                                     B binner, int nbins, int seg, int b0, int nbp, int rb,
+                                                     double *__restrict__ partials) {
     typedef typename Cplx<T>::type C;
-    constexpr bool kRuns = sizeof(T) == 4;   // FP32 modes: whole runs per bin lookup
-    // [4 warps][HR][nbp] histograms, bin table, [4 warps][2][sbuf] staging buffers, [4 warps][2] mbarriers
+    constexpr bool kF32 = sizeof(T) == 4;
+    // [4 warps][HR][nbp] histograms, bin table, [4 warps][rb][seg] staged modes (FP64: [4 warps][seg] sums)
     extern __shared__ double hist[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int nh = N / 2 + 1;
@@ -1150,234 +1172,173 @@ __global__ void __launch_bounds__(128, 8) k_bin_runs(const typename Cplx<T>::typ
     constexpr int HR = KS ? 3 : 1;   // histogram rows: power (and |n|, count on a binning's first call)
     for (int i = threadIdx.x; i < 4 * HR * nbp; i += blockDim.x) hist[i] = 0.0;
     const B bins = binner.staged(hist + 4 * HR * nbp);
-    // Row segments arrive by bulk copies into two staging buffers per warp: the
-    // next unit's copy is in flight while this one is binned. A buffer holds a
-    // segment and up to one mode either side (the copy starts and ends on 16
-    // bytes); buffers start 16-byte aligned, the warp's two mbarriers follow.
-    const int sbuf = (seg + 3) & ~1;
-    C *stg = reinterpret_cast<C *>(hist + ((4 * HR * nbp + B::kSmemTable * nbins + 1) & ~1)) + (size_t)w * 2 * sbuf;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(reinterpret_cast<C *>(hist + ((4 * HR * nbp + B::kSmemTable * nbins + 1) & ~1)) +
-                                                  (size_t)4 * 2 * sbuf) + 2 * w;
-    if (lane == 0) {
-        mbar_init(smem_u32(&bars[0]), 1);
-        mbar_init(smem_u32(&bars[1]), 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
+    float2 *const stg = reinterpret_cast<float2 *>(hist + 4 * HR * nbp + B::kSmemTable * nbins) + (size_t)w * rb * seg;
     __syncthreads();
     double *hp = hist + (size_t)w * HR * nbp;   // indexed by bin - b0
     double *hk = hp + nbp;
     double *hc = hk + nbp;
     auto in_pass = [&](int bb) { return bb >= b0 && bb < b1; };
-    // A unit is (group, segment si). A group holds the rows whose frequencies
-    // are (+-gz, +-gy), gz and gy in 0 .. N/2 (2D: +-gy): up to four rows with
-    // the same c = fy^2 + fz^2, hence the same bin at every x. A lane's slice
-    // has the same runs in each of them, so its first and last runs are summed
-    // over the group's rows in registers, and the segmented scan and the
-    // histogram updates run once per group instead of once per row. There are
-    // (N/2 + 1)^2 nseg < 2^31 units (3D N <= 4096; 2D far fewer): int.
-    const int gh = N / 2 + 1;
-    const int units = (ndims == 3 ? gh * gh : gh) * nseg;
-    const int nwarps = gridDim.x * 4;
-    // The mode offset of unit uu's copy below its first mode (FP32 modes are 8
-    // bytes; the array and every row-segment copy start on 16 bytes), and the
-    // copy itself (lane 0). The copy ends on 16 bytes too: at most one mode
-    // past the segment, which exists (the array holds an even number of modes,
-    // so the last segment's copy ends exactly at its end).
-    auto unit_off = [&](int rr, int ssi) -> int {
-        return sizeof(C) == 8 ? (int)(((unsigned)rr * (unsigned)nh + (unsigned)(ssi * seg)) & 1u) : 0;
-    };
-    auto issue = [&](int rr, int ssi, int buf) {
-        const int ss0 = ssi * seg, ssl = min(seg, nh - ss0);
-        const int off = unit_off(rr, ssi);
-        const uint32_t bytes = (uint32_t)(((size_t)(ssl + off) * sizeof(C) + 15) & ~(size_t)15);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // after this warp's reads of the buffer
-        mbar_expect_tx(smem_u32(&bars[buf]), bytes);
-        bulk_load(smem_u32(stg + (size_t)buf * sbuf), F + (int64_t)rr * nh + ss0 - off, bytes, smem_u32(&bars[buf]));
-    };
-    struct Unit {
-        int gz, gy, si, ny, cnt;   // ny: 1 or 2 values of y; cnt: rows in the group
-    };
-    auto unit_at = [&](int uu) {
-        const int g = uu / nseg;
-        Unit q;
-        q.si = uu - g * nseg;
-        q.gz = ndims == 3 ? g / gh : 0;
-        q.gy = ndims == 3 ? g - q.gz * gh : g;
-        q.ny = (q.gy == 0 || 2 * q.gy == N) ? 1 : 2;
-        q.cnt = q.ny * ((ndims == 2 || q.gz == 0 || 2 * q.gz == N) ? 1 : 2);
-        return q;
-    };
-    // row m of a group: y = gy, then N - gy; z = gz, then N - gz
-    auto row_of = [&](const Unit &q, int m) {
-        const int jz = m >= q.ny ? 1 : 0, jy = m - jz * q.ny;
-        const int iy = jy ? N - q.gy : q.gy;
-        return ndims == 2 ? iy : (jz ? N - q.gz : q.gz) * N + iy;
-    };
-    const int ufirst = blockIdx.x * 4 + w;
-    if (lane == 0 && ufirst < units) {
-        const Unit q0 = unit_at(ufirst);
-        issue(row_of(q0, 0), q0.si, 0);
-    }
-    int it = 0;            // row copies taken by this warp: buffer it & 1, phase (it >> 1) & 1
-    bool ok = true;
-    bool more = false;     // a copy after the current one is in flight
-    for (int u = ufirst; u < units; u += nwarps) {
-        const Unit q = unit_at(u);
-        const int s0 = q.si * seg, sl = min(seg, nh - s0);
+    // There are nh^2 nseg < 2^31 units (3D N <= 4096; 2D far fewer): int.
+    const int units = (ndims == 3 ? nh * nh : nh) * nseg;
+    for (int u = blockIdx.x * 4 + w; u < units; u += gridDim.x * 4) {
+        const int g = u / nseg, s0 = (u - g * nseg) * seg;
+        const int gz = ndims == 3 ? g / nh : 0, gy = g - gz * nh;
+        // |n|^2 = ix^2 + fy^2 (+ fz^2) <= 2 (N/2)^2 < 2^31 in 2D (N <= 32768), 3 (N/2)^2 in 3D (N <= 4096): int
+        const int c2 = gy * gy + gz * gz;
+        const int sl = min(seg, nh - s0);
+        const int ll = min(sl, bins.limit(c2) - s0);   // modes of the segment that may have bins
+        if (ll <= 0) continue;
+        // row m of the group: y = gy, then N - gy; z = gz, then N - gz
+        const int ny = (gy == 0 || 2 * gy == N) ? 1 : 2;
+        const int cnt = ny * ((ndims == 2 || gz == 0 || 2 * gz == N) ? 1 : 2);
+        auto row_of = [&](int m) {
+            const int jz = m >= ny ? 1 : 0, jy = m - jz * ny;
+            const int iy = jy ? N - gy : gy;
+            return F + (int64_t)(ndims == 2 ? iy : (jz ? N - gz : gz) * N + iy) * nh + s0;
+        };
         // Lane slices of an odd number of modes: lanes reading mode k of their
         // slices at once are 2 * chunk words apart, which spreads them over the
         // 32 banks (an even chunk such as 16 put every lane on one bank).
         const int chunk = ((sl + 31) / 32) | 1;
-        const int lo = s0 + min(sl, lane * chunk), hi = s0 + min(sl, lane * chunk + chunk);
-        // |n|^2 = ix^2 + fy^2 (+ fz^2) <= 2 (N/2)^2 < 2^31 in 2D (N <= 32768), 3 (N/2)^2 in 3D (N <= 4096): int
-        const int c2 = q.gy * q.gy + q.gz * q.gz;
+        const int lo = s0 + min(ll, lane * chunk), hi = s0 + min(ll, lane * chunk + chunk);
         int fb = -1, lb = -1;   // the slice's first and last runs' bins, the same in every row of the group
-        int nr = 0, r1b = -1, r1e = 0, r2b = -1;   // FP32: the slice's runs in the group's first row (count, bins, first end)
         FF fv{0.f, 0.f}, fk{0.f, 0.f}, lv{0.f, 0.f}, lk{0.f, 0.f};
         int fc = 0, lc = 0;
-        for (int m = 0; m < q.cnt; ++m, ++it) {
-            const int cur = it & 1;
-            __syncwarp();   // every lane is done with the other buffer (the previous row)
-            more = m + 1 < q.cnt || u + nwarps < units;
-            if (lane == 0 && more) {
-                if (m + 1 < q.cnt) {
-                    issue(row_of(q, m + 1), q.si, cur ^ 1);
-                } else {
-                    const Unit qn = unit_at(u + nwarps);
-                    issue(row_of(qn, 0), qn.si, cur ^ 1);
+        for (int m0 = 0; m0 < cnt; m0 += kF32 ? rb : cnt) {
+            const int rows = kF32 ? min(rb, cnt - m0) : 1;   // staged rows
+            if constexpr (kF32) {
+                for (int r = 0; r < rows; ++r) {
+                    const C *src = row_of(m0 + r);
+                    for (int x = lane; x < ll; x += 32) cp_async_ca(smem_u32(stg + r * seg + x), src + x, 8);
+                }
+                cp_async_commit();
+                cp_async_wait<0>();
+            } else {
+                const C *r0 = row_of(0), *r1 = row_of(min(1, cnt - 1)), *r2 = row_of(min(2, cnt - 1)), *r3 = row_of(cnt - 1);
+                for (int x = lane; x < ll; x += 32) {   // cnt is 1, 2 or 4
+                    const C f0 = __ldcs(r0 + x);
+                    C f1{0, 0}, f2{0, 0}, f3{0, 0};
+                    if (cnt >= 2) f1 = __ldcs(r1 + x);
+                    if (cnt == 4) {
+                        f2 = __ldcs(r2 + x);
+                        f3 = __ldcs(r3 + x);
+                    }
+                    double pa = f0.x * f0.x + f0.y * f0.y, pb = f1.x * f1.x + f1.y * f1.y;
+                    pa += f2.x * f2.x + f2.y * f2.y;
+                    pb += f3.x * f3.x + f3.y * f3.y;
+                    const double v = pa + pb;
+                    const float wt = (s0 + x == 0 || s0 + x == nh - 1) ? 1.f : 2.f;   // x1 or x2: exact
+                    const float h = __double2float_rn(v);
+                    stg[x] = make_float2(wt * h, wt * __double2float_rn(v - (double)h));
                 }
             }
-            ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&bars[cur]), (uint32_t)((it >> 1) & 1)));
-            if (!ok) break;
-            const C *stage = stg + (size_t)cur * sbuf + unit_off(row_of(q, m), q.si);
+            __syncwarp();
             int b = -1;
             int up = 0;          // the bin is looked up again once n2 reaches this
-            bool inp = false;    // in_pass(b)
-            bool first = true;   // no run of this row has ended yet
+            bool first = true;   // no run has ended yet
             FF v{0.f, 0.f}, kk{0.f, 0.f};
             int c = 0;
-            // a run of bin b ended inside the slice: the row's first (summed over
-            // the group's rows), or one strictly inside, straight to the histogram
-            auto close_run = [&]() {
-                if (b < 0) return;
-                if (first) {
-                    fb = b;
-                    fv = ff_add(fv, v);
-                    if constexpr (KS) {
+            // the bin of n2 >= up; the run of the bin before it, if any, ended inside the slice
+            auto next_run = [&](int n2) {
+                const int nb = bins.next(b, n2);
+                up = bins.upper(nb, n2);
+                if (b >= 0) {
+                    if (first) {
+                        fb = b;
+                        fv = ff_add(fv, v);
                         fk = ff_add(fk, kk);
                         fc += c;
-                    }
-                    first = false;
-                } else if (in_pass(b)) {
-                    ff_acc(hp + (b - b0), v);
-                    if constexpr (KS) {
-                        ff_acc(hk + (b - b0), kk);
-                        ff_acc(hc + (b - b0), FF{(float)c, 0.f});
+                        first = false;
+                    } else if (in_pass(b)) {
+                        ff_acc(hp + (b - b0), v);
+                        if constexpr (KS) {
+                            ff_acc(hk + (b - b0), kk);
+                            ff_acc(hc + (b - b0), FF{(float)c, 0.f});
+                        }
                     }
                 }
+                b = nb;
+                v = kk = FF{0.f, 0.f};
+                c = 0;
             };
-            if constexpr (kRuns) {
-                // FP32: jump from run to run. A run ends where n2 reaches `up`, at
-                // ix = ceil(sqrt(up - c2)); its power is summed by run_power, so a
-                // binning's first call (KS: also |n| and the mode count, per mode)
-                // and its later calls give the same power sums. The group's later
-                // rows have the first row's runs: a slice of one or two runs
-                // replays them without the bin lookups.
-                const float2 *sf = reinterpret_cast<const float2 *>(stage);
-                if (m > 0 && nr <= 2) {
-                    if (nr > 0) {
-                        b = r1b;
-                        if (b >= 0 && in_pass(b)) v = run_power(sf, s0, lo, r1e, nh, v);
+            // the |n| sum and count of mode a: the same in every row of the group,
+            // so once, times the rows (1, 2 or 4: exact)
+            auto count_mode = [&](int a) {
+                const int wt = ((a == 0 || a == nh - 1) ? 1 : 2) * cnt;
+                kk = ff_add(kk, ff_scale(mode_norm(a * a + c2), (float)wt));
+                c += wt;
+            };
+            if (kF32 && chunk < 16) {
+                // The lanes take their slices mode by mode, in step. A run is at most
+                // one block of run_power's (and the row's first and last modes, of
+                // weight 1, blocks by themselves): its two chains over the staged
+                // rows in registers, the same bits.
+                float t0[4] = {0.f, 0.f, 0.f, 0.f}, t1[4] = {0.f, 0.f, 0.f, 0.f}, wt = 0.f;
+                auto end_block = [&]() {
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        if (r < rows) {
+                            v = ff_add(v, FF{wt * (t0[r] + t1[r]), 0.f});
+                            t0[r] = t1[r] = 0.f;
+                        }
+                };
+                const float2 *q = stg + (lo - s0);
+                for (int ix = lo; ix < hi; ++ix, ++q) {
+                    const int n2 = ix * ix + c2;
+                    if (n2 >= up || ix == 1 || ix == nh - 1) {
+                        end_block();
+                        wt = (ix == 0 || ix == nh - 1) ? 1.f : 2.f;
+                        if (n2 >= up) next_run(n2);
                     }
-                    if (nr == 2) {
-                        close_run();
-                        b = r2b;
-                        v = FF{0.f, 0.f};
-                        if (b >= 0 && in_pass(b)) v = run_power(sf, s0, r1e, hi, nh, v);
-                    }
-                } else
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        if (r < rows) {
+                            const float2 f = q[r * seg];
+                            const float t = fmaf(f.x, f.x, fmaf(f.y, f.y, t0[r]));
+                            t0[r] = t1[r];   // the chains take the modes in turn
+                            t1[r] = t;
+                        }
+                    if constexpr (KS)
+                        if (m0 == 0) count_mode(ix);
+                }
+                end_block();
+            } else {
+                // From run to run: a run ends where n2 reaches `up`, at ix = ceil(sqrt(up - c2)).
                 for (int ix = lo; ix < hi;) {
                     const int n2 = ix * ix + c2;
-                    if (n2 >= up) {   // every pass but the first: n2 reached the bound of b's run
-                        const int nb = bins.next(b, n2);
-                        up = bins.upper(nb, n2);
-                        close_run();
-                        b = nb;
-                        v = kk = FF{0.f, 0.f};
-                        c = 0;
-                    }
+                    if (n2 >= up) next_run(n2);   // every pass but the first: n2 reached the bound of b's run
                     const int e = up == INT_MAX ? hi : min(hi, ceil_isqrt(up - c2));
-                    if (m == 0) {   // the slice's runs, for the group's later rows
-                        if (nr == 0) {
-                            r1b = b;
-                            r1e = e;
-                        } else if (nr == 1) {
-                            r2b = b;
-                        }
-                        ++nr;
-                    }
                     if (b >= 0 && in_pass(b)) {
-                        v = run_power(sf, s0, ix, e, nh, v);
-                        // the |n| sums and mode counts are the same in every row of
-                        // the group: the first row's, times the rows (1, 2 or 4: exact)
+                        if constexpr (kF32) {
+                            for (int r = 0; r < rows; ++r) v = run_power(stg + r * seg, s0, ix, e, nh, v);
+                        } else {
+                            for (int a = ix; a < e; ++a) {
+                                const float2 t = stg[a - s0];
+                                v = ff_add(v, FF{t.x, t.y});
+                            }
+                        }
                         if constexpr (KS)
-                            if (m == 0)
-                                for (int a = ix; a < e; ++a) {
-                                    const int wt = ((a == 0 || 2 * a == N) ? 1 : 2) * q.cnt;
-                                    kk = ff_add(kk, ff_scale(mode_norm(a * a + c2), (float)wt));
-                                    c += wt;
-                                }
+                            if (m0 == 0)
+                                for (int a = ix; a < e; ++a) count_mode(a);
                     }
                     ix = e;
                 }
-            } else
-            for (int ix = lo; ix < hi; ++ix) {
-                const int n2 = ix * ix + c2;
-                int nb = b;
-                if (n2 >= up) {
-                    nb = bins.next(b, n2);
-                    up = bins.upper(nb, n2);
-                }
-                if (nb != b) {
-                    close_run();
-                    b = nb;
-                    inp = in_pass(b);
-                    v = kk = FF{0.f, 0.f};
-                    c = 0;
-                }
-                if (inp) {
-                    const int wt = (ix == 0 || 2 * ix == N) ? 1 : 2;
-                    const float fw = (float)wt;   // x1 or x2: exact in float-float
-                    const FF p = mode_power<T>(stage[ix - s0]);
-                    v = ff_add(v, FF{fw * p.hi, fw * p.lo});
-                    if constexpr (KS) {
-                        if (m == 0) {   // as above: the first row's |n| and count, times the rows
-                            kk = ff_add(kk, ff_scale(mode_norm(n2), fw * (float)q.cnt));
-                            c += wt * q.cnt;
-                        }
-                    }
-                }
             }
-            if (b >= 0) {   // the open run: the row's first if none ended, else the slice's last
+            if (b >= 0) {   // the open run: the slice's first if none ended, else its last
                 if (first) {
                     fb = b;
                     fv = ff_add(fv, v);
-                    if constexpr (KS) {
-                        fk = ff_add(fk, kk);
-                        fc += c;
-                    }
+                    fk = ff_add(fk, kk);
+                    fc += c;
                 } else {
                     lb = b;
                     lv = ff_add(lv, v);
-                    if constexpr (KS) {
-                        lk = ff_add(lk, kk);
-                        lc += c;
-                    }
+                    lk = ff_add(lk, kk);
+                    lc += c;
                 }
             }
+            __syncwarp();   // inside runs are in; the staged modes are no longer read
         }
-        if (!ok) break;
-        __syncwarp();   // inside runs are in; the staged rows are no longer read
         // first runs: inclusive segmented scan over lanes with equal bins
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -1412,14 +1373,6 @@ __global__ void __launch_bounds__(128, 8) k_bin_runs(const typename Cplx<T>::typ
                 ff_acc(hk + (lb - b0), lk);
                 ff_acc(hc + (lb - b0), FF{(float)lc, 0.f});
             }
-        }
-        __syncwarp();
-    }
-    if (!ok) {   // a copy never completed: flag it, then wait (bounded) for this warp's copies in flight
-        if (lane == 0) {
-            atomicOr(derr, DEVERR_TIMEOUT);
-            mbar_wait_bounded(smem_u32(&bars[it & 1]), (uint32_t)((it >> 1) & 1));
-            if (more) mbar_wait_bounded(smem_u32(&bars[(it + 1) & 1]), (uint32_t)(((it + 1) >> 1) & 1));
         }
         __syncwarp();
     }
@@ -1472,14 +1425,6 @@ __global__ void k_gather_axion(const typename Cplx<T>::type *__restrict__ psi, c
 // staged tiles R + 1 planes ahead. Reading the 4R in-plane neighbours from
 // global memory left the warps waiting on L1/L2 latency, and register-held
 // column loads could keep too few bytes in flight for the DRAM rate.
-
-__device__ __forceinline__ void cp_async_ca(uint32_t dst, const void *src, int bytes) {
-    if (bytes == 16) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int P>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(P) : "memory"); }
 
 // Geometry of the radius-R march. A plane tile is TH = 8 + 2R rows of
 // TW = 32 + 2RX elements (the block's columns and their periodic halo);
@@ -1897,33 +1842,31 @@ static BinPending bin_spectrum_enqueue(Lattice *L, const B &binner, int kind, co
     const bool ks = geom == nullptr;
     const int N = L->p.N;
     const int nh = N / 2 + 1;
-    // shared memory of one block: 4 warp histograms of nbp bins x 3 rows (1 row
-    // when only the power is summed), the bin table, two staging buffers of a
-    // segment of seg modes per warp. Whole rows and every bin in one pass when
-    // they fit (up to N ~ 1500); else segments of 2048 modes, then passes over
-    // the bins.
-    // k_bin_runs' layout: histograms (hr rows), table, 4 x 2 buffers, 8 mbarriers
-    auto smem_of = [&](int nbp, int seg, int hr) {
-        return (size_t)((4 * hr * nbp + B::kSmemTable * nbins + 1) & ~1) * sizeof(double) +
-               (size_t)4 * 2 * ((seg + 3) & ~1) * 2 * L->esz + 8 * sizeof(uint64_t);
-    };
-    // The segments, the bin passes and the grid fix which modes each lane and
-    // each warp sums, hence the bits: they follow from the first call's layout
-    // (three histogram rows) for every call, so later calls (one row) give the
-    // first call's power sums exactly.
+    // The segments and the bin passes fix which modes each lane sums, hence the
+    // bits of FP32 spectra: they follow from one layout (4 warp histograms of nbp
+    // bins x 3 rows, the bin table, two rows' segments per warp) for every call.
+    // Whole rows and every bin in one pass when that fits (up to N ~ 3000); else
+    // segments of 2048 modes, then passes over the bins.
     const size_t cap = 200 * 1024;
     int nbp = nbins, seg = nh;
-    while (smem_of(nbp, seg, 3) > cap) {
+    while ((size_t)((12 * nbp + B::kSmemTable * nbins + 1) & ~1) * sizeof(double) +
+               (size_t)4 * 2 * ((seg + 3) & ~1) * 2 * L->esz + 64 > cap) {
         if (seg > 2048) seg = 2048;
         else if (nbp > 512) nbp = (nbp + 1) / 2;
         else if (seg > 256) seg /= 2;
         else fail(AXS_ERR_ARG, "spectrum binning with %d bins does not fit shared memory", nbins);
     }
-    const size_t sm = smem_of(nbp, seg, ks ? 3 : 1);
+    // k_bin_runs' layout: histograms (hr rows), table, staged rows. All four rows of
+    // a 3D group at once while four blocks fit an SM, else two (2D groups have two).
+    auto smem_of = [&](int hr, int rb) {
+        return (size_t)(4 * hr * nbp + B::kSmemTable * nbins) * sizeof(double) + (size_t)4 * rb * seg * sizeof(float2);
+    };
+    const int rb = L->esz == 8 ? 1 : (L->p.NDIMS == 3 && smem_of(1, 4) <= cap / 4 && smem_of(3, 4) <= cap ? 4 : 2);
+    const size_t sm = smem_of(ks ? 3 : 1, rb);
     // as many 4-warp blocks as the later calls' layout fits on the SMs (up to 16
-    // per SM): the per-warp histograms leave this kernel latency-bound at low
-    // occupancy; the first call runs the same grid in more waves
-    int per_sm = (int)std::max<size_t>(1, std::min<size_t>(16, cap / std::max<size_t>(smem_of(nbp, seg, 1), 1)));
+    // per SM), in the first call too: the per-warp histograms leave this kernel
+    // latency-bound at low occupancy
+    int per_sm = (int)std::max<size_t>(1, std::min<size_t>(16, cap / std::max<size_t>(smem_of(1, rb), 1)));
     // k_bin_runs' units: groups of up to four rows (+-gz, +-gy) times segments
     const int64_t groups = L->p.NDIMS == 2 ? (int64_t)nh : (int64_t)nh * nh;
     const int64_t units = groups * ((nh + seg - 1) / seg);
@@ -1931,23 +1874,22 @@ static BinPending bin_spectrum_enqueue(Lattice *L, const B &binner, int kind, co
     int nblk = (int)std::min<int64_t>((int64_t)num_sms() * per_sm, (units + 3) / 4);   // whole units per warp
     double *part = (double *)lattice_tmp(L, 0, (size_t)nblk * 3 * nbp * sizeof(double) + (size_t)3 * nbp * sizeof(double));
     double *out = part + (size_t)nblk * 3 * nbp;
-    auto kern = L->esz == 4 ? (ks ? (const void *)k_bin_runs<float, B, true> : (const void *)k_bin_runs<float, B, false>)
-                            : (ks ? (const void *)k_bin_runs<double, B, true> : (const void *)k_bin_runs<double, B, false>);
-    if (sm > 48 * 1024) AXS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    auto launch = [&](auto kern, const auto *F, int b0, int nb) {
+        if (sm > 48 * 1024) AXS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        kern<<<nblk, 128, sm, L->stream>>>(F, N, L->p.NDIMS, binner, nbins, seg, b0, nb, rb, part);
+    };
     for (int b0 = 0; b0 < nbins; b0 += nbp) {
         const int nb = std::min(nbp, nbins - b0);
-        if (L->esz == 4) {
-            if (ks) k_bin_runs<float, B, true><<<nblk, 128, sm, L->stream>>>((const float2 *)L->fft_out, N, L->p.NDIMS, binner, nbins, seg, b0, nb, part, L->derr);
-            else k_bin_runs<float, B, false><<<nblk, 128, sm, L->stream>>>((const float2 *)L->fft_out, N, L->p.NDIMS, binner, nbins, seg, b0, nb, part, L->derr);
-        } else {
-            if (ks) k_bin_runs<double, B, true><<<nblk, 128, sm, L->stream>>>((const double2 *)L->fft_out, N, L->p.NDIMS, binner, nbins, seg, b0, nb, part, L->derr);
-            else k_bin_runs<double, B, false><<<nblk, 128, sm, L->stream>>>((const double2 *)L->fft_out, N, L->p.NDIMS, binner, nbins, seg, b0, nb, part, L->derr);
-        }
+        if (L->esz == 4) ks ? launch(k_bin_runs<float, B, true>, (const float2 *)L->fft_out, b0, nb)
+                            : launch(k_bin_runs<float, B, false>, (const float2 *)L->fft_out, b0, nb);
+        else ks ? launch(k_bin_runs<double, B, true>, (const double2 *)L->fft_out, b0, nb)
+                : launch(k_bin_runs<double, B, false>, (const double2 *)L->fft_out, b0, nb);
         AXS_CUDA(cudaGetLastError());
         // rows (power, |n|, count) of this pass at host[3 b0 ..], which the kernel
         // writes itself when host is page-locked; otherwise the next pass
         // overwrites `out` only after this copy (stream order)
-        k_bin_final3<<<nb, 256, 0, L->stream>>>(part, nblk, nb, pinned ? host + 3 * (size_t)b0 : out);
+        k_bin_final3<<<nb, 256, 0, L->stream>>>(part, nblk, nb, pinned ? host + 3 * (size_t)b0 : out, L->derr,
+                                               pinned ? (int *)(host + 3 * (size_t)nbins) : nullptr);
         AXS_CUDA(cudaGetLastError());
         count_launches(2);
         if (!pinned)
@@ -1955,7 +1897,8 @@ static BinPending bin_spectrum_enqueue(Lattice *L, const B &binner, int kind, co
                                      L->stream));
     }
     // the lattice's error flag into the slot after the rows (host holds 3 nbins + 1 doubles)
-    AXS_CUDA(cudaMemcpyAsync(host + 3 * (size_t)nbins, L->derr, sizeof(int), cudaMemcpyDeviceToHost, L->stream));
+    if (!pinned)
+        AXS_CUDA(cudaMemcpyAsync(host + 3 * (size_t)nbins, L->derr, sizeof(int), cudaMemcpyDeviceToHost, L->stream));
     BinPending pd;
     pd.nbins = nbins;
     pd.nbp = nbp;
@@ -1972,11 +1915,11 @@ static BinPending bin_spectrum_enqueue(Lattice *L, const B &binner, int kind, co
 static void bin_spectrum_finish(Lattice *L, const BinPending &pd, std::vector<double> &psum, std::vector<double> &nsum,
                                 std::vector<unsigned long long> &cnt) {
     const int nbins = pd.nbins;
-    int flag = 0;   // the error flag copied after the rows (k_bin_runs' row copies complete on bounded waits)
+    int flag = 0;   // the lattice's error flag, copied after the rows: set by a step before this call
     memcpy(&flag, pd.host + 3 * (size_t)nbins, sizeof(int));
     if (flag & DEVERR_TIMEOUT) {
         AXS_CUDA(cudaMemsetAsync(L->derr, 0, sizeof(int), L->stream));
-        fail(AXS_ERR_TIMEOUT, "the spectrum binner gave up waiting for a row copy; the spectrum was not computed");
+        fail(AXS_ERR_TIMEOUT, "a step kernel gave up waiting for a TMA load; the spectrum was not computed");
     }
     psum.assign(nbins, 0.0);
     std::vector<double> nk(pd.ks ? nbins : 0, 0.0), cc(pd.ks ? nbins : 0, 0.0);
