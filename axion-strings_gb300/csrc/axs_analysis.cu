@@ -1268,8 +1268,11 @@ __global__ void __launch_bounds__(128, 8) k_bin_runs(const typename Cplx<T>::typ
                 kk = ff_add(kk, ff_scale(mode_norm(a * a + c2), (float)wt));
                 c += wt;
             };
-            if (kF32 && chunk < 16) {
-                // The lanes take their slices mode by mode, in step. A run is at most
+            if (kF32 && chunk < 16 && (cnt <= rb || !B::kSmemTable)) {
+                // The lanes take their slices mode by mode, in step, unless the bins are
+                // long (logarithmic) and the group's rows take more than one round:
+                // 720^3 FP32, two rows at a time, 128 logarithmic bins 543 us in step and
+                // 398 from run to run, the reference's 565 and 828. A run is at most
                 // one block of run_power's (and the row's first and last modes, of
                 // weight 1, blocks by themselves): its two chains over the staged
                 // rows in registers, the same bits.
@@ -1857,11 +1860,13 @@ static BinPending bin_spectrum_enqueue(Lattice *L, const B &binner, int kind, co
         else fail(AXS_ERR_ARG, "spectrum binning with %d bins does not fit shared memory", nbins);
     }
     // k_bin_runs' layout: histograms (hr rows), table, staged rows. All four rows of
-    // a 3D group at once while four blocks fit an SM, else two (2D groups have two).
+    // a 3D group at once while enough blocks fit an SM, else two (2D groups have two):
+    // 720^3 FP32, the reference's bins 472 us with four rows and three blocks, 565
+    // with two rows and seven; logarithmic bins 511 and 398.
     auto smem_of = [&](int hr, int rb) {
         return (size_t)(4 * hr * nbp + B::kSmemTable * nbins) * sizeof(double) + (size_t)4 * rb * seg * sizeof(float2);
     };
-    const int rb = L->esz == 8 ? 1 : (L->p.NDIMS == 3 && smem_of(1, 4) <= cap / 4 && smem_of(3, 4) <= cap ? 4 : 2);
+    const int rb = L->esz == 8 ? 1 : (L->p.NDIMS == 3 && smem_of(1, 4) <= cap / (B::kSmemTable ? 4 : 3) && smem_of(3, 4) <= cap ? 4 : 2);
     const size_t sm = smem_of(ks ? 3 : 1, rb);
     // as many 4-warp blocks as the later calls' layout fits on the SMs (up to 16
     // per SM), in the first call too: the per-warp histograms leave this kernel
