@@ -386,8 +386,8 @@ def gpu_arm(args, dist):
     sites_all = dist.sum(main["sites"])
     value = sites_all * args.steps / (main["ms"] * 1e-3)
     launches = max(1, main["launches"])
-    # steps per launch: 3 or 2 for the multi-step kernels (an interval's last
-    # one or two steps run on their partners, each pass moving the same bytes)
+    # steps per launch: up to 4 for the multi-step kernels (an interval's last
+    # steps run in shorter passes, each pass moving the same bytes)
     steps_per_launch = args.steps / launches
     per_launch_ms = main["ms"] / launches
     achieved = BYTES_PER_SITE[args.precision] * main["sites"] / (per_launch_ms * 1e-3) / 1e9
@@ -395,7 +395,9 @@ def gpu_arm(args, dist):
     three_step = "three steps per pass" in main["desc"]
     traffic = None
     tfile = os.path.join(ROOT, "profiles", "k_zmarch_traffic.txt")
-    if three_step:
+    if "register-tile" in main["desc"]:
+        tkey = "zmarch_k_fp32_1024_per_launch_bytes:"
+    elif three_step:
         tkey = "zmarch_3step_fp32_1024_per_launch_bytes:"
     elif two_step:
         tkey = ("zmarch_2step_lean_fp32_1024_per_launch_bytes:" if "lean" in main["desc"] else
@@ -466,7 +468,7 @@ def gpu_arm(args, dist):
                                        if steps_per_launch > 1 else "one step per pass: equals frac_per_pass",
                      "traffic": traffic, "traffic_unit": "GB per launch (ncu dram read+write)",
                      "traffic_source": ("profiles/k_zmarch_traffic.txt: dram__bytes_read.sum + dram__bytes_write.sum "
-                                        "of this kernel in an ncu launch list of this bench command")
+                                        "of this kernel in an ncu launch list of this bench command (register tiles, one-step: 512^3, x8)")
                                        if traffic else None,
                      "algorithmic_gb_per_launch": BYTES_PER_SITE[args.precision] * main["sites"] / 1e9,
                      "peak_source": peak_note,
