@@ -2596,7 +2596,16 @@ __global__ void __launch_bounds__(256, (ZMarch<T, R>::MINB)) k_energies_zcol_r(c
     });
     double v[3];
     acc.sums(v, tau, dx, lam_eff);
-    grid_reduce<3>(v, partials, ticket, hout);
+    if constexpr (sizeof(T) == 4 && R == 3) {
+        // 6 KB of its own leave three blocks per SM, which is faster at radius 3:
+        // 1024^3 6.51 ms, with four 6.65
+        grid_reduce<3>(v, partials, ticket, hout);
+    } else {
+        // in the tiles' memory: 6 KB more per block come off the L1 that the tiles'
+        // overlapping rows hit (radius 4, 1024^3: 7.57 ms, so 7.28)
+        extern __shared__ __align__(16) unsigned char zsm[];
+        grid_reduce<3>(v, partials, ticket, hout, reinterpret_cast<double (*)[256]>(zsm));
+    }
 }
 
 template <typename T>

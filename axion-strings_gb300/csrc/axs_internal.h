@@ -680,10 +680,10 @@ __device__ __forceinline__ bool last_block(unsigned *ticket) {
 // values per lane, then a fixed shuffle tree, 13 FP64 instructions per quantity
 // (summing each quantity in each warp first takes 40 of the FP64 pipe's 16-cycle
 // slots). blockDim.x must be 256.
+// red: K x 256 doubles of shared memory.
 template <int K>
-__device__ __forceinline__ void block_reduce_store(double (&v)[K], double *out, int64_t row) {
-    __shared__ double red[K][256];
-    __syncthreads();   // a previous reduction's readers are done
+__device__ __forceinline__ void block_reduce_store(double (&v)[K], double *out, int64_t row, double (*red)[256]) {
+    __syncthreads();   // a previous use of red is over
 #pragma unroll
     for (int k = 0; k < K; ++k) red[k][threadIdx.x] = v[k];
     __syncthreads();
@@ -699,14 +699,16 @@ __device__ __forceinline__ void block_reduce_store(double (&v)[K], double *out, 
 }
 template <int K>
 __device__ __forceinline__ void block_reduce_store(double (&v)[K], double *out) {
-    block_reduce_store<K>(v, out, blockIdx.x);
+    __shared__ double red[K][256];
+    block_reduce_store<K>(v, out, blockIdx.x, red);
 }
 // The grid's sum of v: block partials, which the last block adds (thread t
 // those of blocks t, t + 256, ..., then the fixed tree) into hout, page-locked
 // host memory. The order is fixed, so the sums are deterministic.
 template <int K>
-__device__ __forceinline__ void grid_reduce(double (&v)[K], double *partials, unsigned *ticket, double *hout) {
-    block_reduce_store<K>(v, partials, blockIdx.y * gridDim.x + blockIdx.x);
+__device__ __forceinline__ void grid_reduce(double (&v)[K], double *partials, unsigned *ticket, double *hout,
+                                            double (*red)[256]) {
+    block_reduce_store<K>(v, partials, blockIdx.y * gridDim.x + blockIdx.x, red);
     if (!last_block(ticket)) return;
     const int n = gridDim.x * gridDim.y;
     double s[K];
@@ -715,7 +717,12 @@ __device__ __forceinline__ void grid_reduce(double (&v)[K], double *partials, un
     for (int b = threadIdx.x; b < n; b += 256)
 #pragma unroll
         for (int k = 0; k < K; ++k) s[k] += __ldcg(partials + (int64_t)b * K + k);
-    block_reduce_store<K>(s, hout, 0);
+    block_reduce_store<K>(s, hout, 0, red);
+}
+template <int K>
+__device__ __forceinline__ void grid_reduce(double (&v)[K], double *partials, unsigned *ticket, double *hout) {
+    __shared__ double red[K][256];
+    grid_reduce<K>(v, partials, ticket, hout, red);
 }
 
 }  // namespace axs
