@@ -2543,8 +2543,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_energies_zcol(c
     grid_reduce<3>(v, partials, ticket, hout);
 }
 
-// The same for 2D and every radius: one thread per site of 32 x 8 tiles, the
-// neighbours from L1/L2.
+// The same for FP64 2D lattices of every radius: one thread per site of 32 x 8
+// tiles, the neighbours from L1/L2.
 template <typename T, int R>
 __global__ void __launch_bounds__(256) k_energies_2d(const typename Cplx<T>::type *__restrict__ psi,
                                                      const typename Cplx<T>::type *__restrict__ pih,
@@ -2647,16 +2647,17 @@ static void energies_fd(Lattice *L, double lam, double *hout) {
         kern<<<g, 256, smem, L->stream>>>(f, q, part, clk, p.N, dt, idx2, la, t3, p.prs, p.form, L->fresh, L->tau, dx, lam,
                                           L->dticket, hout);
     };
-    if (p.NDIMS == 2) {
-        const dim3 g(std::min(((p.N + 31) / 32) * ((p.N + 7) / 8), num_sms() * 8));
-        switch (p.stencil_setting) {
-        case 0: go(k_energies_2d<T, 1>, g, 0); break;
-        case 1: go(k_energies_2d<T, 2>, g, 0); break;
-        case 2: go(k_energies_2d<T, 3>, g, 0); break;
-        default: go(k_energies_2d<T, 4>, g, 0); break;
+    if constexpr (sizeof(T) == 8)
+        if (p.NDIMS == 2) {
+            const dim3 g(std::min(((p.N + 31) / 32) * ((p.N + 7) / 8), num_sms() * 8));
+            switch (p.stencil_setting) {
+            case 0: go(k_energies_2d<T, 1>, g, 0); break;
+            case 1: go(k_energies_2d<T, 2>, g, 0); break;
+            case 2: go(k_energies_2d<T, 3>, g, 0); break;
+            default: go(k_energies_2d<T, 4>, g, 0); break;
+            }
+            return;
         }
-        return;
-    }
     switch (p.stencil_setting) {
     case 0: go(k_energies_zcol<T>, zcol_grid<T, 1>(p.N), 0); break;
     case 1: go(k_energies_zcol_r<T, 2>, zcol_grid<T, 2>(p.N), ZMarch<T, 2>::SMEM); break;
@@ -2703,10 +2704,13 @@ void energies(Lattice *L, double out[3]) {
     double lam = (double)L->p.lambda * (L->p.prs ? 1.0 : L->tau * L->tau);
     double dx = L->p.space_step;
     double *s = host_slot(L);
-    if (L->p.laplacian == 0) {
+    if (L->p.laplacian == 0 && (L->p.NDIMS == 3 || L->esz == 8)) {
         if (L->esz == 4) energies_fd<float>(L, lam, s);
         else energies_fd<double>(L, lam, s);
-    } else {   // the spectral Laplacian: pi_n through scratch
+    } else {
+        // The spectral Laplacian, and 2D FP32: pi_n through scratch. In one pass, with
+        // the factors applied to the sums, 2D FP32 energies move by 5e-8 (1/tau is
+        // rounded to float per site here); with this kernel's terms in it, by 1e-9.
         launch_sync_pi(L);
         const int g = reduce_grid(L->length), N = L->p.N;
         double *part = ensure_partials(L, g, 3);
