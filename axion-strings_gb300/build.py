@@ -43,7 +43,7 @@ def _stale(target, deps):
 
 def build(verbose=False, force=False):
     os.makedirs(BUILD, exist_ok=True)
-    headers = [os.path.join(CSRC, "axs_internal.h"), os.path.join(CSRC, "axs_tma.cuh"), os.path.join(ROOT, "include", "axs.h")]
+    headers = [os.path.join(CSRC, "axs_internal.h"), os.path.join(CSRC, "axs_tma.cuh"), os.path.join(CSRC, "axs_touch.h"), os.path.join(ROOT, "include", "axs.h")]
     jobs = []
     objs = []
     for src in CUDA_SOURCES:

@@ -10,14 +10,10 @@
 #include <vector>
 #include <algorithm>
 
-#include <atomic>
 #include <mutex>
-#include <system_error>
-#include <thread>
-
-#include <unistd.h>
 
 #include "axs_internal.h"
+#include "axs_touch.h"
 
 struct axs_lattice {
     axs::Lattice L;
@@ -181,52 +177,6 @@ static void *device_alias(const void *p) {
 // Chunked, double-buffered staging of pageable host arrays: copies run on a
 // second stream and overlap the (un)packing kernels on the lattice stream.
 static const int64_t kXferChunk = (int64_t)1 << 25;   // elements per chunk
-
-// First touch of a pageable destination, ahead of the copies into it. Copies
-// into pages that exist run at the link's rate (134 MB in 0.72 ms); into fresh
-// ones (a new numpy array) one thread takes the page faults inside the copy,
-// 5.6 ms. Up to six threads write one byte per page, chunk by chunk (every byte
-// is overwritten by the copy), so that the faults of the next chunks run beside
-// the copy of this one. Small destinations are left to the copy.
-class Touch {
-  public:
-    Touch(std::initializer_list<void *> dst, size_t bytes, size_t chunk_bytes) : dst_(dst), bytes_(bytes), chunk_(chunk_bytes) {
-        if (bytes * dst_.size() < ((size_t)8 << 20)) return;
-        const int n = (int)std::min<unsigned>(6, std::max(1u, std::thread::hardware_concurrency() / 2));
-        done_ = std::vector<std::atomic<int>>((bytes + chunk_ - 1) / chunk_);
-        try {
-            for (int t = 0; t < n; ++t) threads_.emplace_back([this, t, n] { work(t, n); });
-        } catch (const std::system_error &) {   // fewer threads than asked for: the copies take their share of the faults
-            stop_ = true;
-        }
-    }
-    ~Touch() {
-        stop_ = true;
-        for (std::thread &t : threads_) t.join();
-    }
-    Touch(const Touch &) = delete;
-    void wait(size_t c) {   // until chunk c's pages exist
-        if (done_.empty()) return;
-        while (!stop_ && done_[c] < (int)threads_.size()) std::this_thread::yield();
-    }
-
-  private:
-    void work(int t, int n) {
-        const size_t page = (size_t)std::max(4096l, sysconf(_SC_PAGESIZE));
-        for (size_t c = 0; c < done_.size() && !stop_; ++c) {
-            const size_t lo = c * chunk_, len = std::min(chunk_, bytes_ - lo), a = lo + len / n * t,
-                         b = t == n - 1 ? lo + len : lo + len / n * (t + 1);
-            for (void *d : dst_)
-                for (size_t o = a; o < b && !stop_; o = (o / page + 1) * page) ((volatile char *)d)[o] = 0;
-            ++done_[c];
-        }
-    }
-    std::vector<void *> dst_;
-    size_t bytes_, chunk_;
-    std::vector<std::atomic<int>> done_;
-    std::atomic<bool> stop_{false};
-    std::vector<std::thread> threads_;
-};
 
 struct Xfer {
     cudaStream_t copy = nullptr;
