@@ -268,7 +268,9 @@ static void download_pair(Lattice *L, const void *src, S *a, S *b) {
     const size_t cs = (size_t)2 * L->esz;
     const int64_t chunk = std::min(x.chunk, kFetchChunk);
     int64_t nch = (L->length + chunk - 1) / chunk;
-    Touch touch({a, b}, (size_t)L->length * sizeof(S), (size_t)chunk * sizeof(S));
+    // the host writes to pageable arrays only: the other array of the pair may be device memory
+    Touch touch({da ? nullptr : a, db ? nullptr : b}, (size_t)L->length * sizeof(S), (size_t)chunk * sizeof(S));
+    const cudaMemcpyKind ka = da ? cudaMemcpyDefault : cudaMemcpyDeviceToHost, kb = db ? cudaMemcpyDefault : cudaMemcpyDeviceToHost;
     for (int64_t c = 0; c < nch; ++c) {
         int s = (int)(c & 1);
         int64_t off = c * chunk, n = std::min(chunk, L->length - off);
@@ -279,8 +281,8 @@ static void download_pair(Lattice *L, const void *src, S *a, S *b) {
         AXS_CUDA(cudaEventRecord(x.copied[s], L->stream));
         AXS_CUDA(cudaStreamWaitEvent(x.copy, x.copied[s], 0));
         touch.wait((size_t)c);
-        AXS_CUDA(cudaMemcpyAsync(a + off, sa, (size_t)n * sizeof(S), cudaMemcpyDeviceToHost, x.copy));
-        AXS_CUDA(cudaMemcpyAsync(b + off, sb, (size_t)n * sizeof(S), cudaMemcpyDeviceToHost, x.copy));
+        AXS_CUDA(cudaMemcpyAsync(a + off, sa, (size_t)n * sizeof(S), ka, x.copy));
+        AXS_CUDA(cudaMemcpyAsync(b + off, sb, (size_t)n * sizeof(S), kb, x.copy));
         AXS_CUDA(cudaEventRecord(x.done[s], x.copy));
     }
     AXS_CUDA(cudaStreamSynchronize(x.copy));
@@ -338,7 +340,7 @@ static void download_fields(Lattice *L, S *f0, S *f1, S *f2, S *f3) {
             if (!dst[f]) continue;
             void *st = stage(L);
             launch_unpack(L, src, 0, f & 1, st, is_d);
-            Touch touch({dst[f]}, device_alias(dst[f]) ? 0 : (size_t)L->length * sizeof(S), (size_t)L->length * sizeof(S));
+            Touch touch({device_alias(dst[f]) ? nullptr : dst[f]}, (size_t)L->length * sizeof(S), (size_t)L->length * sizeof(S));
             touch.wait(0);
             AXS_CUDA(cudaMemcpyAsync(dst[f], st, (size_t)L->length * sizeof(S), cudaMemcpyDeviceToHost, L->stream));
             AXS_CUDA(cudaStreamSynchronize(L->stream));
@@ -662,7 +664,7 @@ int axs_checkpoint(axs_lattice *h, void *buf, size_t bytes) {
     memcpy(buf, &hd, sizeof hd);
     char *b = (char *)buf + sizeof hd;
     {
-        Touch touch({b}, device_alias(b) ? 0 : 2 * cb, 2 * cb);
+        Touch touch({device_alias(b) ? nullptr : b}, 2 * cb, 2 * cb);
         touch.wait(0);
     }
     AXS_CUDA(cudaMemcpyAsync(b, L->psi[L->cur], cb, cudaMemcpyDeviceToHost, L->stream));

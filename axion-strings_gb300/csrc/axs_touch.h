@@ -18,10 +18,12 @@ namespace axs {
 // ones (a new numpy array) one thread takes the page faults inside the copy,
 // 5.6 ms. Up to six threads write one byte per page, chunk by chunk (every byte
 // is overwritten by the copy), so that the faults of the next chunks run beside
-// the copy of this one. Small destinations are left to the copy.
+// the copy of this one. Small destinations are left to the copy, null ones skipped.
 class Touch {
   public:
-    Touch(std::initializer_list<void *> dst, size_t bytes, size_t chunk_bytes) : dst_(dst), bytes_(bytes), chunk_(chunk_bytes) {
+    Touch(std::initializer_list<void *> dst, size_t bytes, size_t chunk_bytes) : bytes_(bytes), chunk_(chunk_bytes) {
+        for (void *d : dst)
+            if (d) dst_.push_back(d);
         if (bytes * dst_.size() < ((size_t)8 << 20)) return;
         const int n = (int)std::min<unsigned>(6, std::max(1u, std::thread::hardware_concurrency() / 2));
         try {

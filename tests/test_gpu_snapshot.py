@@ -85,3 +85,31 @@ def test_large_pageable_downloads(axs, fields):
                 assert np.array_equal(a, b.array)
         for o in pins:
             o.free()
+
+
+@pytest.mark.parametrize("where", ["pinned", "device"])
+@pytest.mark.parametrize("first", [True, False])
+def test_pair_of_two_kinds_of_memory(axs, where, first):
+    """One array of a pair page-locked or on the device, the other pageable and large enough to be touched by host
+    threads: both get the values, and the host writes to the pageable one only."""
+    p = params(axs, nd=3, N=128, precision=64)
+    with axs.Lattice(p) as L:
+        L.init_flat(7, 1.0)
+        L.evolve(3)
+        want = L.download()
+        host = np.empty(L.shape)
+        assert host.nbytes >= 8 << 20
+        if where == "pinned":
+            other = axs.PinnedBuffer(L.shape, np.float64)
+            ptr, get = other.array.ctypes.data, lambda: other.array
+        else:
+            torch = pytest.importorskip("torch")
+            dev = torch.full(L.shape, -7.0, dtype=torch.float64, device="cuda")
+            torch.cuda.synchronize()
+            ptr, get = dev.data_ptr(), lambda: dev.cpu().numpy()
+        pair = (ptr, host.ctypes.data) if first else (host.ctypes.data, ptr)
+        axs._check(axs._lib.axs_download(L._h, None, None, *pair))
+        a, b = (get(), host) if first else (host, get())
+        assert np.array_equal(a, want[2]) and np.array_equal(b, want[3])
+        if where == "pinned":
+            other.free()
