@@ -251,7 +251,7 @@ static void upload_pair(Lattice *L, const S *a, const S *b, void *dst, bool drif
     }
 }
 
-static const int64_t kFetchChunk = (int64_t)1 << 22;   // elements per chunk of a download
+static const int64_t kFetchChunk = (int64_t)1 << 25;   // bytes per array and chunk of a download
 
 template <typename S>
 static void download_pair(Lattice *L, const void *src, S *a, S *b) {
@@ -266,23 +266,31 @@ static void download_pair(Lattice *L, const void *src, S *a, S *b) {
     AXS_CUDA(cudaEventRecord(x.entry, x.copy));
     AXS_CUDA(cudaStreamWaitEvent(L->stream, x.entry, 0));
     const size_t cs = (size_t)2 * L->esz;
-    const int64_t chunk = std::min(x.chunk, kFetchChunk);
+    const int64_t chunk = std::min(x.chunk, kFetchChunk / (int64_t)sizeof(S));
     int64_t nch = (L->length + chunk - 1) / chunk;
     // the host writes to pageable arrays only: the other array of the pair may be device memory
     Touch touch({da ? nullptr : a, db ? nullptr : b}, (size_t)L->length * sizeof(S), (size_t)chunk * sizeof(S));
     const cudaMemcpyKind ka = da ? cudaMemcpyDefault : cudaMemcpyDeviceToHost, kb = db ? cudaMemcpyDefault : cudaMemcpyDeviceToHost;
-    for (int64_t c = 0; c < nch; ++c) {
-        int s = (int)(c & 1);
-        int64_t off = c * chunk, n = std::min(chunk, L->length - off);
-        char *sa = x.buf + (size_t)(2 * s) * x.chunk * sizeof(double);
-        char *sb = sa + (size_t)x.chunk * sizeof(double);
+    // A copy into a pageable array holds the host until it is done, so a chunk is
+    // unpacked before the copies of the one before are asked for (four chunks
+    // in turn took 7 % longer than one).
+    auto slot = [&](int64_t c) { return x.buf + (size_t)(2 * (c & 1)) * x.chunk * sizeof(double); };
+    auto unpack = [&](int64_t c) {
+        const int s = (int)(c & 1);
         if (c >= 2) AXS_CUDA(cudaStreamWaitEvent(L->stream, x.done[s], 0));
-        launch_unpack2(L, (const char *)src + (size_t)off * cs, sa, sb, is_d, n, L->stream);
+        launch_unpack2(L, (const char *)src + (size_t)(c * chunk) * cs, slot(c), slot(c) + (size_t)x.chunk * sizeof(double),
+                       is_d, std::min(chunk, L->length - c * chunk), L->stream);
         AXS_CUDA(cudaEventRecord(x.copied[s], L->stream));
+    };
+    unpack(0);
+    for (int64_t c = 0; c < nch; ++c) {
+        const int s = (int)(c & 1);
+        const int64_t off = c * chunk, n = std::min(chunk, L->length - off);
         AXS_CUDA(cudaStreamWaitEvent(x.copy, x.copied[s], 0));
+        if (c + 1 < nch) unpack(c + 1);
         touch.wait((size_t)c);
-        AXS_CUDA(cudaMemcpyAsync(a + off, sa, (size_t)n * sizeof(S), ka, x.copy));
-        AXS_CUDA(cudaMemcpyAsync(b + off, sb, (size_t)n * sizeof(S), kb, x.copy));
+        AXS_CUDA(cudaMemcpyAsync(a + off, slot(c), (size_t)n * sizeof(S), ka, x.copy));
+        AXS_CUDA(cudaMemcpyAsync(b + off, slot(c) + (size_t)x.chunk * sizeof(double), (size_t)n * sizeof(S), kb, x.copy));
         AXS_CUDA(cudaEventRecord(x.done[s], x.copy));
     }
     AXS_CUDA(cudaStreamSynchronize(x.copy));

@@ -20,3 +20,7 @@ def run(tmp_path, name):
 
 def test_no_write_after_a_thread_could_not_be_created(tmp_path):
     run(tmp_path, "touch_threads")
+
+
+def test_only_missing_pages_are_touched(tmp_path):
+    run(tmp_path, "touch_resident")
