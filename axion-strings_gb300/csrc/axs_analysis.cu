@@ -2239,18 +2239,25 @@ __device__ __forceinline__ float abs_theta(float a, float b) { return fabsf(fast
 // of the library's FP64 cost (GB300's FP64 pipe bounds the FP64 means). The
 // float angle picks the nearest of the angles k pi/512 (k = -512 .. 512); the
 // vector (b, a) is rotated by -k pi/512 with that angle's double cosine and
-// sine (formed on the host) to (x, y), a small angle from the x axis. With
-// u = y/x (the reciprocal from the float one by one Newton-Raphson step, within
-// 2^-44: u is below 0.0031, so its error is below 2^-52.4, and of either sign),
-// the remainder angle
-// atan(u) is the Taylor series to u^5 (truncated below 4e-19) and |(a, b)| =
-// x sqrt(1 + u^2) the binomial series to u^4 (6e-17 of it at most). |theta| is
+// sine (formed on the host) to (x, y), a small angle from the x axis: |y/x| is
+// below kRotU (tan(pi/1024 + 9e-7), the float angle's error and the rounding of k). With
+// u = y/x (the float reciprocal i of x, its residual h = 1 - x i below 2^-22, and
+// 1/x = i (1 + h + h^2) up to h^3: rounding alone is left), the remainder angle
+// atan(u) is the Taylor series to u^5 and |(a, b)| = x sqrt(1 + u^2) the binomial
+// series to u^4, with the next term of each (up to 1.2e-16 and 5e-17 of the result)
+// economised into the two before it: t^3 for t = u^2 in [0, T] is replaced by its
+// interpolation at 0 and the other two roots of the Chebyshev polynomial so placed,
+// within T^3/25. |theta| is
 // the table's |k| pi/512 plus atan(u) with k's sign: for k = +-512 the angle
-// past pi counts back from it, |theta| = pi - |atan(u)|. Signs are set in the
+// past pi counts back from it, |theta| = pi - |atan(u)|; for k = 0 it is atan(u) alone, within 2 ulp
+// of itself. Signs are set in the
 // high words, ranges and conversions read from the bits (no FP64 instructions):
-// 13 FP64 operations. Vectors outside that (a zero, tiny, huge or non-finite
+// 16 FP64 operations. Vectors outside that (a zero, tiny, huge or non-finite
 // component) take the library's atan2 and square root.
 static constexpr int kRot = 512;
+static constexpr double kRotU = 0.00307, kRotT = kRotU * kRotU;
+// t^3 ~ kRotA t^2 - kRotB t
+static constexpr double kRotA = 1.3923048454132638 * kRotT, kRotB = 0.430780618346945 * kRotT * kRotT;
 struct ThetaRot {
     double c, s, angle, pad;   // cosine and sine of k pi/512, |k| pi/512
 };
@@ -2268,16 +2275,17 @@ __device__ __forceinline__ void abs_phi_theta(double a, double b, double &aphi, 
         const ThetaRot &r = g_theta_rot[k + kRot];
         const double x = fma(b, r.c, a * r.s), y = fma(a, r.c, -(b * r.s));   // x > 0: within a step of the axis
         double i = double_bits(__frcp_rn(float_bits(x)));
-        i = fma(i, fma(-x, i, 1.0), i);
+        const double h = fma(-x, i, 1.0);
+        i = fma(i, fma(h, h, h), i);
         const double u = y * i, u2 = u * u;
-        double q = fma(u2, 1.0 / 5.0, -1.0 / 3.0);
+        double q = fma(u2, 1.0 / 5.0 - kRotA / 7.0, -1.0 / 3.0 + kRotB / 7.0);
         const double t = fma(u * u2, q, u);   // atan(u)
         // + t for k > 0, - t for k < 0, |t| for k = 0, -|t| for k = +-512
         unsigned hi = (unsigned)__double2hiint(t);
         if (k == 0 || k == kRot || k == -kRot) hi &= 0x7fffffffu;
         if (k < 0 || k == kRot) hi ^= 0x80000000u;
         ath = r.angle + __hiloint2double((int)hi, __double2loint(t));
-        q = fma(u2, -1.0 / 8.0, 0.5);
+        q = fma(u2, -1.0 / 8.0 + kRotA / 16.0, 0.5 - kRotB / 16.0);
         aphi = fma(x * u2, q, x);
         return;
     }

@@ -77,3 +77,20 @@ def test_background_angle_and_modulus_edge_cases(axs):
     ph = np.mean(np.sqrt(p1 * p1 + p2 * p2))
     assert abs(bg[4] - th) <= 1e-15 * th, (bg[4], th)
     assert abs(bg[5] - ph) <= 1e-15 * ph, (bg[5], ph)
+
+
+@pytest.mark.parametrize("b", [1.0 + 2.0 ** -23 * (1 - 2.0 ** -20), 1.5, 3.0 - 2.0 ** -22 * (1 - 2.0 ** -20), 1.9999999])
+@pytest.mark.parametrize("t", [3.0e-3, -1.0e-3, 7.0e-5, 1.0e-9])
+def test_background_small_angle_to_double_precision(axs, t, b):
+    """FP64 sites next to the positive phi2 axis: |theta| is the quotient's series alone, no table entry is added that
+    would cover a short reciprocal. Every site is the same, 64 of them, so the mean is the site's value: three roundings of
+    2^-53 for |theta|, one and a small part of one for |phi|."""
+    a = t * b
+    z = np.zeros((4, 4, 4))
+    with axs.Lattice(params(axs, 3, 4, 64)) as L:
+        L.upload(z + a, z + b, z, z)
+        bg = L.background()
+    la, lb = np.longdouble(a), np.longdouble(b)
+    th, ph = abs(np.arctan2(la, lb)), np.sqrt(la * la + lb * lb)
+    assert abs(bg[4] - th) <= 3.1 * 2.0 ** -53 * th, float((bg[4] - th) / th)
+    assert abs(bg[5] - ph) <= 1.1 * 2.0 ** -53 * ph, float((bg[5] - ph) / ph)
