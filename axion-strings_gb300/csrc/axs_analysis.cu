@@ -2291,7 +2291,10 @@ __device__ __forceinline__ void abs_phi_theta(double a, double b, double &aphi, 
     }
     abs_phi_theta_lib(a, b, aphi, ath);
 }
-// the rotation table of abs_phi_theta, once per device
+// the rotation table of abs_phi_theta, once per device. The copy runs on the
+// default stream, which the lattices' streams do not wait for, and from pageable memory it may
+// return before the table has reached the device: the wait orders every later
+// launch, of any stream and thread, behind it.
 static void ensure_theta_table() {
     static PerDevice done;
     done.get([] {
@@ -2301,6 +2304,7 @@ static void ensure_theta_table() {
             tab[k + kRot] = ThetaRot{cos(t), sin(t), fabs(t), 0.0};
         }
         AXS_CUDA(cudaMemcpyToSymbol(g_theta_rot, tab.data(), tab.size() * sizeof(ThetaRot)));
+        AXS_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
         return 1;
     });
 }

@@ -94,3 +94,34 @@ def test_background_small_angle_to_double_precision(axs, t, b):
     th, ph = abs(np.arctan2(la, lb)), np.sqrt(la * la + lb * lb)
     assert abs(bg[4] - th) <= 3.1 * 2.0 ** -53 * th, float((bg[4] - th) / th)
     assert abs(bg[5] - ph) <= 1.1 * 2.0 ** -53 * ph, float((bg[5] - ph) / ph)
+
+
+def test_first_fp64_background_of_a_process(axs):
+    """The call that brings the angle table to the device uses it on another stream at once: a new process's first call,
+    and one from a second thread started with it, give what later calls give."""
+    import subprocess
+    import sys
+    code = """
+import sys, threading
+sys.path[:0] = %r
+import numpy as np, axs
+rng = np.random.default_rng(0)
+N = 8
+f = [rng.standard_normal((N, N, N)) for _ in range(4)]
+lats = [axs.Lattice(axs.default_params(NDIMS=3, N=N, precision=axs.F64)) for _ in range(2)]
+for L in lats:
+    L.upload(*f)
+first = [None, None]
+def go(i):
+    first[i] = lats[i].background()
+ts = [threading.Thread(target=go, args=(i,)) for i in range(2)]
+[t.start() for t in ts]
+[t.join() for t in ts]
+again = lats[0].background()
+assert np.array_equal(first[0], again) and np.array_equal(first[1], again), (first, again)
+th = np.mean(np.abs(np.arctan2(f[0], f[1])))
+assert abs(again[4] - th) <= 1e-14, (again[4], th)
+""" % ([p for p in sys.path if p],)
+    for _ in range(3):
+        r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
+        assert r.returncode == 0, r.stderr
