@@ -394,16 +394,43 @@ __device__ __forceinline__ StepCoefs<T> make_coefs(double tau, double dt, double
 // place of the largest one before the one rounding (to nearest, ties away from
 // zero), where the chain of five FP64 additions rounds five times: against the
 // exact sum its largest error over random, smooth and wide-range terms is
-// about half the chain's. The result does not depend on the order of the
-// terms. Terms all tiny (E < 64: zeros, subnormals), huge or not finite take
-// the FP64 additions, out of line: inline, the compiler predicates them, and a
-// predicated-off FP64 instruction still takes its slot of the pipe. One 3D
+// about half the chain's. Where the terms cancel to below 2^-14 of 2^E that loss could
+// be a larger share of the sum than the chain's (0.7 - 0.7 + 1e-9 + ... is exact there), so
+// such a sum takes FP64 additions that carry their rounding errors along (Knuth's
+// two-sum, TAOCP vol. 2, 4.2.2): the error is below 2^-53 + 2^-42 of the sum, or 2^-100
+// of the largest term. Terms all tiny (E < 64: zeros, subnormals), huge or not finite take
+// plain FP64 additions. Both are out of line: inline, the compiler predicates them, and a
+// predicated-off FP64 instruction still takes its slot of the pipe. The result depends on
+// the order of the terms in those cases only. One 3D
 // site's kick and drift (two sums of six, nine other FP64 operations): 343
 // cycles per warp and SM with FP64 sums, 161 with these, the integer work under the
 // nine operations.
-__device__ __noinline__ static double sum4_fp64(double a, double b, double c, double d) { return (a + b) + (c + d); }
+__device__ __forceinline__ bool fixed_serves(unsigned E) { return E - 64u < 0x7f0u - 64u; }
+template <int K>
+__device__ __forceinline__ double sum_fp64(const double (&v)[K]) {
+    unsigned top = 0;
+#pragma unroll
+    for (int i = 0; i < K; ++i) top = max(top, (unsigned)__double2hiint(v[i]) & 0x7fffffffu);
+    if (fixed_serves(top >> 20)) {
+        double s = v[0], err = 0.0;
+#pragma unroll
+        for (int i = 1; i < K; ++i) {
+            const double t = s + v[i], w = t - s;
+            err += (s - (t - w)) + (v[i] - w);
+            s = t;
+        }
+        return s + err;
+    }
+    if constexpr (K == 4) return (v[0] + v[1]) + (v[2] + v[3]);
+    else return ((v[0] + v[1]) + (v[2] + v[3])) + (v[4] + v[5]);
+}
+__device__ __noinline__ static double sum4_fp64(double a, double b, double c, double d) {
+    const double v[4] = {a, b, c, d};
+    return sum_fp64<4>(v);
+}
 __device__ __noinline__ static double sum6_fp64(double a, double b, double c, double d, double e, double f) {
-    return ((a + b) + (c + d)) + (e + f);
+    const double v[6] = {a, b, c, d, e, f};
+    return sum_fp64<6>(v);
 }
 template <int K>
 __device__ __forceinline__ double sum_fixed(const double (&v)[K]) {
@@ -415,10 +442,6 @@ __device__ __forceinline__ double sum_fixed(const double (&v)[K]) {
         top = max(top, m[i]);
     }
     const unsigned E = top >> 20;
-    if (E - 64u >= 0x7f0u - 64u) {
-        if constexpr (K == 4) return sum4_fp64(v[0], v[1], v[2], v[3]);
-        else return sum6_fp64(v[0], v[1], v[2], v[3], v[4], v[5]);
-    }
     top |= 0xfffffu;   // (top - m) >> 20 is then the difference of the exponents
     uint64_t s = 0;
 #pragma unroll
@@ -433,7 +456,10 @@ __device__ __forceinline__ double sum_fixed(const double (&v)[K]) {
     // s 2^(E - 1023 - 59): magnitude, leading bit to bit 63, 53 bits kept, the next one rounds
     const int sg = (int)(s >> 32) >> 31;
     const uint64_t a = (s ^ (uint64_t)(int64_t)sg) - (uint64_t)(int64_t)sg;
-    if (a == 0) return 0.0;
+    if (!fixed_serves(E) || (unsigned)(a >> 32) < 1u << 13) {   // a below 2^45: 2^-14 of 2^E
+        if constexpr (K == 4) return sum4_fp64(v[0], v[1], v[2], v[3]);
+        else return sum6_fp64(v[0], v[1], v[2], v[3], v[4], v[5]);
+    }
     const int lz = __clzll((long long)a);
     const uint64_t t = a << lz;
     const uint64_t b = ((uint64_t)(unsigned)((int)E + 3 - lz) << 52) + (t >> 11) + ((t >> 10) & 1);

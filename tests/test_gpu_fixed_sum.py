@@ -61,3 +61,28 @@ def test_fixed_point_sum(axs, kind, nd, N):
         assert abs(Fraction(float(got[at])) - want) <= (err + 2.0 ** -53 * abs(float(want))) * (1 + 2.0 ** -40) + 2.0 ** -1074, (at, v)
     if kind == "integers":
         assert np.array_equal(got, nb.sum(-1) - 2 * nd * f)   # exact sums stay exact
+
+
+@pytest.mark.parametrize("nd,N", [(2, 12), (3, 8)])
+@pytest.mark.parametrize("depth", [8, 13, 28, 60, 200])   # the small terms' exponents below the cancelling ones'
+def test_fixed_point_sum_of_cancelling_terms(axs, depth, nd, N):
+    """Every second site is 0 and its neighbours are +-0.7 or far smaller, so the large ones often cancel exactly. The sum
+    keeps its own relative accuracy: below 2^-14 of the largest term's power of two by rounding alone (or 2^-100 of that
+    term), above it within the alignment's loss."""
+    rng = np.random.default_rng(depth)
+    odd = np.indices((N,) * nd).sum(0) % 2 == 1
+    big = 0.7 * rng.choice([-1.0, 1.0], (N,) * nd)
+    f = np.where(odd, np.where(rng.random((N,) * nd) < 0.5, big, np.ldexp(rng.uniform(-1.0, 1.0, (N,) * nd), -depth)), 0.0)
+    with axs.Lattice(params(axs, nd=nd, N=N, precision=64, space_step=1.0)) as L:
+        L.upload(f, np.zeros_like(f))
+        got = L.laplacian(axs.PHI1)
+    nb = np.stack([np.roll(f, s, d) for d in range(nd) for s in (1, -1)], -1)
+    cancelled = 0
+    for at in np.argwhere(~odd):
+        at = tuple(at)
+        v = [float(x) for x in nb[at]]
+        exact, top = sum(map(Fraction, v)), max(abs(x) for x in v)
+        cancelled += top == 0.7 and abs(exact) < 2.0 ** -16
+        loss = 2.0 ** -100 * top if abs(exact) < 2.0 ** -16 * top else len(v) * 2.0 ** -59 * top
+        assert abs(Fraction(float(got[at])) - exact) <= 2.0 ** -53 * abs(exact) * (1 + 2.0 ** -40) + loss, (at, v)
+    assert cancelled > 3 or depth < 28
