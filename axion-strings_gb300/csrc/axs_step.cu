@@ -2026,7 +2026,7 @@ static int radius(const ZVariant &v) { return v.r > 0 ? v.r : 1; }
 
 std::string StepConfig::describe() const {
     char b[200];
-    if (kind == 0) snprintf(b, sizeof b, "generic kernel (3D: z-march by columns, 2D: steps per launch)");
+    if (kind == 0) snprintf(b, sizeof b, "generic kernel (3D: column march, 2D: several steps per launch)");
     else if (two_step(variant))
         snprintf(b, sizeof b, "TMA z-march variant %d (two steps per pass, halo depth 2%s; odd step on variant %d), tx=%d, zchunk=%d",
                  variant, kZVariants[variant].lean ? ", lean" : "", kZVariants[variant].partner, tx, zchunk);

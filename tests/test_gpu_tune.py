@@ -41,3 +41,20 @@ def test_tuning_skips_non_finite_state(axs):
     assert np.isposinf(g[2][5, 6, 7])
     for q in range(4):
         assert np.array_equal(g[q], f[q]), q
+
+
+def test_descriptions_tell_the_kernels_apart(axs):
+    """The description of the generic kernel does not pass for a z-march's (2D lattices, which have no other, and a 3D one
+    pinned to it), so what a tuned lattice says of itself means the kernel it runs."""
+    import os
+    with axs.Lattice(params(axs, 2, 64, 32)) as L:
+        L.autotune()
+        assert "generic" in L.describe() and "z-march" not in L.describe(), L.describe()
+    os.environ["AXS_FORCE_CONFIG"] = "0,0,64"
+    try:
+        with axs.Lattice(params(axs, 3, 48, 64)) as L:
+            L.init_flat(1, 1.0)
+            L.evolve(2)
+            assert "generic" in L.describe() and "z-march" not in L.describe(), L.describe()
+    finally:
+        del os.environ["AXS_FORCE_CONFIG"]
