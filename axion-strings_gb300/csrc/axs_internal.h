@@ -153,7 +153,8 @@ struct Lattice {
     ZLat *dzlat = nullptr;
     int zlat_variant = -1, zlat_tx = -1, zlat_zchunk = -1;
     void *zlat_pih[2] = {nullptr, nullptr};   // host copy of the table's pih[]
-    int debug_tx_excess = 0;  // set by axs_inject_wait_timeout for one step
+    int debug_tx_excess = 0;  // set by axs_inject_wait_timeout for one launch
+    StepConfig inject_cfg;    // the configuration to go back to after that launch
     int64_t zitems = 0;
     // analysis buffers (lazily allocated)
     uint8_t *dmask = nullptr;

@@ -2337,6 +2337,12 @@ static bool variant_resident(int esz, int variant) {
     }
 }
 
+// AXS_FORCE_CONFIG pins a configuration; it applies with AXS_AUTOTUNE=0 too.
+static bool forced_config() {
+    const char *f = getenv("AXS_FORCE_CONFIG");
+    return f && *f;
+}
+
 static int variant_smem(const ZVariant &v, int esz) {
     int cs = 2 * esz;
     if (v.gen == 4) {   // mirrors ZRCfg
@@ -2434,14 +2440,21 @@ static bool variant_fits(const ZVariant &v, const axs_params &p, int esz) {
     return radius(v) == p.stencil_setting + 1 && variant_tx(v, p.N, esz) > 0;
 }
 
-// For the injected wait timeout: a kernel with device-side waits (TMA) in place
-// of one without, false when none serves the lattice.
+// For the injected wait timeout: a kernel with device-side waits (TMA) for the
+// next launch in place of one without (the generic kernel where the tuner picked it, a
+// register tile), false when none serves the lattice or the generic kernel is pinned.
 bool use_waiting_kernel(Lattice *L) {
-    if (L->p.laplacian != 0 || L->cfg.kind != 1) return false;
-    if (!reg_tile(L->cfg.variant)) return true;
+    if (L->p.laplacian != 0 || L->p.NDIMS != 3) return false;
+    if (L->debug_tx_excess) return true;   // an injection is pending already
+    L->inject_cfg = L->cfg;
+    if (L->cfg.kind == 1 && !reg_tile(L->cfg.variant)) return true;
+    if (L->cfg.kind == 0 && forced_config()) return false;
     for (int v = 0; v < kNumZVariants; ++v)
-        if (!reg_tile(v) && variant_fits(kZVariants[v], L->p, L->esz)) {
+        if (!reg_tile(v) && variant_fits(kZVariants[v], L->p, L->esz) && variant_resident(L->esz, v)) {
+            L->cfg.kind = 1;
             L->cfg.variant = v;
+            L->cfg.zchunk = 32;
+            L->cfg.ctas_per_sm = 0;
             return true;
         }
     return false;
@@ -2747,6 +2760,7 @@ int lattice_advance(Lattice *L, int max_steps) {
         if (L->debug_tx_excess) {   // an injected stall lasts one launch: rebuild the table before the next
             L->debug_tx_excess = 0;
             L->zlat_variant = -1;
+            L->cfg = L->inject_cfg;
         }
     } else if (L->p.NDIMS == 2) {
         k = step2d_launch(L, max_steps);
@@ -2773,12 +2787,6 @@ void count_launches(int64_t n) {
     else __atomic_fetch_add(&g_launches, n, __ATOMIC_RELAXED);
 }
 int64_t total_launches() { return __atomic_load_n(&g_launches, __ATOMIC_RELAXED); }
-
-// AXS_FORCE_CONFIG pins a configuration; it applies with AXS_AUTOTUNE=0 too.
-static bool forced_config() {
-    const char *f = getenv("AXS_FORCE_CONFIG");
-    return f && *f;
-}
 
 static bool env_flag(const char *name, bool dflt) {
     const char *v = getenv(name);
@@ -2831,8 +2839,8 @@ void lattice_evolve(Lattice *L, int nsteps) {
         if (--nsteps == 0) return;
     }
     prepare_tables(L);
-    // a graph only where it saves launches: not for one or two
-    const bool few = nsteps < 2 || (L->p.NDIMS == 2 && L->p.laplacian == 0 && nsteps <= 2 * step2d_steps(L, nsteps));
+    // a graph only where it saves launches: not for one or two, nor for an interval whose first launch is to stall
+    const bool few = nsteps < 2 || L->debug_tx_excess || (L->p.NDIMS == 2 && L->p.laplacian == 0 && nsteps <= 2 * step2d_steps(L, nsteps));
     if (few || !env_flag("AXS_GRAPHS", true) || L->p.laplacian == 1) {   // spectral: transforms run eagerly
         while (nsteps > 0) nsteps -= lattice_advance(L, nsteps);
         return;
@@ -2915,6 +2923,11 @@ static double time_launches(cudaStream_t st, int reps, const std::function<void(
 // at every z-chunk (32 to 256 planes) at full length, and the time per step
 // decides.
 void lattice_autotune(Lattice *L) {
+    if (L->debug_tx_excess) {   // an injected stall that no step has taken yet is withdrawn: it is not for trials
+        L->debug_tx_excess = 0;
+        L->zlat_variant = -1;
+        L->cfg = L->inject_cfg;
+    }
     L->tuned = true;
     if (L->fresh == 2) L->fresh = 1;   // the trials overwrite the drift formed at upload
     // AXS_FORCE_CONFIG="kind,variant,zchunk" pins a configuration (tests use it

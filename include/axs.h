@@ -277,8 +277,10 @@ int axs_autotune(axs_lattice *h);
  * kernel records the timeout, drains its own copies and returns, and the next
  * synchronising call (axs_evolve_timed, axs_download, ...) returns
  * AXS_ERR_TIMEOUT. The CUDA context stays usable; the lattice's state after
- * that step is undefined. Requires the TMA step kernel (AXS_ERR_STATE
- * otherwise). */
+ * that step is undefined. Where the lattice's own step kernel has no such waits
+ * (the generic kernel where the tuner picked it, a register tile), that launch runs a TMA
+ * kernel instead; AXS_ERR_STATE where none serves the lattice (2D, the spectral
+ * Laplacian, a pinned generic kernel). */
 int axs_inject_wait_timeout(axs_lattice *h);
 /* Describe the step kernel configuration in use (for logs and benches). */
 int axs_describe(axs_lattice *h, char *buf, size_t len);

@@ -48,3 +48,31 @@ def test_injection_needs_the_tma_kernel(axs):
             assert e.value.code == axs.ERR_STATE
     finally:
         del os.environ["AXS_FORCE_CONFIG"]
+
+
+@pytest.mark.parametrize("N,precision,steps", [(64, 64, 1), (64, 32, 1), (96, 32, 1), (64, 64, 5)])
+def test_injection_on_tuned_lattices(axs, oracle, N, precision, steps):
+    """Whatever kernel the tuner picked (FP64 and small FP32 lattices take the generic one, others a register tile, neither
+    of which waits): the stall lasts one launch, and the lattice goes back to its own configuration."""
+    p = params(axs, 3, N, precision)
+    f = oracle.init_thermal(orc(p), 4)
+    with axs.Lattice(p) as L:
+        L.upload(*f)
+        L.evolve(2)
+        d = L.describe()
+        L.inject_wait_timeout()
+        with pytest.raises(axs.AxsError) as e:
+            L.evolve_timed(steps)
+        assert e.value.code == axs.ERR_TIMEOUT
+        assert L.describe() == d
+        L.set_time(1.0)
+        L.upload(*f)
+        L.evolve(6)   # a graph again, of the lattice's own kernel
+        g = L.download()
+        L.inject_wait_timeout()
+        L.autotune()   # withdraws it
+        assert L.describe() == d
+        L.evolve_timed(1)
+    o = oracle.evolve(orc(p), *f, 6)
+    for q in range(4):
+        assert rel(g[q], o[q]) <= (1e-12 if precision == 64 else 1e-5)
