@@ -2062,6 +2062,7 @@ static AxionPending axion_spectrum_enqueue(Lattice *L, int nbins, double *host, 
     AxionPending pd;
     pd.thr.assign(nbins, 0);
     for (int b = 1; b < nbins; ++b) { double t = exp(log(ratio) * (double)b / (double)nbins); pd.thr[b] = (int)ceil(t * t); }
+    if (L->tmp_cap[1] < nbins * sizeof(int)) L->thr_on_device.clear();   // they go with the old buffer, also if there is no new one
     int *de2 = (int *)lattice_tmp(L, 1, nbins * sizeof(int));
     if (L->thr_on_device != pd.thr) {   // the thresholds stay on the device while the binning is the same
         L->thr_on_device.clear();
@@ -2153,7 +2154,8 @@ static void ensemble_fan_out(Ensemble *E, Fn fn) {
             fn(L, i);
         } catch (...) {
             L->stream = own;
-            join();   // later work on the ensemble stays ordered after what did get enqueued
+            join();   // later work on the ensemble stays ordered after what did get enqueued ...
+            cudaStreamSynchronize(E->stream);   // ... and the next call may write the page-locked buffer
             throw;
         }
         L->stream = own;

@@ -135,3 +135,33 @@ def test_repeated_spectra_reuse_bin_geometry(axs, oracle, nd, N):
     ok = cso > 0
     assert rel(ps[ok], pso[ok]) <= 1e-11
     assert rel(ks[ok], kso[ok]) <= 1e-11
+
+
+@pytest.mark.parametrize("batched", [False, True])
+def test_axion_bins_changed_from_call_to_call(axs, batched):
+    """The bin thresholds stay on the device between calls with the same bins: calls with fewer, more (a larger buffer) and
+    the first number again give what a new lattice gives."""
+    p = params(axs, nd=3, N=24, precision=64)
+
+    def new(nbins):
+        with axs.Lattice(p) as L:
+            L.init_flat(3, 1.0)
+            L.evolve(2)
+            return L.axion_spectrum(nbins)
+
+    def check(call):
+        for nbins in (16, 5, 128, 16, 16, 700, 128, 5):
+            for a, b in zip(call(nbins), new(nbins)):
+                assert np.array_equal(np.asarray(a).reshape(-1)[:nbins], b)
+
+    if batched:
+        with axs.Ensemble([p, p]) as E:
+            for m in E.members:
+                m.init_flat(3, 1.0)
+            E.evolve(2)
+            check(E.axion_spectrum)
+    else:
+        with axs.Lattice(p) as L:
+            L.init_flat(3, 1.0)
+            L.evolve(2)
+            check(L.axion_spectrum)
