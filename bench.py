@@ -159,7 +159,7 @@ class Dist:
 CPU_KIND = ("oracle port of vvsl_field_rescaled in the reference's six passes, Laplacian as a sparse "
             "matrix-vector product over build_coefficient_matrix's matrix (CSR), float data_t, OpenMP")
 CPU_CALIBRATION = ("1.6-1.9x the reference's own FP64 step built from its sources with the project's SpMV shim "
-                   "(8-core x86, 256^3; profiles/cpu_baseline_calibration.md)")
+                   "(8-core x86, 256^3; calibration record in profiles/)")
 
 
 def cpu_port_rate(n=256, target_s=10.0, max_steps=200, min_steps=2):
@@ -376,6 +376,23 @@ def reference_arm(args, dist):
     print(json.dumps(line), flush=True)
 
 
+def captured_traffic(desc):
+    """The key in profiles/k_zmarch_traffic.txt of the 1024^3 FP32 radius-1 step kernel that `desc` describes, and where its
+    figure comes from; (None, None) for a kernel that was not captured."""
+    if "register-tile" in desc:   # one shape was: variant 58, three steps per pass
+        if "register-tile z-march variant 58 " not in desc:
+            return None, None
+        return "zmarch_k_fp32_1024_per_launch_bytes:", "8x a 512^3 capture of this kernel (three steps, z-chunks of 128 planes)"
+    if "three steps per pass" in desc:
+        return None, None
+    if "two steps per pass" in desc:
+        return ("zmarch_2step_lean_fp32_1024_per_launch_bytes:" if "lean" in desc else
+                "zmarch_2step_fp32_1024_per_launch_bytes:"), "an ncu launch list of this bench command"
+    if "z-march" in desc:
+        return "zmarch_fp32_1024_per_launch_bytes:", "8x a 512^3 capture of the one-step kernel"
+    return None, None
+
+
 def gpu_arm(args, dist):
     axs = load_axs()
     axs.set_device(dist.local)
@@ -391,20 +408,10 @@ def gpu_arm(args, dist):
     steps_per_launch = args.steps / launches
     per_launch_ms = main["ms"] / launches
     achieved = BYTES_PER_SITE[args.precision] * main["sites"] / (per_launch_ms * 1e-3) / 1e9
-    two_step = "two steps per pass" in main["desc"]
-    three_step = "three steps per pass" in main["desc"]
-    traffic = None
+    traffic = traffic_note = None
     tfile = os.path.join(ROOT, "profiles", "k_zmarch_traffic.txt")
-    if "register-tile" in main["desc"]:
-        tkey = "zmarch_k_fp32_1024_per_launch_bytes:"
-    elif three_step:
-        tkey = "zmarch_3step_fp32_1024_per_launch_bytes:"
-    elif two_step:
-        tkey = ("zmarch_2step_lean_fp32_1024_per_launch_bytes:" if "lean" in main["desc"] else
-                "zmarch_2step_fp32_1024_per_launch_bytes:")
-    else:
-        tkey = "zmarch_fp32_1024_per_launch_bytes:"
-    if args.precision == 32 and args.n == N_MAIN and args.stencil == 0 and os.path.exists(tfile):
+    tkey, traffic_note = captured_traffic(main["desc"])
+    if tkey and args.precision == 32 and args.n == N_MAIN and args.stencil == 0 and os.path.exists(tfile):
         for line in open(tfile):
             if line.startswith(tkey):
                 traffic = float(line.split(":", 1)[1]) / 1e9     # GB per launch, like `achieved`'s bytes
@@ -467,8 +474,8 @@ def gpu_arm(args, dist):
                                                                                steps_per_launch))
                                        if steps_per_launch > 1 else "one step per pass: equals frac_per_pass",
                      "traffic": traffic, "traffic_unit": "GB per launch (ncu dram read+write)",
-                     "traffic_source": ("profiles/k_zmarch_traffic.txt: dram__bytes_read.sum + dram__bytes_write.sum "
-                                        "of this kernel in an ncu launch list of this bench command (register tiles, one-step: 512^3, x8)")
+                     "traffic_source": ("profiles/k_zmarch_traffic.txt: dram__bytes_read.sum + dram__bytes_write.sum, "
+                                        + traffic_note)
                                        if traffic else None,
                      "algorithmic_gb_per_launch": BYTES_PER_SITE[args.precision] * main["sites"] / 1e9,
                      "peak_source": peak_note,

@@ -71,3 +71,19 @@ def test_reference_arm_prints_one_line_from_rank0():
     assert d["impl"] == "reference" and d["unit"] == "site-updates/s" and d["value"] > 0
     assert d["cpu_baseline"]["kind"] == "port" and d["cpu_baseline"]["cores"] >= 1
     assert d["e2e"]["h2d_bytes_per_step"] == 0 and d["e2e"]["d2h_bytes_per_step"] == 0
+
+
+def test_bench_traffic_belongs_to_the_kernel_that_ran():
+    """The bench's DRAM traffic is that of a captured kernel or absent: of the register tiles one shape was captured."""
+    import bench
+    have = {line.split(":")[0] for line in open(os.path.join(bench.ROOT, "profiles", "k_zmarch_traffic.txt")) if ":" in line}
+    tile = "register-tile z-march variant %d (up to %d steps per pass, %d warps), tx=56, zchunk=128"
+    key, note = bench.captured_traffic(tile % (58, 3, 12))
+    assert key.rstrip(":") in have and "512^3" in note
+    for other in (tile % (59, 4, 8), tile % (60, 4, 12), tile % (61, 3, 8), "generic kernel (3D: column march)",
+                  "TMA z-march variant 46 (three steps per pass, halo depth 3; last steps on variant 10), tx=64, zchunk=64"):
+        assert bench.captured_traffic(other) == (None, None), other
+    for d in ("TMA z-march variant 30 (two steps per pass, halo depth 2, lean; odd step on variant 16), tx=64, zchunk=32",
+              "TMA z-march variant 13 (two steps per pass, halo depth 2; odd step on variant 6), tx=64, zchunk=32",
+              "TMA z-march variant 7, tx=256, zchunk=64"):
+        assert bench.captured_traffic(d)[0].rstrip(":") in have, d
