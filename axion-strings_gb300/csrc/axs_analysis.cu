@@ -812,49 +812,23 @@ void string_positions(Lattice *L, int32_t *pos, int64_t cap, int64_t *n) {
 
 struct RefBins {     // pk_estimation.cpp:92-100: floor(|n|) - 1 for 0 < |n| < N/2
     int half;
-    __device__ __forceinline__ RefBins staged(double *) const { return *this; }
-    static constexpr int kSmemTable = 0;
     __device__ __forceinline__ int bin(int64_t n2) const {
         double kmag = sqrt((double)n2);
         if (kmag == 0.0 || kmag >= half) return -1;
         return (int)floor(kmag) - 1;
     }
 };
-struct LogBins {     // nbins log-spaced in |n| between 1 and sqrt(d) N/2
-    const double *edge2;   // edge2[b] = t_b^2, b = 1..nbins-1
-    int nbins;
-    // copy of the edge table in shared memory (s: nbins doubles)
-    __device__ __forceinline__ LogBins staged(double *s) const {
-        for (int i = threadIdx.x; i < nbins; i += blockDim.x) s[i] = edge2[i];
-        return LogBins{s, nbins};
-    }
-    static constexpr int kSmemTable = 1;
-    __device__ __forceinline__ int bin(int64_t n2) const {
-        if (n2 == 0) return -1;
-        double v = (double)n2;
-        int lo = 0, hi = nbins - 1;    // largest b with edge2[b] <= v (edge2[0] = 0)
-        while (lo < hi) {
-            int mid = (lo + hi + 1) >> 1;
-            if (edge2[mid] <= v) lo = mid; else hi = mid - 1;
-        }
-        return lo;
-    }
-};
-
-// ROWS = 2: per-bin counts by global integer atomics (the allocation-free
-// binner's layout); ROWS = 3: counts accumulated like the sums, as a third
-// per-warp row (exact: integer-valued doubles), one partial row each.
-template <typename T, typename B, int ROWS = 2>
+// Per-bin counts go by global integer atomics (the allocation-free binner's layout).
+template <typename T, typename B>
 __global__ void __launch_bounds__(128) k_bin(const typename Cplx<T>::type *__restrict__ F, int N, int ndims, B binner,
                                              int nbins, double *__restrict__ partials, unsigned long long *__restrict__ counts) {
-    extern __shared__ double hist[];   // [4 warps][ROWS][nbins], then the bin table if the binner has one
+    constexpr int ROWS = 2;
+    extern __shared__ double hist[];   // [4 warps][ROWS][nbins]
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < 4 * ROWS * nbins; i += blockDim.x) hist[i] = 0.0;
-    const B bins = binner.staged(hist + 4 * ROWS * nbins);
     __syncthreads();
     double *hp = hist + (size_t)w * ROWS * nbins;
     double *hk = hp + nbins;
-    double *hc = hk + nbins;   // ROWS == 3 only
     const int nh = N / 2 + 1;
     const int64_t rows = ndims == 2 ? (int64_t)N : (int64_t)N * N;
     const int64_t total = rows * nh;
@@ -877,7 +851,7 @@ __global__ void __launch_bounds__(128) k_bin(const typename Cplx<T>::type *__res
                 int64_t fz = iz < N / 2 ? iz : iz - N, fy = iy < N / 2 ? iy : iy - N;
                 n2 = fx * fx + fy * fy + fz * fz;
             }
-            b = bins.bin(n2);
+            b = binner.bin(n2);
             if (b >= 0) {
                 auto f = F[q];
                 wt = (ix == 0 || 2 * ix == N) ? 1.0 : 2.0;
@@ -903,8 +877,7 @@ __global__ void __launch_bounds__(128) k_bin(const typename Cplx<T>::type *__res
             if (lane == 0) {
                 hp[bl] += sv;
                 hk[bl] += sk;
-                if (ROWS == 3) hc[bl] += (double)sc;
-                else atomicAdd(&counts[bl], sc);
+                atomicAdd(&counts[bl], sc);
             }
             active &= ~same;
         }
@@ -2175,7 +2148,7 @@ void ensemble_release_pool(Ensemble *E) {
 
 void ensemble_find_strings(Ensemble *E, int64_t *nplaq, int64_t *ncores) {
     const size_t n = E->members.size();
-    if (E->members[0]->p.NDIMS == 2) {   // 2D: the neighbouring-pair count needs each member's list
+    if (E->members[0]->p.NDIMS == 2) {   // 2D: member by member, the pair count is a second kernel
         for (size_t i = 0; i < n; ++i) find_strings(E->members[i], nullptr, nullptr, &nplaq[i], &ncores[i]);
         return;
     }

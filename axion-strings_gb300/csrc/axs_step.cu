@@ -2716,7 +2716,8 @@ static int even_steps(int steps, int most) {
 }
 
 // Advances a lattice by one launch of at most max_steps (>= 1) steps and
-// returns the steps taken: two for a two-step variant when allowed, else one.
+// returns the steps taken: as many as the kernel takes per pass (two, three, up to four on
+// register tiles, up to twelve in 2D), evened out over the interval where it can; one for the others.
 // The handle's bookkeeping advances here; the kernels may run later inside a
 // graph.
 int lattice_advance(Lattice *L, int max_steps) {

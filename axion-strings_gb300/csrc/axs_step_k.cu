@@ -5,8 +5,8 @@
 // pih_{n+k-1}: 32 B per site for k site-updates. The two-step kernel
 // (k_zmarch_2step_lean) is at 0.89 of the HBM copy rate, so more steps per pass is what
 // is left; through shared-memory rings a third step made the pass issue-bound
-// (80 instructions per site-update, most of them shared-memory traffic). Here a
-// site-update takes about 20:
+// (80 instructions per site-update, most of them shared-memory traffic). Here it takes
+// 43 (three steps per pass on 12 warps of four rows), 32 per computed one:
 //  * a block takes a tile of tx x TY sites with a k-site halo (columns rounded
 //    up to pairs) through a z-chunk; lane i of warp w holds two neighbouring
 //    sites of V rows, the warps lie above one another. The x neighbours come by
@@ -29,9 +29,11 @@
 //
 // Measured (GB300, us per step; two steps per pass through shared memory in
 // brackets): 1024^3 2287 (2840), 512^3 313 (378), 256^3 47 (68), 128^3 9.9 (12.4).
-// At 512^3 the pass issues 47 % of the time with three warps per scheduler, 28
-// instructions per computed site and step, DRAM 45 %: the bound is the latency
-// between issues, and the halo (1.3 times the tile). Tried and slower at 1024^3:
+// (The 1024^3 figure is that of intervals of whole three-step passes; 20 steps are seven
+// passes that cost the same, 2410 per step.) At 512^3 with z-chunks of 128 planes (more
+// planes than the tuner's choice there) a three-step pass issues 47 % of the time with three
+// warps per scheduler, DRAM 54 %: the bound is the latency
+// between issues, and the halo (1.35 sites computed per site kept). Tried and slower at 1024^3:
 // rows chained through all steps with the planes in rotation (no register moves,
 // less parallelism), 2420; barriers between neighbouring warps only, 2470; 16 warps
 // of three rows (128 registers, spills), over 2490.
