@@ -1481,7 +1481,7 @@ __device__ __forceinline__ void tile_stencil(const typename Cplx<T>::type *t, co
     for (int l = 1; l <= R; ++l) {
         const auto xm = t[-l], xp = t[l], ym = t[-l * TW], yp = t[l * TW];
         const auto &zm = zr[(g + W - l) % W], &zp = zr[(g + l) % W];
-        const T s1 = nsum7<T>(xm.x, xp.x, ym.x, yp.x, zm.x, zp.x), s2 = nsum7<T>(xm.y, xp.y, ym.y, yp.y, zm.y, zp.y);
+        const T s1 = nsum7<T, true>(xm.x, xp.x, ym.x, yp.x, zm.x, zp.x), s2 = nsum7<T, true>(xm.y, xp.y, ym.y, yp.y, zm.y, zp.y);
         const T cl = (T)stencil_coef(R - 1, 3, l);
         a1 = fma(cl, s1, a1);
         a2 = fma(cl, s2, a2);

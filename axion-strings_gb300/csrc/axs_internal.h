@@ -433,9 +433,17 @@ __device__ __noinline__ static double sum6_fp64(double a, double b, double c, do
     const double v[6] = {a, b, c, d, e, f};
     return sum_fp64<6>(v);
 }
-template <int K>
+// LATE: the two tests that lead out of line are one, after the alignment: a branch less per
+// sum, but the terms are held longer. The 3D step of radius 1 takes 297 us at 256^3 with it and 288
+// without, so it is for the sums of radius 2 to 4: the radius-2 step 546 and 561, the energies of radius 3
+// 1455 and 1785.
+template <int K, bool LATE>
 __device__ __forceinline__ double sum_fixed(const double (&v)[K]) {
     static_assert(K == 4 || K == 6, "four or six neighbours: the sum stays below 2^63");
+    auto fp64 = [&] {
+        if constexpr (K == 4) return sum4_fp64(v[0], v[1], v[2], v[3]);
+        else return sum6_fp64(v[0], v[1], v[2], v[3], v[4], v[5]);
+    };
     unsigned m[K], top = 0;
 #pragma unroll
     for (int i = 0; i < K; ++i) {
@@ -443,6 +451,7 @@ __device__ __forceinline__ double sum_fixed(const double (&v)[K]) {
         top = max(top, m[i]);
     }
     const unsigned E = top >> 20;
+    if (!LATE && !fixed_serves(E)) return fp64();
     top |= 0xfffffu;   // (top - m) >> 20 is then the difference of the exponents
     uint64_t s = 0;
 #pragma unroll
@@ -457,20 +466,17 @@ __device__ __forceinline__ double sum_fixed(const double (&v)[K]) {
     // s 2^(E - 1023 - 59): magnitude, leading bit to bit 63, 53 bits kept, the next one rounds
     const int sg = (int)(s >> 32) >> 31;
     const uint64_t a = (s ^ (uint64_t)(int64_t)sg) - (uint64_t)(int64_t)sg;
-    if (!fixed_serves(E) || (unsigned)(a >> 32) < 1u << 13) {   // a below 2^45: 2^-14 of 2^E
-        if constexpr (K == 4) return sum4_fp64(v[0], v[1], v[2], v[3]);
-        else return sum6_fp64(v[0], v[1], v[2], v[3], v[4], v[5]);
-    }
+    if ((LATE && !fixed_serves(E)) || (unsigned)(a >> 32) < 1u << 13) return fp64();   // a below 2^45: 2^-14 of 2^E
     const int lz = __clzll((long long)a);
     const uint64_t t = a << lz;
     const uint64_t b = ((uint64_t)(unsigned)((int)E + 3 - lz) << 52) + (t >> 11) + ((t >> 10) & 1);
     return __longlong_as_double((long long)(b | ((uint64_t)(unsigned)sg << 63)));
 }
-template <typename T>
+template <typename T, bool LATE = false>
 __device__ __forceinline__ T nsum7(T xm, T xp, T ym, T yp, T zm, T zp) {
     if constexpr (sizeof(T) == 8) {
         const double v[6] = {xm, xp, ym, yp, zm, zp};
-        return sum_fixed<6>(v);
+        return sum_fixed<6, LATE>(v);
     } else {
         return ((xm + xp) + (ym + yp)) + (zm + zp);
     }
@@ -479,7 +485,7 @@ template <typename T>
 __device__ __forceinline__ T nsum5(T xm, T xp, T ym, T yp) {
     if constexpr (sizeof(T) == 8) {
         const double v[4] = {xm, xp, ym, yp};
-        return sum_fixed<4>(v);
+        return sum_fixed<4, false>(v);
     } else {
         return (xm + xp) + (ym + yp);
     }

@@ -181,8 +181,8 @@ __global__ void __launch_bounds__(256) k_step_generic(const typename Cplx<T>::ty
 #pragma unroll
             for (int l = 1; l <= R; ++l) {
                 const T w = (T)stencil_coef(R - 1, 3, l);
-                a1 = fma(w, nsum7<T>(xm[l - 1].x, xp[l - 1].x, ym[l - 1].x, yp[l - 1].x, zr[R - l].x, zr[R + l].x), a1);
-                a2 = fma(w, nsum7<T>(xm[l - 1].y, xp[l - 1].y, ym[l - 1].y, yp[l - 1].y, zr[R - l].y, zr[R + l].y), a2);
+                a1 = fma(w, nsum7<T, true>(xm[l - 1].x, xp[l - 1].x, ym[l - 1].x, yp[l - 1].x, zr[R - l].x, zr[R + l].x), a1);
+                a2 = fma(w, nsum7<T, true>(xm[l - 1].y, xp[l - 1].y, ym[l - 1].y, yp[l - 1].y, zr[R - l].y, zr[R + l].y), a2);
             }
             site_update<T>(ctr.x, ctr.y, a1, a2, p.x, p.y, o.x, o.y, c);
         }
