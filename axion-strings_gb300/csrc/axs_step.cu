@@ -102,22 +102,24 @@ __device__ __forceinline__ void stencil_at(const typename Cplx<T>::type *__restr
 }
 
 // One 3D step of any N and stencil radius: a thread per (x, y) column of a
-// z-chunk, blocks of 32 x 8 columns. psi's z-neighbours stay in registers, the
+// z-chunk, blocks of 32 x 8 columns (rows) or of 256 columns in a plane's order. psi's
+// z-neighbours stay in registers, the
 // in-plane neighbours come from L1/L2 (the neighbouring threads' loads), the
 // in-plane offsets are fixed for the column, and one thread forms the block's
 // time coefficients. FP64 steps are bound by the FP64 pipe (nine operations per
 // site at radius 1) with the neighbour sums' integer work under them, so this
-// kernel without barriers beats the TMA march there: 45 / 290 us per step at
+// kernel without barriers beats the TMA march there: 46 / 288 us per step at
 // 128^3 / 256^3 (37 / 298 at 18.5 cycles per operation and SM), where the march
 // takes 62 / 400 and one thread per site with 64-bit index divisions took 60 /
-// 371. FP32 lattices that lie in L2 take it too (64^3: 5.0 us per step where the
-// two-step march takes 6.5, 144^3: 19.3 and 20.6), beyond that where no tile fits.
+// 371. FP32 lattices that lie in L2 take it too (64^3: 4.2 us per step where the
+// two-step march takes 6.5, 144^3: 15.7 and 20.6), beyond that where no tile fits.
 template <typename T, int R>
 __global__ void __launch_bounds__(256) k_step_generic(const typename Cplx<T>::type *__restrict__ psi,
                                                       typename Cplx<T>::type *__restrict__ out,
                                                       typename Cplx<T>::type *__restrict__ pih,
                                                       const double *clock_in, double *clock_out, int N, double dt,
-                                                      double inv_dx2, double lambda, double T0sq3, int prs, int form) {
+                                                      double inv_dx2, double lambda, double T0sq3, int prs, int form,
+                                                      int rows) {
     typedef typename Cplx<T>::type C;
     __shared__ StepCoefs<T> sc;
     __shared__ T skctr;
@@ -127,8 +129,16 @@ __global__ void __launch_bounds__(256) k_step_generic(const typename Cplx<T>::ty
         skctr = sc.kdt_idx2 * (T)-6;
         if (blockIdx.x == 0 && blockIdx.y == 0) *clock_out = tau + dt;
     }
-    const int nbx = (N + 31) / 32;
-    const int x = (int)(blockIdx.x % nbx) * 32 + (threadIdx.x & 31), y = (int)(blockIdx.x / nbx) * 8 + (threadIdx.x >> 5);
+    int x, y;
+    if (rows) {
+        const int nbx = (N + 31) / 32;
+        x = (int)(blockIdx.x % nbx) * 32 + (threadIdx.x & 31);
+        y = (int)(blockIdx.x / nbx) * 8 + (threadIdx.x >> 5);
+    } else {   // past the plane: y >= N
+        const int q = (int)blockIdx.x * 256 + threadIdx.x;
+        y = q / N;
+        x = q - y * N;
+    }
     const int za = (int)((int64_t)blockIdx.y * N / gridDim.y), zb = (int)((int64_t)(blockIdx.y + 1) * N / gridDim.y);
     __syncthreads();
     if (x >= N || y >= N) return;
@@ -2618,17 +2628,24 @@ void step_release(Lattice *L) {
 }
 
 // About 16 blocks per SM (their work evens out over the SMs), in chunks of at
-// least 4 planes.
+// least 4 planes; lattices too small for that many blocks in shorter ones, where a chunk's planes,
+// each a trip to L2, are the step's time: FP64 at 22^3 4.0 us per step with one plane and 8.2
+// with four (radius 4: 5.7 and 16), at 56^3 7.3 with two, 8.4 with one, 8.9 with four; at 64^3
+// 10.9 with one and 9.1 with four. Blocks in a plane's order waste no lanes where 32 does not divide N
+// (FP64 50^3 7.5 against 8.2 us, 200^3 146 against 163); where it does, and for FP32 lattices of
+// radius 3 and 4 past 160^3 (250^3 radius 4: 214 against 197 us), 8 rows reuse more in L1.
 template <typename T, int R>
 static void launch_generic_t(Lattice *L, const double *cin, double *cout) {
     typedef typename Cplx<T>::type C;
     const axs_params &p = L->p;
     const double dx = p.space_step, T0 = p.T_initial;
-    const int cols = ((p.N + 31) / 32) * ((p.N + 7) / 8);
-    const dim3 grid(cols, std::max(1, std::min((16 * num_sms() + cols - 1) / cols, p.N / 4)));
+    const int rows = p.N % 32 == 0 || (sizeof(T) == 4 && R >= 3 && p.N > 160);
+    const int cols = rows ? ((p.N + 31) / 32) * ((p.N + 7) / 8) : (p.N * p.N + 255) / 256, sms = num_sms();
+    const int least = cols * p.N <= 4 * sms ? 1 : cols * p.N <= 6 * sms ? 2 : 4;
+    const dim3 grid(cols, std::max(1, std::min((16 * sms + cols - 1) / cols, p.N / least)));
     k_step_generic<T, R><<<grid, 256, 0, L->stream>>>(
         (const C *)L->psi[L->cur], (C *)L->psi[L->cur ^ 1], (C *)L->pih, cin, cout, p.N, (double)p.time_step,
-        1.0 / (dx * dx), (double)p.lambda, (T0 * T0) / 3.0, p.prs, p.form);
+        1.0 / (dx * dx), (double)p.lambda, (T0 * T0) / 3.0, p.prs, p.form, rows);
     AXS_CUDA(cudaGetLastError());
     count_launches(1);
 }
