@@ -1571,11 +1571,17 @@ __device__ __forceinline__ void zcol_march(const typename Cplx<T>::type *__restr
 // z-chunks as fill the resident blocks once (FP64, bound by its pipe, four times:
 // the work evens out over the SMs), none shorter than 8 planes (a
 // chunk stages A planes more than it has; lattices small enough to be cut that
-// far lie in L2). At 128^3 whole columns are 64 blocks for 152 SMs.
+// far lie in L2). At 128^3 whole columns are 64 blocks for 152 SMs. Where chunks of 8 leave
+// most SMs without a block, they are of 4 or 2 planes: FP64 radius 4, us per call, 22^3 pi_n and its
+// spectrum 111 with 8 planes, 90 with 4, 76 with 2 (86 with a thread per site), energies 78 / 51 / 29;
+// 64^3 energies 63 / 51 / 59. FP32, whose chunks are through sooner, at half the
+// blocks (64^3 radius 1: 21 / 25 / 33).
 template <typename T, int R>
 static dim3 zcol_grid(int N) {
     const int cols = ((N + 31) / 32) * ((N + 7) / 8), slots = num_sms() * ZMarch<T, R>::MINB;
-    return dim3(cols, std::max(1, std::min((sizeof(T) == 8 ? 4 * slots : slots) / cols, N / 8)));
+    const int few = (sizeof(T) == 8 ? 2 : 1) * num_sms();
+    const int least = cols * (N / 2) <= few / 2 ? 2 : cols * (N / 4) <= few ? 4 : 8;
+    return dim3(cols, std::max(1, std::min((sizeof(T) == 8 ? 4 * slots : slots) / cols, N / least)));
 }
 
 // One thread's coefficients for the block: GB300's FP64 pipe makes them cost
