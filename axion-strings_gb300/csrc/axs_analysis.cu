@@ -954,6 +954,8 @@ struct RefBinsI {
         const int m = half * half - c2;
         return m <= 0 ? 0 : (int)sqrtf((float)m) + 2;
     }
+    // the least n2 of bin b
+    __device__ __forceinline__ int least(int b) const { return (b + 1) * (b + 1); }
 };
 struct LogBinsI {
     const int *thr;   // thr[b] for b = 1..nbins-1 (thr[0] = 0)
@@ -986,6 +988,7 @@ struct LogBinsI {
         return 1;   // b < 0 only at the origin (n2 = 0)
     }
     __device__ __forceinline__ int limit(int) const { return INT_MAX; }
+    __device__ __forceinline__ int least(int b) const { return thr[b]; }
 };
 
 // Float-float values (hi + lo, about 48 significant bits): the warp-level sums
@@ -1142,7 +1145,10 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // Large spectra run in pieces that fit shared memory: a row of the half
 // spectrum is taken in segments of `seg` modes (each segment is binned like a
 // row: bins still only grow along it), and the bins in passes of `nbp`, this
-// launch summing bins b0 .. b0+nbp-1 only (modes of other bins are skipped).
+// launch summing bins b0 .. b0+nbp-1 only: it stages and takes the slices (below) that
+// hold modes of those bins, whole, so that the sums are those of all slices taken (2D FP64
+// 2712^2, four passes: power spectrum 2857 us with every mode staged in each, 2744 by
+// the bulk copies of single rows).
 // One segment per row and one pass is the common case.
 template <typename T, typename B, bool KS>
 __global__ void __launch_bounds__(128, 8) k_bin_runs(const typename Cplx<T>::type *__restrict__ F, int N, int ndims,
@@ -1187,7 +1193,11 @@ __global__ void __launch_bounds__(128, 8) k_bin_runs(const typename Cplx<T>::typ
         // slices at once are 2 * chunk words apart, which spreads them over the
         // 32 banks (an even chunk such as 16 put every lane on one bank).
         const int chunk = ((sl + 31) / 32) | 1;
-        const int lo = s0 + min(ll, lane * chunk), hi = s0 + min(ll, lane * chunk + chunk);
+        int la = 0, le = ll;   // the modes of the slices to take
+        if (b0 > 0) la = max(ceil_isqrt(bins.least(b0) - c2) - s0, 0) / chunk * chunk;
+        if (b1 < nbins) le = min(ll, (ceil_isqrt(bins.least(b1) - c2) - s0 + chunk - 1) / chunk * chunk);
+        if (la >= le) continue;
+        const int lo = s0 + min(max(lane * chunk, la), le), hi = s0 + min(max(lane * chunk + chunk, la), le);
         int fb = -1, lb = -1;   // the slice's first and last runs' bins, the same in every row of the group
         FF fv{0.f, 0.f}, fk{0.f, 0.f}, lv{0.f, 0.f}, lk{0.f, 0.f};
         int fc = 0, lc = 0;
@@ -1196,13 +1206,13 @@ __global__ void __launch_bounds__(128, 8) k_bin_runs(const typename Cplx<T>::typ
             if constexpr (kF32) {
                 for (int r = 0; r < rows; ++r) {
                     const C *src = row_of(m0 + r);
-                    for (int x = lane; x < ll; x += 32) cp_async_ca(smem_u32(stg + r * seg + x), src + x, 8);
+                    for (int x = la + lane; x < le; x += 32) cp_async_ca(smem_u32(stg + r * seg + x), src + x, 8);
                 }
                 cp_async_commit();
                 cp_async_wait<0>();
             } else {
                 const C *r0 = row_of(0), *r1 = row_of(min(1, cnt - 1)), *r2 = row_of(min(2, cnt - 1)), *r3 = row_of(cnt - 1);
-                for (int x = lane; x < ll; x += 32) {   // cnt is 1, 2 or 4
+                for (int x = la + lane; x < le; x += 32) {   // cnt is 1, 2 or 4
                     const C f0 = __ldcs(r0 + x);
                     C f1{0, 0}, f2{0, 0}, f3{0, 0};
                     if (cnt >= 2) f1 = __ldcs(r1 + x);

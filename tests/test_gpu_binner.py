@@ -38,3 +38,11 @@ def test_groups_of_rows(axs, oracle, nd, N, nbins, precision):
     ok = acnto > 0
     assert np.array_equal(acnt, acnto)
     assert rel(apk[ok], apko[ok]) <= (1e-10 if precision == 64 else 1e-4) and rel(k[ok], ko[ok]) <= 1e-11
+
+
+@pytest.mark.parametrize("nd,N,precision,nbins", [(2, 2600, 64, 700), (2, 2712, 64, 12), (2, 250, 32, 3000), (3, 34, 64, 2100),
+                                                  (3, 66, 32, 4000)])
+def test_bins_in_passes(axs, oracle, nd, N, precision, nbins):
+    """More bins than one pass holds (the reference's at 2600^2 and, with rows in segments, 2712^2; logarithmic ones from
+    about 2000): each pass takes only the slices that hold its modes."""
+    test_groups_of_rows(axs, oracle, nd, N, nbins, precision)
