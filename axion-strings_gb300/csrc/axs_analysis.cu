@@ -6,6 +6,7 @@
 #include <vector>
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "axs_internal.h"
 #include "axs_tma.cuh"
@@ -1149,8 +1150,8 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // hold modes of those bins, whole, so that the sums are those of all slices taken (2D FP64
 // 2712^2, four passes: power spectrum 2857 us with every mode staged in each, 2744 by
 // the bulk copies of single rows).
-// One segment per row and one pass is the common case.
-template <typename T, typename B, bool KS>
+// One segment per row and one pass (PASSES false) is the common case.
+template <typename T, typename B, bool KS, bool PASSES>
 __global__ void __launch_bounds__(128, 8) k_bin_runs(const typename Cplx<T>::type *__restrict__ F, int N, int ndims,
                                                      B binner, int nbins, int seg, int b0, int nbp, int rb,
                                                      double *__restrict__ partials) {
@@ -1194,9 +1195,9 @@ __global__ void __launch_bounds__(128, 8) k_bin_runs(const typename Cplx<T>::typ
         // 32 banks (an even chunk such as 16 put every lane on one bank).
         const int chunk = ((sl + 31) / 32) | 1;
         int la = 0, le = ll;   // the modes of the slices to take
-        if (b0 > 0) la = max(ceil_isqrt(bins.least(b0) - c2) - s0, 0) / chunk * chunk;
-        if (b1 < nbins) le = min(ll, (ceil_isqrt(bins.least(b1) - c2) - s0 + chunk - 1) / chunk * chunk);
-        if (la >= le) continue;
+        if (PASSES && b0 > 0) la = max(ceil_isqrt(bins.least(b0) - c2) - s0, 0) / chunk * chunk;
+        if (PASSES && b1 < nbins) le = min(ll, (ceil_isqrt(bins.least(b1) - c2) - s0 + chunk - 1) / chunk * chunk);
+        if (PASSES && la >= le) continue;
         const int lo = s0 + min(max(lane * chunk, la), le), hi = s0 + min(max(lane * chunk + chunk, la), le);
         int fb = -1, lb = -1;   // the slice's first and last runs' bins, the same in every row of the group
         FF fv{0.f, 0.f}, fk{0.f, 0.f}, lv{0.f, 0.f}, lk{0.f, 0.f};
@@ -1888,10 +1889,15 @@ static BinPending bin_spectrum_enqueue(Lattice *L, const B &binner, int kind, co
     };
     for (int b0 = 0; b0 < nbins; b0 += nbp) {
         const int nb = std::min(nbp, nbins - b0);
-        if (L->esz == 4) ks ? launch(k_bin_runs<float, B, true>, (const float2 *)L->fft_out, b0, nb)
-                            : launch(k_bin_runs<float, B, false>, (const float2 *)L->fft_out, b0, nb);
-        else ks ? launch(k_bin_runs<double, B, true>, (const double2 *)L->fft_out, b0, nb)
-                : launch(k_bin_runs<double, B, false>, (const double2 *)L->fft_out, b0, nb);
+        auto run = [&](auto passes) {
+            constexpr bool P = decltype(passes)::value;
+            if (L->esz == 4) ks ? launch(k_bin_runs<float, B, true, P>, (const float2 *)L->fft_out, b0, nb)
+                                : launch(k_bin_runs<float, B, false, P>, (const float2 *)L->fft_out, b0, nb);
+            else ks ? launch(k_bin_runs<double, B, true, P>, (const double2 *)L->fft_out, b0, nb)
+                    : launch(k_bin_runs<double, B, false, P>, (const double2 *)L->fft_out, b0, nb);
+        };
+        if (nbp < nbins) run(std::true_type());
+        else run(std::false_type());
         AXS_CUDA(cudaGetLastError());
         // rows (power, |n|, count) of this pass at host[3 b0 ..], which the kernel
         // writes itself when host is page-locked; otherwise the next pass
