@@ -58,6 +58,7 @@ def test_injection_on_tuned_lattices(axs, oracle, N, precision, steps):
     f = oracle.init_thermal(orc(p), 4)
     with axs.Lattice(p) as L:
         L.upload(*f)
+        L.autotune()   # also where the environment turns it off for the first step
         L.evolve(2)
         d = L.describe()
         L.inject_wait_timeout()
