@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3)
 // angles (turns) once per site through shared memory, as in k_cores3_tiled.
 // A thread per cell took four fast_atan2 and 64-bit divisions each. At small
 // sizes the launches and synchronisations bound the call: a search and its
-// list at 352^2 FP32 go from 112 to 73 us with this, k_pairs2 and the results in
+// list at 352^2 FP32 go from 112 to 49 us with this, k_pairs2 and the results in
 // page-locked memory.
 template <typename T>
 __global__ void __launch_bounds__(256) k_cores2_tiled(const typename Cplx<T>::type *__restrict__ psi,
