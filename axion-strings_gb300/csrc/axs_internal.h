@@ -49,6 +49,11 @@ struct StepConfig {
     int zchunk = 64;     // planes per work item
     int tx = 0;          // x tile (sites)
     int ctas_per_sm = 0; // persistent grid occupancy
+    // register tiles: a two-step variant for the passes of one (its partner) and two steps
+    // that it takes faster, -1: none; and the measured time of a pass of k steps, 0: not measured
+    int end_variant = -1, end_zchunk = 0;
+    bool end_pass[3] = {false, false, false};
+    float pass_ms[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
     std::string describe() const;
 };
 
@@ -150,12 +155,12 @@ struct Lattice {
     StepConfig cfg;
     bool tuned = false;
     // z-march launch table for this lattice alone
-    ZLat *dzlat = nullptr;
-    int zlat_variant = -1, zlat_tx = -1, zlat_zchunk = -1;
+    ZLat *dzlat = nullptr;   // [2]: the variant's entry, the end variant's
+    int zlat_variant = -1, zlat_tx = -1, zlat_zchunk = -1, zlat_end = -1, zlat_end_zchunk = 0;
     void *zlat_pih[2] = {nullptr, nullptr};   // host copy of the table's pih[]
     int debug_tx_excess = 0;  // set by axs_inject_wait_timeout for one launch
     StepConfig inject_cfg;    // the configuration to go back to after that launch
-    int64_t zitems = 0;
+    int64_t zitems = 0, zitems_end = 0;
     // analysis buffers (lazily allocated)
     uint8_t *dmask = nullptr;
     int32_t *dchunk = nullptr;       // flagged cells per chunk of the mask, then their scan
@@ -206,8 +211,8 @@ struct Ensemble {
     cudaStream_t stream = nullptr;
     StepConfig cfg;
     bool tuned = false;
-    ZLat *dzlat = nullptr;
-    int64_t zitems = 0;
+    ZLat *dzlat = nullptr;   // [2][members], as the lattice's
+    int64_t zitems = 0, zitems_end = 0;
     int *dcounter = nullptr;
     int *derr = nullptr;
     // per member (in members order): its cur when the table was built, and the

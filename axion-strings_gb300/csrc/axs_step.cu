@@ -2043,9 +2043,13 @@ std::string StepConfig::describe() const {
     else if (three_step(variant))
         snprintf(b, sizeof b, "TMA z-march variant %d (three steps per pass, halo depth 3; last steps on variant %d), tx=%d, zchunk=%d",
                  variant, kZVariants[variant].partner, tx, zchunk);
-    else if (reg_tile(variant))
-        snprintf(b, sizeof b, "register-tile z-march variant %d (up to %d steps per pass, %d warps), tx=%d, zchunk=%d", variant,
-                 kZVariants[variant].slots, kZVariants[variant].ncw, tx, zchunk);
+    else if (reg_tile(variant)) {
+        char e[64] = "";
+        if (end_pass[1] || end_pass[2])
+            snprintf(e, sizeof e, "; %s on variant %d", end_pass[1] && end_pass[2] ? "1 and 2" : end_pass[1] ? "1" : "2", end_variant);
+        snprintf(b, sizeof b, "register-tile z-march variant %d (up to %d steps per pass, %d warps%s), tx=%d, zchunk=%d", variant,
+                 kZVariants[variant].slots, kZVariants[variant].ncw, e, tx, zchunk);
+    }
     else if (variant >= 0 && variant < kNumZVariants && kZVariants[variant].gen == 4)
         snprintf(b, sizeof b, "TMA z-march variant %d (stencil radius %d), tx=%d, zchunk=%d", variant,
                  kZVariants[variant].r, tx, zchunk);
@@ -2461,10 +2465,10 @@ bool use_waiting_kernel(Lattice *L) {
     if (L->cfg.kind == 0 && forced_config()) return false;
     for (int v = 0; v < kNumZVariants; ++v)
         if (!reg_tile(v) && variant_fits(kZVariants[v], L->p, L->esz) && variant_resident(L->esz, v)) {
+            L->cfg = StepConfig();
             L->cfg.kind = 1;
             L->cfg.variant = v;
             L->cfg.zchunk = 32;
-            L->cfg.ctas_per_sm = 0;
             return true;
         }
     return false;
@@ -2579,21 +2583,25 @@ static thread_local int64_t t_captured = 0;
 // The lattice's own table uses absolute parity: a launch passes L->cur.
 static void ensure_single_table(Lattice *L) {
     if (t_capturing) fail(AXS_ERR_STATE, "internal: z-march table rebuilt inside a graph capture");
-    ZLat z;
-    int64_t items = fill_zlat(z, L, L->cfg.variant, L->cfg.zchunk, 0, 0);
-    if (!L->dzlat) L->dzlat = (ZLat *)dalloc(sizeof(ZLat));
-    AXS_CUDA(cudaMemcpyAsync(L->dzlat, &z, sizeof(ZLat), cudaMemcpyHostToDevice, L->stream));
+    ZLat z[2];
+    const int n = L->cfg.end_variant >= 0 ? 2 : 1;
+    L->zitems = fill_zlat(z[0], L, L->cfg.variant, L->cfg.zchunk, 0, 0);
+    if (n == 2) L->zitems_end = fill_zlat(z[1], L, L->cfg.end_variant, L->cfg.end_zchunk, 0, 0);
+    if (!L->dzlat) L->dzlat = (ZLat *)dalloc(2 * sizeof(ZLat));
+    AXS_CUDA(cudaMemcpyAsync(L->dzlat, z, n * sizeof(ZLat), cudaMemcpyHostToDevice, L->stream));
     AXS_CUDA(cudaStreamSynchronize(L->stream));
     L->zlat_variant = L->cfg.variant;
     L->zlat_zchunk = L->cfg.zchunk;
-    L->zlat_pih[0] = z.pih[0];
-    L->zlat_pih[1] = z.pih[1];
-    L->zitems = items;
-    L->cfg.tx = z.tx;
+    L->zlat_end = L->cfg.end_variant;
+    L->zlat_end_zchunk = L->cfg.end_zchunk;
+    L->zlat_pih[0] = z[0].pih[0];   // the end variant's are the same: both write the momentum out of place
+    L->zlat_pih[1] = z[0].pih[1];
+    L->cfg.tx = z[0].tx;
 }
 
 static bool single_table_valid(const Lattice *L) {
     if (!L->dzlat || L->zlat_variant != L->cfg.variant || L->zlat_zchunk != L->cfg.zchunk) return false;
+    if (L->zlat_end != L->cfg.end_variant || L->zlat_end_zchunk != L->cfg.end_zchunk) return false;
     if (L->zlat_pih[L->cur] != L->pih) return false;
     return out_of_place(L->cfg.variant, L) ? L->zlat_pih[L->cur ^ 1] == L->scratch : L->zlat_pih[L->cur ^ 1] == L->pih;
 }
@@ -2731,6 +2739,37 @@ static int even_steps(int steps, int most) {
     const int passes = (steps + most - 1) / most;
     return (steps + passes - 1) / passes;
 }
+// The steps of a register-tile configuration's next pass, `steps` before the end of the
+// interval: by the passes' measured times the fastest sequence, else evened out. A register-tile
+// pass takes about as long for two steps as for three (1024^3), and one and two steps go
+// faster through the shared-memory kernels from about 200^3 up: 512^3 FP32, us per
+// interval of 1 / 2 / 4 steps, all on register tiles 801 / 1007 / 1255, the
+// two-step kernel alone 674 / 749 / 1495.
+static int next_pass(const StepConfig &c, int steps) {
+    const int most = steps_per_pass(c.variant);
+    if (c.pass_ms[1] <= 0.f) return even_steps(steps, most);
+    constexpr int kEnd = 24;   // before that, the pass with the least time per step
+    if (steps > kEnd) {
+        int k = 1;
+        for (int i = 2; i <= most; ++i)
+            if (c.pass_ms[i] * k < c.pass_ms[k] * i) k = i;
+        return k;
+    }
+    float ms[kEnd + 1] = {0.f};
+    int first[kEnd + 1] = {0};
+    for (int n = 1; n <= steps; ++n)
+        for (int k = 1; k <= std::min(n, most); ++k)
+            if (k == 1 || c.pass_ms[k] + ms[n - k] < ms[n]) {
+                ms[n] = c.pass_ms[k] + ms[n - k];
+                first[n] = k;
+            }
+    return first[steps];
+}
+// The variant that takes a pass of k steps of a register-tile configuration, and whether it is the end variant's table.
+static int pass_variant(const StepConfig &c, int k, bool &end) {
+    end = k <= 2 && c.end_pass[k];
+    return !end ? c.variant : k == 2 ? c.end_variant : kZVariants[c.end_variant].partner;
+}
 
 // Advances a lattice by one launch of at most max_steps (>= 1) steps and
 // returns the steps taken: as many as the kernel takes per pass (two, three, up to four on
@@ -2773,8 +2812,13 @@ int lattice_advance(Lattice *L, int max_steps) {
             if (max_steps >= 2) k = 2;
             else kv = kZVariants[kv].partner;
         }
-        if (reg_tile(kv)) k = even_steps(max_steps, steps_per_pass(kv));
-        launch_zmarch(L->esz, kv, L->dzlat, 1, L->zitems, L->dcounter, L->cur, L->derr, L->stream, L->cfg.ctas_per_sm, k);
+        bool end = false;
+        if (reg_tile(kv)) {
+            k = next_pass(L->cfg, max_steps);
+            kv = pass_variant(L->cfg, k, end);
+        }
+        launch_zmarch(L->esz, kv, L->dzlat + end, 1, end ? L->zitems_end : L->zitems, L->dcounter, L->cur, L->derr, L->stream,
+                      L->cfg.ctas_per_sm, k);
         if (L->debug_tx_excess) {   // an injected stall lasts one launch: rebuild the table before the next
             L->debug_tx_excess = 0;
             L->zlat_variant = -1;
@@ -2928,6 +2972,20 @@ static double time_launches(cudaStream_t st, int reps, const std::function<void(
     return ms / reps;
 }
 
+// The passes' times of a register-tile configuration: launch(variant, end variant's
+// table, steps) runs one.
+static void measure_passes(StepConfig &c, cudaStream_t st, int nrep, const std::function<void(int, bool, int)> &launch) {
+    for (int k = 1; k <= steps_per_pass(c.variant); ++k) {
+        c.pass_ms[k] = (float)time_launches(st, nrep, [&] { launch(c.variant, false, k); }, 1);
+        if (k > 2 || c.end_variant < 0) continue;
+        const int kv = k == 2 ? c.end_variant : kZVariants[c.end_variant].partner;
+        const float ms = (float)time_launches(st, nrep, [&] { launch(kv, true, k); }, 1);
+        c.end_pass[k] = ms < c.pass_ms[k];
+        c.pass_ms[k] = std::min(c.pass_ms[k], ms);
+    }
+    if (!c.end_pass[1] && !c.end_pass[2]) c.end_variant = -1;
+}
+
 // Candidate steps run with dt = 0 on the lattice's own buffers:
 // psi_out = psi + 0*pih and pih + 0*K are bit-identical copies for finite
 // values (a -0.0 comes back as +0.0, which compares equal and gives the same
@@ -2939,7 +2997,8 @@ static double time_launches(cudaStream_t st, int reps, const std::function<void(
 // variants, and two-step variants with halo depth 2). Every variant is first
 // screened with one launch at one z-chunk; the three fastest are then timed
 // at every z-chunk (32 to 256 planes) at full length, and the time per step
-// decides.
+// decides; a register-tile kernel's passes are then timed step count by step count
+// (next_pass).
 void lattice_autotune(Lattice *L) {
     if (L->debug_tx_excess) {   // an injected stall that no step has taken yet is withdrawn: it is not for trials
         L->debug_tx_excess = 0;
@@ -3047,6 +3106,38 @@ void lattice_autotune(Lattice *L) {
             auto r = trial(screen[k].second, zc, reps, 2);
             if (r.second < best_ms) { best_ms = r.second; best = r.first; }
         }
+    if (best.kind == 1 && reg_tile(best.variant)) {
+        // passes of one and two steps: the fastest two-step variant of the screening and its
+        // partner, where they take them faster than the register tiles
+        const int nrep = L->length >= (1 << 27) ? 2 : L->length >= (1 << 24) ? 4 : 10;
+        StepConfig two;
+        double two_ms = 1e30;
+        for (const auto &s : screen)
+            if (two_step(s.second)) {
+                for (int zc : zchunks) {
+                    if (zc > L->p.N) continue;
+                    auto r = trial(s.second, zc, nrep, 1);
+                    if (r.second < two_ms) { two_ms = r.second; two = r.first; }
+                }
+                break;
+            }
+        if (two_ms < best_ms) {
+            best = two;
+        } else {
+            if (two.kind == 1) {
+                best.end_variant = two.variant;
+                best.end_zchunk = two.zchunk;
+            }
+            L->cfg = best;
+            ensure_single_table(L);
+            measure_passes(best, L->stream, nrep, [&](int kv, bool end, int k) {
+                launch_zmarch(L->esz, kv, L->dzlat + end, 1, end ? L->zitems_end : L->zitems, L->dcounter, L->cur, L->derr,
+                              L->stream, 0, k);
+                L->cur ^= 1;
+                std::swap(L->pih, L->scratch);
+            });
+        }
+    }
     L->p.time_step = dt_save;
     // dt = 0 steps copied psi (and, out of place, pih) back and forth; values
     // are identical, but keep the psi buffer the caller had as current.
@@ -3087,25 +3178,28 @@ static void ensemble_table(Ensemble *E, float dt_override, bool use_override) {
     std::vector<int> order(nm);
     for (size_t i = 0; i < nm; ++i) order[i] = (int)i;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return E->members[a]->length > E->members[b]->length; });
-    std::vector<ZLat> tab(nm);
+    const size_t nt = E->cfg.end_variant >= 0 ? 2 * nm : nm;
+    std::vector<ZLat> tab(nt);
     E->tab_cur.assign(nm, 0);
     E->tab_pih.assign(2 * nm, nullptr);
-    int64_t base = 0;
+    int64_t base = 0, base_end = 0;
     for (size_t k = 0; k < nm; ++k) {
         const int i = order[k];
         Lattice *m = E->members[i];
         float dt = m->p.time_step;
         if (use_override) m->p.time_step = dt_override;
         base += fill_zlat(tab[k], m, E->cfg.variant, E->cfg.zchunk, base, m->cur);
+        if (nt > nm) base_end += fill_zlat(tab[nm + k], m, E->cfg.end_variant, E->cfg.end_zchunk, base_end, m->cur);
         m->p.time_step = dt;
         E->tab_cur[i] = m->cur;
         E->tab_pih[2 * i] = tab[k].pih[0];
         E->tab_pih[2 * i + 1] = tab[k].pih[1];
     }
-    if (!E->dzlat) E->dzlat = (ZLat *)dalloc(sizeof(ZLat) * std::max<size_t>(1, nm));
-    AXS_CUDA(cudaMemcpyAsync(E->dzlat, tab.data(), sizeof(ZLat) * nm, cudaMemcpyHostToDevice, E->stream));
+    if (!E->dzlat) E->dzlat = (ZLat *)dalloc(sizeof(ZLat) * std::max<size_t>(1, 2 * nm));
+    AXS_CUDA(cudaMemcpyAsync(E->dzlat, tab.data(), sizeof(ZLat) * nt, cudaMemcpyHostToDevice, E->stream));
     AXS_CUDA(cudaStreamSynchronize(E->stream));
     E->zitems = base;
+    E->zitems_end = base_end;
 }
 
 void ensemble_setup(Ensemble *E) {
@@ -3163,9 +3257,14 @@ static int ensemble_advance(Ensemble *E, int max_steps) {
         if (max_steps >= 2) k = 2;
         else kv = kZVariants[kv].partner;
     }
-    if (reg_tile(kv)) k = even_steps(max_steps, steps_per_pass(kv));
-    launch_zmarch(E->members[0]->esz, kv, E->dzlat, (int)E->members.size(), E->zitems, E->dcounter, ensemble_parity(E),
-                  E->derr, E->stream, E->cfg.ctas_per_sm, k);
+    bool end = false;
+    if (reg_tile(kv)) {
+        k = next_pass(E->cfg, max_steps);
+        kv = pass_variant(E->cfg, k, end);
+    }
+    const int nm = (int)E->members.size();
+    launch_zmarch(E->members[0]->esz, kv, E->dzlat + (end ? nm : 0), nm, end ? E->zitems_end : E->zitems, E->dcounter,
+                  ensemble_parity(E), E->derr, E->stream, E->cfg.ctas_per_sm, k);
     for (Lattice *m : E->members) {
         m->cur ^= 1;
         if (out_of_place(E->cfg.variant, m)) std::swap(m->pih, m->scratch);
@@ -3187,6 +3286,7 @@ void ensemble_autotune(Ensemble *E) {
         int k = 0, v = 0, zc = 64;
         if (sscanf(force, "%d,%d,%d", &k, &v, &zc) >= 2 && k == 1 && v >= 0 && v < kNumZVariants &&
             ensemble_variant_ok(E, v)) {
+            E->cfg = StepConfig();
             E->cfg.kind = 1;
             E->cfg.variant = v;
             E->cfg.zchunk = zc > 0 ? zc : 64;
@@ -3236,6 +3336,36 @@ void ensemble_autotune(Ensemble *E) {
     best_ms = 1e30;
     for (size_t k = 0; k < screen.size() && k < 3; ++k)
         for (int zc : {32, 64, 128, 256}) trial(screen[k].second, zc, 6, 2);
+    if (reg_tile(best.variant)) {   // passes of one and two steps, as for a single lattice
+        StepConfig c = best;
+        double two_ms = 1e30;
+        for (const auto &s : screen)
+            if (two_step(s.second)) {
+                for (int zc : {32, 64, 128, 256}) {
+                    const double ms = trial(s.second, zc, 3, 1);
+                    if (ms < two_ms) {
+                        two_ms = ms;
+                        c.end_variant = s.second;
+                        c.end_zchunk = zc;
+                    }
+                }
+                break;
+            }
+        if (reg_tile(best.variant)) {   // not overtaken by one of those trials
+            E->cfg = c;
+            ensemble_table(E, 0.f, true);
+            const int nm = (int)E->members.size();
+            measure_passes(c, E->stream, 4, [&](int kv, bool end, int k) {
+                launch_zmarch(E->members[0]->esz, kv, E->dzlat + (end ? nm : 0), nm, end ? E->zitems_end : E->zitems, E->dcounter,
+                              ensemble_parity(E), E->derr, E->stream, 0, k);
+                for (Lattice *m : E->members) {
+                    m->cur ^= 1;
+                    std::swap(m->pih, m->scratch);
+                }
+            });
+            best = c;
+        }
+    }
     for (size_t i = 0; i < E->members.size(); ++i) {
         Lattice *m = E->members[i];
         if (m->cur != cur_save[i]) {
