@@ -3091,11 +3091,14 @@ void lattice_autotune(Lattice *L) {
     for (int zc : zchunks)
         if (zc <= L->p.N && zc <= 128) zc0 = zc;
     std::vector<std::pair<double, int>> screen;
+    // A launch over a large lattice needs no other before it. The three-step variants are pinned
+    // only: 1.7 times the two-step kernels' time.
+    const int warm = L->length >= (1 << 24) ? 0 : 1;
     if (zc0 > 0)
         for (int v = 0; v < kNumZVariants; ++v)
-            if (variant_fits(kZVariants[v], L->p, L->esz) && variant_resident(L->esz, v)) {
+            if (!three_step(v) && variant_fits(kZVariants[v], L->p, L->esz) && variant_resident(L->esz, v)) {
                 // register tiles take the whole SM: small lattices need short chunks
-                double ms = trial(v, zc0, 1, 1).second;
+                double ms = trial(v, zc0, 1, warm).second;
                 if (reg_tile(v) && L->p.N <= 512 && zc0 > 32) ms = std::min(ms, trial(v, 32, 1, 1).second);
                 screen.push_back({ms, v});
             }
