@@ -235,7 +235,9 @@ static constexpr int kRS = kCX + 4;                   // shared row stride: 16-b
 // FP32: four CTAs per SM (64 registers); the march is issue-bound, and 32
 // warps per SM ran 3.12 against 3.36 ms at 1024^3 for 24. FP64 holds twice
 // the prefetched field in registers: three CTAs.
-template <typename T, bool VEC>
+// LIST: flagged cells are counted per chunk as well (chunks); without, the counts'
+// registers do not spill the search (602^3 FP32 769 us with them, 730 without).
+template <typename T, bool VEC, bool LIST>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3)
     k_cores3_tiled(const typename Cplx<T>::type *__restrict__ psi, uint8_t *__restrict__ mask, int N, double accept,
                    unsigned long long *count, int32_t *__restrict__ chunks, unsigned *ticket, int64_t *hout) {
@@ -379,7 +381,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3)
             word &= vbytes;   // cells past the lattice's edge
             und &= vmask;
             local += __popc(word);
-            if (chunks && word) {
+            if (LIST && word) {
                 if (VEC) {
                     atomicAdd(&chunks[mo / kChunk], __popc(word));   // 4 divides mo and kChunk
                 } else {
@@ -424,7 +426,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3)
             if (cell3_exact<T, false>(cn, gx + j, gy, zz, N, accept)) {
                 const int64_t m = (int64_t)zz * NN + (int64_t)gy * N + gx + j;
                 mask[m] = 1;
-                if (chunks) atomicAdd(&chunks[m / kChunk], 1);
+                if (LIST) atomicAdd(&chunks[m / kChunk], 1);
                 ++local;
             }
         }
@@ -741,10 +743,9 @@ static void launch_cores(Lattice *L, double accept, int32_t *chunks, int64_t *ho
         k_cores2_tiled<T><<<grid, 256, 0, L->stream>>>(psi, L->dmask, N, accept, L->dtally);
     } else {
         const dim3 grid((N + kCX - 1) / kCX, (N + kCY - 1) / kCY, (N + kCZ - 1) / kCZ);
-        if ((N & 3) == 0)
-            k_cores3_tiled<T, true><<<grid, 256, 0, L->stream>>>(psi, L->dmask, N, accept, L->dtally, chunks, L->dticket, hout);
-        else
-            k_cores3_tiled<T, false><<<grid, 256, 0, L->stream>>>(psi, L->dmask, N, accept, L->dtally, chunks, L->dticket, hout);
+        auto go = [&](auto kern) { kern<<<grid, 256, 0, L->stream>>>(psi, L->dmask, N, accept, L->dtally, chunks, L->dticket, hout); };
+        if ((N & 3) == 0) chunks ? go(k_cores3_tiled<T, true, true>) : go(k_cores3_tiled<T, true, false>);
+        else chunks ? go(k_cores3_tiled<T, false, true>) : go(k_cores3_tiled<T, false, false>);
     }
     AXS_CUDA(cudaGetLastError());
     count_launches(1);
