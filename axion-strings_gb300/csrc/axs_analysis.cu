@@ -2628,13 +2628,27 @@ __global__ void __launch_bounds__(256, (ZMarch<T, R>::MINB)) k_energies_zcol_r(c
     }
 }
 
+// Reads psi and pih once, 16 bytes per load, one array after the other, with every block
+// of the grid resident: 512^3 FP32 303 us a call (7.1 TB/s), in two launches of 4-byte
+// loads 325, both arrays in one loop of such loads 341; FP64, whose comparisons took the FP64
+// pipe, 1115 -> 595.
 template <typename T>
-__global__ void __launch_bounds__(256) k_finite(const T *__restrict__ a, const T *__restrict__ b, int64_t n,
+__global__ void __launch_bounds__(256, 8) k_finite(const T *__restrict__ a, const T *__restrict__ b, int64_t n,
                                                 unsigned long long *bad_blocks, unsigned *ticket, int64_t *hout) {
-    int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t nv = n * (int)sizeof(T) / 16;   // 16-byte vectors: n = 2 N^d, N even
+    // Inf and NaN have the largest exponent: in every word of a float vector, in the odd words of a double one
+    auto word = [](unsigned w) {
+        const unsigned e = sizeof(T) == 4 ? 0x7f800000u : 0x7ff00000u;
+        return (w & e) == e;
+    };
+    auto vec = [&](const uint4 &v) { return sizeof(T) == 4 ? word(v.x) | word(v.y) | word(v.z) | word(v.w) : word(v.y) | word(v.w); };
     int bad = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-        bad |= !isfinite(a[i]) | !isfinite(b[i]);
+    for (const T *p : {a, b}) {
+        const uint4 *q = reinterpret_cast<const uint4 *>(p);
+#pragma unroll 4
+        for (int64_t i = i0; i < nv; i += stride) bad |= vec(q[i]);
+    }
     if (__syncthreads_or(bad) && threadIdx.x == 0) atomicAdd(bad_blocks, 1ull);
     if (last_block(ticket) && threadIdx.x == 0) {
         *hout = (int64_t)__ldcg(bad_blocks);
@@ -2757,7 +2771,7 @@ void energies(Lattice *L, double out[3]) {
 int check_finite(Lattice *L) {
     int64_t *h = (int64_t *)host_slot(L);
     const int64_t n = L->length * 2;
-    const int g = grid_cap(n, 256, 8);
+    const int g = grid_cap(n * L->esz / 16, 256, 8);
     if (L->esz == 4)
         k_finite<float><<<g, 256, 0, L->stream>>>((const float *)L->psi[L->cur], (const float *)L->pih, n, L->dtally,
                                                   L->dticket, h);

@@ -125,3 +125,26 @@ assert abs(again[4] - th) <= 1e-14, (again[4], th)
     for _ in range(3):
         r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
         assert r.returncode == 0, r.stderr
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("nd,N", [(2, 4), (2, 6), (3, 4), (3, 10)])
+def test_finite_check_at_every_place(axs, nd, N, precision):
+    """One NaN or infinity anywhere (first, last and other components of psi and of pih) is seen; the largest and smallest
+    finite values are not."""
+    dt = np.float32 if precision == 32 else np.float64
+    info = np.finfo(dt)
+    rng = np.random.default_rng(N)
+    ok = [rng.choice([info.max, -info.max, info.tiny, -info.smallest_subnormal, 0.0, -0.0, 1.0], (N,) * nd).astype(dt) for _ in range(4)]
+    with axs.Lattice(params(axs, nd, N, precision)) as L:
+        L.upload(*ok, dtype=dt)
+        assert L.check_finite()
+        places = [0, 1, 2, 3, N ** nd - 2, N ** nd - 1, *rng.integers(0, N ** nd, 6)]
+        for f in range(4):
+            for at, bad in zip(places, [np.nan, np.inf, -np.inf] * 4):
+                g = [a.copy() for a in ok]
+                g[f].reshape(-1)[at] = bad
+                L.upload(*g, dtype=dt)
+                assert not L.check_finite(), (f, at, bad)
+        L.upload(*ok, dtype=dt)
+        assert L.check_finite()
