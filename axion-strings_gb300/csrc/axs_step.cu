@@ -3333,8 +3333,11 @@ void ensemble_autotune(Ensemble *E) {
     // member up to 256^3). Each ensemble is tuned anew: timing every variant at every
     // z-chunk took 450 ms for 24 members
     std::vector<std::pair<double, int>> screen;
+    int64_t sites = 0;
+    for (Lattice *m : E->members) sites += m->length;
+    const int warm = sites >= (1 << 24) ? 0 : 1;   // as for a single lattice
     for (int v = 0; v < kNumZVariants; ++v)
-        if (ensemble_variant_ok(E, v) && variant_resident(E->members[0]->esz, v)) screen.push_back({trial(v, 64, 1, 1), v});
+        if (ensemble_variant_ok(E, v) && variant_resident(E->members[0]->esz, v)) screen.push_back({trial(v, 64, 1, warm), v});
     std::sort(screen.begin(), screen.end());
     best_ms = 1e30;
     for (size_t k = 0; k < screen.size() && k < 3; ++k)
@@ -3344,8 +3347,8 @@ void ensemble_autotune(Ensemble *E) {
         double two_ms = 1e30;
         for (const auto &s : screen)
             if (two_step(s.second)) {
-                for (int zc : {32, 64, 128, 256}) {
-                    const double ms = trial(s.second, zc, 3, 1);
+                for (int zc : {64, 128}) {
+                    const double ms = trial(s.second, zc, 2, 1);
                     if (ms < two_ms) {
                         two_ms = ms;
                         c.end_variant = s.second;
@@ -3358,7 +3361,7 @@ void ensemble_autotune(Ensemble *E) {
             E->cfg = c;
             ensemble_table(E, 0.f, true);
             const int nm = (int)E->members.size();
-            measure_passes(c, E->stream, 4, [&](int kv, bool end, int k) {
+            measure_passes(c, E->stream, 2, [&](int kv, bool end, int k) {
                 launch_zmarch(E->members[0]->esz, kv, E->dzlat + (end ? nm : 0), nm, end ? E->zitems_end : E->zitems, E->dcounter,
                               ensemble_parity(E), E->derr, E->stream, 0, k);
                 for (Lattice *m : E->members) {
