@@ -29,8 +29,8 @@
 //
 // Measured (GB300, us per step; two steps per pass through shared memory in
 // brackets): 1024^3 2287 (2840), 512^3 313 (378), 256^3 47 (68), 128^3 9.9 (12.4).
-// (The 1024^3 figure is that of intervals of whole three-step passes; 20 steps are seven
-// passes that cost the same, 2410 per step.) At 512^3 with z-chunks of 128 planes (more
+// (The 1024^3 figure is that of intervals of whole three-step passes; a pass of two steps
+// costs as much, so the tuner gives it to the two-step kernel: 20 steps 2340 per step.) At 512^3 with z-chunks of 128 planes (more
 // planes than the tuner's choice there) a three-step pass issues 47 % of the time with three
 // warps per scheduler, DRAM 54 %: the bound is the latency
 // between issues, and the halo (1.35 sites computed per site kept). Tried and slower at 1024^3:
